@@ -32,7 +32,7 @@ CANDIDATES = {
     "blocks_per_sm": (3, 4),
     "long_seg": (32, 48, 64, 1 << 30),
 }
-DEFAULT = (1, 4, 32)
+DEFAULT = (1, 4, 64)
 SPMM_CANDIDATES = {
     "spmm_rows": (0, 1, 2, 4),
     "spmm_long_row": (0, 512, 1024, 2048),

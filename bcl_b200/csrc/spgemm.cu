@@ -46,6 +46,7 @@
 #include <initializer_list>
 #include <mutex>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 namespace bclx {
@@ -58,9 +59,18 @@ constexpr int kMaxCols = kMaxWords * 32;
 constexpr int kWarpsSym = 8;
 constexpr int kWarpsNum = 8;
 constexpr int kNoStage = 0xff;
-constexpr int kLongSegDefault = 32;       // B segments at least this long are walked in direct mode
+// B segments at least this long are walked in direct mode.  A shorter bound
+// ends more packed batches before they are full (a segment's products follow
+// those before it): R-MAT s16 numeric pass 3.54 ms with 32, 3.42 with 64, 3.44
+// with 96; R-MAT s18 37.0, 35.1 and 34.9.
+constexpr int kLongSegDefault = 64;
 constexpr int kQueueSlots = 256;          // work-queue heads in a plan (one per stage launch)
 constexpr int64_t kVeryHeavyUb = 32768;  // rows above this many products get a whole block in the symbolic pass
+
+constexpr int kBlockWords = kFineCols / 32;  // bitmap words of a fine block
+// Bitmap words of w columns, in whole fine blocks.
+__host__ __device__ __forceinline__ int64_t padded_words(int64_t w) { return (w + kFineCols - 1) / kFineCols * kBlockWords; }
+__device__ __forceinline__ int block_words(int w) { return (w + kFineCols - 1) / kFineCols * kBlockWords; }
 
 struct Geom {
   int64_t gm, gk, gn;   // C grid is gm x gn; the k grid has gk tiles
@@ -80,11 +90,18 @@ struct Geom {
   const int32_t* rot_j = nullptr;
 };
 
-// Rotation of C tile (ti, tj): stage position kk is k = (kk + rotation) mod gk.
-__device__ __forceinline__ int64_t tile_rotation(const Geom& g, int64_t ti, int64_t tj) {
-  const int64_t gi = g.rot_i ? (int64_t)__ldg(g.rot_i + ti) : ti;
-  const int64_t gj = g.rot_j ? (int64_t)__ldg(g.rot_j + tj) : tj;
-  return (gi + gj) % g.gk;
+// Rotation of C tile (ti, tj): stage position kk is k = (kk + rotation) mod gk
+// (stage_k).  Row items, tiles and stages are all below 2^31 (check_grids), so
+// the divisions here are 32-bit ones: an item's set-up is a fifth of the
+// numeric pass, and each 64-bit division is some 70 instructions of it.
+__device__ __forceinline__ int32_t tile_rotation(const Geom& g, int64_t ti, int64_t tj) {
+  const uint32_t gi = g.rot_i ? (uint32_t)__ldg(g.rot_i + ti) : (uint32_t)ti;
+  const uint32_t gj = g.rot_j ? (uint32_t)__ldg(g.rot_j + tj) : (uint32_t)tj;
+  return (int32_t)((gi + gj) % (uint32_t)g.gk);
+}
+__device__ __forceinline__ int64_t stage_k(const Geom& g, int kk, int rot) {
+  const int k = kk + rot;
+  return k < (int)g.gk ? k : k - (int)g.gk;
 }
 
 __device__ __forceinline__ int stage_count(const Geom& g, int64_t ti, int64_t tj) {
@@ -136,17 +153,17 @@ __device__ __forceinline__ void b_block_range(const int32_t* trows, const int32_
 }
 
 struct RowInfo {
-  int64_t ti, tj, r;
-  int64_t rot;  // the C tile's stage rotation (tile_rotation)
+  int32_t ti, tj, r;
+  int32_t rot;  // the C tile's stage rotation (tile_rotation)
   int w;        // width of the C tile (columns)
 };
 
 __device__ __forceinline__ RowInfo decode_row(const Geom& g, int64_t ri) {
   RowInfo x;
-  const int64_t t = ri / g.tm;
-  x.r = ri - t * g.tm;
-  x.ti = t / g.gn;
-  x.tj = t - x.ti * g.gn;
+  const uint32_t t = (uint32_t)ri / (uint32_t)g.tm;
+  x.r = (int32_t)((uint32_t)ri - t * (uint32_t)g.tm);
+  x.ti = (int32_t)(t / (uint32_t)g.gn);
+  x.tj = (int32_t)(t - (uint32_t)x.ti * (uint32_t)g.gn);
   x.rot = tile_rotation(g, x.ti, x.tj);
   int64_t w = g.n - x.tj * g.tn;
   x.w = (int)(w < g.tn ? w : g.tn);
@@ -176,26 +193,52 @@ __device__ __forceinline__ P* shfl_ptr(P* p, int src) {
   return reinterpret_cast<P*>(u);
 }
 
+// Shared-memory table of one warp's walk: the entries of a packed run.
+template <typename VT>
+struct WalkTable {
+  ulonglong2 seg[32];  // column and value addresses of product 0 of the run, as this entry's segment continues them
+  struct {
+    VT a;
+    int32_t stage;
+  } av[32];
+};
+
 // Walk the product stream of C-tile row `x` over stages [s0, s1), restricted
-// to fine blocks [fb_lo, fb_hi) of the row when RANGED (through the B-row
+// to fine blocks [fb_lo, fb_hi) of the row when `ranged` (through the B-row
 // table `tab`), in the reference's order.
 //
 // One lane per stage first reads that stage's A-row segment and B-tile
 // pointers.  The A entries of the row (all stages, flattened) are then taken
 // 32 at a time, one per lane, each finding its B segment.  An entry whose B
-// segment has at least kLongSeg products is walked in "direct" mode: lanes
+// segment has at least long_seg products is walked in "direct" mode: lanes
 // stride over the segment and each lane calls fd(j, a, b, stage) for its own
 // products (the columns of one B row are distinct, so lanes never touch the
 // same column; a __syncwarp follows the segment).  Runs of shorter entries
 // are packed 32 products per batch and every lane calls f(valid, j, a, b,
-// stage) once per batch (warp-uniform); valid lanes form a prefix of the warp
-// and lane order is product order.  The loads of batch n+1 are issued before
-// f runs on batch n.
-template <typename VT, bool RANGED, typename F, typename FD>
+// stage, one) once per batch (warp-uniform); valid lanes form a prefix of the
+// warp and lane order is product order; `one`: the batch is 32 products of
+// one entry.  The loads of batch n+1 are issued before f runs on batch n.
+//
+// The run's non-empty entries go to `tbl`, compacted, with their segment
+// addresses moved back by the entry's first product, so that product q is at
+// seg + q whatever its entry.  Which entry a lane's product belongs to is
+// the number of entries that begin at or before it: each entry sets the bit
+// of its first product in the batch, the bits are or-ed over the warp, and a
+// population count gives the entry (one warp reduction and one broadcast-like
+// 16-byte shared load in place of a five-step search and seven shuffles).
+template <typename VT, typename F, typename FD>
 __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridView& B, const Geom& g,
-                                              const RowInfo& x, int s0, int s1, int fb_lo, int fb_hi,
-                                              const int32_t* __restrict__ tab, int long_seg, F&& f, FD&& fd) {
+                                              const RowInfo& x, int s0, int s1, bool ranged, int fb_lo, int fb_hi,
+                                              const int32_t* __restrict__ tab, int long_seg, WalkTable<VT>& tbl,
+                                              F&& f, FD&& fd) {
   const int lane = lane_id();
+  const unsigned below = (1u << lane) - 1u, upto = below | (1u << lane);
+  // an entry's bounds are bptr[kc * bstep + blo], bptr[kc * bstep + bhi]:
+  // the B row pointer, or the row of the B-row table
+  const bool table = ranged && tab != nullptr;
+  const int64_t bstep = table ? g.nfb + 1 : 1;
+  const int blo = table ? fb_lo : 0, bhi = table ? fb_hi : 1;
+  const bool search = ranged && !table;
   int w0, w1;
   stage_window(g, x.ti, x.tj, s0, s1, w0, w1);
   for (int g0 = w0; g0 < w1; g0 += 32) {
@@ -205,21 +248,19 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
     int32_t as = 0, alen = 0;
     const int32_t* acol = nullptr;
     const VT* aval = nullptr;
-    const int32_t* brow = nullptr;   // B row_ptr
-    const int32_t* btrows = nullptr;  // the stage's B-row table block (RANGED, when there is a table)
+    const int32_t* bptr = nullptr;
     const int32_t* bci = nullptr;
     const VT* bva = nullptr;
     if (si < w1) {
       kk = stage_at(g, x.ti, x.tj, si);
-      const int64_t k = (kk + x.rot) % g.gk;
+      const int64_t k = stage_k(g, kk, x.rot);
       const bclx_csr_t At = A.tile(x.ti, k);
       as = __ldg(At.row_ptr + x.r);
       alen = __ldg(At.row_ptr + x.r + 1) - as;
       acol = At.col_ind + as;
       aval = reinterpret_cast<const VT*>(At.vals) + as;
       const bclx_csr_t Bt = B.tile(k, x.tj);
-      brow = Bt.row_ptr;
-      if (RANGED && tab) btrows = tab + (k * g.gn + x.tj) * g.tk * (g.nfb + 1);
+      bptr = table ? tab + (k * g.gn + x.tj) * g.tk * (g.nfb + 1) : Bt.row_ptr;
       bci = Bt.col_ind;
       bva = reinterpret_cast<const VT*>(Bt.vals);
     }
@@ -233,28 +274,24 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       const int32_t off = e - __shfl_sync(kFull, aexcl, sl);
       const int32_t* sacol = shfl_ptr(acol, sl);
       const VT* saval = shfl_ptr(aval, sl);
-      const int32_t* sbrow = shfl_ptr(brow, sl);
+      const int32_t* sbptr = shfl_ptr(bptr, sl);
       const int32_t* sbci = shfl_ptr(bci, sl);
       const VT* sbva = shfl_ptr(bva, sl);
-      const int32_t* sbtr = RANGED ? shfl_ptr(btrows, sl) : nullptr;
       const int stage = __shfl_sync(kFull, kk, sl);
-      int32_t len = 0;
+      int32_t len = 0, bs = 0;
       VT av = VT(0);
-      const int32_t* bcol = nullptr;
-      const VT* bval = nullptr;
       if (e < atot) {
         const int32_t kc = __ldg(sacol + off);
         av = __ldg(saval + off);
-        int32_t bs, be;
-        if (RANGED) {
-          b_block_range(sbtr, sbrow, sbci, kc, fb_lo, fb_hi, g.nfb, bs, be);
-        } else {
-          bs = __ldg(sbrow + kc);
-          be = __ldg(sbrow + kc + 1);
+        const int32_t* p = sbptr + (int64_t)kc * bstep;
+        int32_t be = __ldg(p + bhi);
+        bs = __ldg(p + blo);
+        if (search) {
+          const int32_t b0 = bs, b1 = be;
+          if (fb_lo > 0) bs = lower_bound_i32(sbci, b0, b1, fb_lo * kFineCols);
+          if (fb_hi < g.nfb) be = lower_bound_i32(sbci, bs, b1, fb_hi * kFineCols);
         }
         len = be - bs;
-        bcol = sbci + bs;
-        bval = sbva + bs;
       }
       const int nent = min(32, atot - e0);
       const unsigned longm = __ballot_sync(kFull, len >= long_seg);
@@ -262,44 +299,59 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       while (e_start < nent) {
         const unsigned lm = longm & (kFull << e_start);
         const int e_long = lm ? __ffs(lm) - 1 : nent;
-        if (e_long > e_start) {
+        const int32_t lenm = (lane >= e_start && lane < e_long) ? len : 0;
+        const unsigned full = __ballot_sync(kFull, lenm > 0);  // the run's non-empty entries
+        if (full) {
           // packed batches over the short entries [e_start, e_long), software pipelined
-          const int32_t lenm = (lane >= e_start && lane < e_long) ? len : 0;
           const int32_t incl = warp_inclusive_scan(lenm);
           const int32_t total = __shfl_sync(kFull, incl, 31);
           const int32_t excl = incl - lenm;
+          if (lenm > 0) {
+            const int at = __popc(full & below);
+            tbl.seg[at] = make_ulonglong2(reinterpret_cast<unsigned long long>(sbci + bs) - 4ull * (unsigned)excl,
+                                          reinterpret_cast<unsigned long long>(sbva + bs) - 4ull * (unsigned)excl);
+            tbl.av[at].a = av;
+            tbl.av[at].stage = stage;
+          }
+          __syncwarp();
+          const int32_t begins = lenm > 0 ? excl : INT_MAX;  // this entry's first product
+          int ahead = -1;                                    // entries begun before the batch, less one
           int32_t nj = -1;
           VT na = VT(0), nb = VT(0);
           int nst = 0;
+          bool none = false;
           auto fetch = [&](int32_t base) {
+            const int32_t d = begins - base;
+            const unsigned heads = __reduce_or_sync(kFull, (unsigned)d < 32u ? 1u << d : 0u);
+            const int src = ahead + __popc(heads & upto);
+            ahead += __popc(heads);
+            none = (heads & ~1u) == 0u;  // no entry begins after the batch's first product
             const int32_t q = base + lane;
-            const int src = warp_search(incl, q);
-            const int32_t pos = q - __shfl_sync(kFull, excl, src);
-            const int32_t* sbcol = shfl_ptr(bcol, src);
-            const VT* sbval = shfl_ptr(bval, src);
-            na = __shfl_sync(kFull, av, src);
-            nst = __shfl_sync(kFull, stage, src);
+            const ulonglong2 sg = tbl.seg[src];
+            na = tbl.av[src].a;
+            nst = tbl.av[src].stage;
             nj = -1;
             nb = VT(0);
             if (q < total) {
-              nj = __ldg(sbcol + pos);
-              nb = __ldg(sbval + pos);
+              nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * (unsigned)q));
+              nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * (unsigned)q));
             }
           };
-          if (total > 0) fetch(0);
+          fetch(0);
           for (int32_t base = 0; base < total; base += 32) {
             const int32_t j = nj;
             const VT a = na, b = nb;
             const int st = nst;
+            const bool one = none && base + 32 <= total;
             if (base + 32 < total) fetch(base + 32);
-            f(j >= 0, j, a, b, st);
+            f(j >= 0, j, a, b, st, one);
           }
         }
         if (e_long < nent) {
           // direct mode over one long segment
           const int32_t dl = __shfl_sync(kFull, len, e_long);
-          const int32_t* dcol = shfl_ptr(bcol, e_long);
-          const VT* dval = shfl_ptr(bval, e_long);
+          const int32_t* dcol = shfl_ptr(sbci + bs, e_long);
+          const VT* dval = shfl_ptr(sbva + bs, e_long);
           const VT da = __shfl_sync(kFull, av, e_long);
           const int dst = __shfl_sync(kFull, stage, e_long);
           int32_t q = lane;
@@ -337,7 +389,7 @@ __device__ __forceinline__ void walk_columns(const SpGridView& A, const SpGridVi
     const int32_t* brp = nullptr;
     const int32_t* bci = nullptr;
     if (si < ns) {
-      const int64_t k = (stage_at(g, x.ti, x.tj, si) + x.rot) % g.gk;
+      const int64_t k = stage_k(g, stage_at(g, x.ti, x.tj, si), x.rot);
       const bclx_csr_t At = A.tile(x.ti, k);
       as = __ldg(At.row_ptr + x.r);
       alen = __ldg(At.row_ptr + x.r + 1) - as;
@@ -437,7 +489,7 @@ __device__ __forceinline__ void walk_columns_ranged(const SpGridView& A, const S
     const int32_t* brp = nullptr;
     const int32_t* bci = nullptr;
     if (si < ns) {
-      const int64_t k = (stage_at(g, x.ti, x.tj, si) + x.rot) % g.gk;
+      const int64_t k = stage_k(g, stage_at(g, x.ti, x.tj, si), x.rot);
       const bclx_csr_t At = A.tile(x.ti, k);
       as = __ldg(At.row_ptr + x.r);
       alen = __ldg(At.row_ptr + x.r + 1) - as;
@@ -573,7 +625,7 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
         const int32_t* acol = nullptr;
         const int32_t* brp = nullptr;
         if (si < ns) {
-          const int64_t k = (stage_at(g, x.ti, x.tj, si) + x.rot) % g.gk;
+          const int64_t k = stage_k(g, stage_at(g, x.ti, x.tj, si), x.rot);
           const bclx_csr_t At = A.tile(x.ti, k);
           as = __ldg(At.row_ptr + x.r);
           alen = __ldg(At.row_ptr + x.r + 1) - as;
@@ -661,7 +713,11 @@ __global__ void k_btable(SpGridView B, Geom g, int32_t* __restrict__ tab) {
 // Symbolic pass.  Heavy rows are numbered 0..n_heavy-1 (the very heavy ones
 // first); a row's column bitmap is built in shared memory, its popcount is
 // the row's output count, and heavy rows also store the bitmap for the
-// numeric pass (hbm_words words per row).
+// numeric pass (hbm_words words per row).  With heavy_span they record
+// their first and one past their last fine block with outputs, and
+// k_symbolic stores only the blocks between; where hbm_words is a whole
+// number of fine blocks, whole blocks are stored (the last one's words past
+// the tile are 0).
 //
 // One warp per row for the light and ordinary heavy rows (heavy first),
 // rows taken from a device counter (each warp grabs its next row while it
@@ -673,7 +729,7 @@ __global__ void __launch_bounds__(kWarpsSym * 32, 4)
                const int32_t* __restrict__ heavy_list, int n_light, int n_heavy, int n_vheavy,
                int32_t* __restrict__ row_count, uint32_t* __restrict__ heavy_bitmaps, int64_t hbm_words,
                int16_t* __restrict__ heavy_span, unsigned long long* __restrict__ queue, int grab) {
-  __shared__ uint32_t bm_all[kWarpsSym][kMaxWords];
+  __shared__ __align__(16) uint32_t bm_all[kWarpsSym][kMaxWords];
   uint32_t* bm = bm_all[threadIdx.x >> 5];
   const int lane = lane_id();
   const unsigned long long n_items = (unsigned long long)((int64_t)n_light + n_heavy - n_vheavy);
@@ -689,34 +745,35 @@ __global__ void __launch_bounds__(kWarpsSym * 32, 4)
     const bool heavy = idx < n_heavy;
     const int64_t ri = heavy ? heavy_list[idx] : light_list[idx - n_heavy];
     const RowInfo x = decode_row(g, ri);
-    const int words = (x.w + 31) >> 5;
-    for (int w = lane; w < words; w += 32) bm[w] = 0u;
+    const int words = block_words(x.w);
+    for (int w = lane * 4; w < words; w += 128) *reinterpret_cast<uint4*>(bm + w) = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
     walk_columns(A, B, g, x, 0, 1, [&](int32_t j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
     __syncwarp();
-    int cnt = 0, w0 = INT_MAX, w1 = -1;
-    uint32_t* out = heavy ? heavy_bitmaps + idx * hbm_words : nullptr;
-    for (int w = lane; w < words; w += 32) {
-      const uint32_t v = bm[w];
-      if (heavy) out[w] = v;
-      cnt += __popc(v);
-      if (v) {
-        w0 = min(w0, w);
-        w1 = max(w1, w);
+    int cnt = 0, b0 = INT_MAX, b1 = 0;  // fine blocks with outputs: [b0, b1)
+    for (int w = lane * 4; w < words; w += 128) {
+      const uint4 v = *reinterpret_cast<const uint4*>(bm + w);
+      cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
+      if (v.x | v.y | v.z | v.w) {
+        b0 = min(b0, w / kBlockWords);
+        b1 = w / kBlockWords + 1;
       }
     }
-    cnt = warp_sum(cnt);
-    if (heavy && heavy_span) {
-      w0 = __reduce_min_sync(kFull, w0);
-      w1 = __reduce_max_sync(kFull, w1);
-    }
-    if (lane == 0) {
-      row_count[ri] = cnt;
-      if (heavy && heavy_span) {
-        heavy_span[2 * idx] = (int16_t)(cnt > 0 ? w0 / (kFineCols / 32) : 0);
-        heavy_span[2 * idx + 1] = (int16_t)(cnt > 0 ? w1 / (kFineCols / 32) + 1 : 0);
+    cnt = __reduce_add_sync(kFull, cnt);
+    if (heavy) {
+      // with a span the blocks outside it are not stored (nothing reads them)
+      uint32_t* out = heavy_bitmaps + idx * hbm_words;
+      int from = 0, to = (hbm_words % kBlockWords) == 0 ? words : (x.w + 31) >> 5;
+      if (heavy_span) {
+        b0 = cnt > 0 ? __reduce_min_sync(kFull, b0) : 0;
+        b1 = __reduce_max_sync(kFull, b1);
+        from = b0 * kBlockWords;
+        to = b1 * kBlockWords;
+        if (lane == 0) *reinterpret_cast<short2*>(heavy_span + 2 * idx) = make_short2((short)b0, (short)b1);
       }
+      for (int w = from + lane; w < to; w += 32) out[w] = bm[w];
     }
+    if (lane == 0) row_count[ri] = cnt;
     __syncwarp();
     }
     base = __shfl_sync(kFull, nx, 0);
@@ -735,7 +792,7 @@ __global__ void __launch_bounds__(kWarpsSym * 32)
   for (int64_t h = blockIdx.x; h < n_vheavy; h += gridDim.x) {
     const int64_t ri = heavy_list[h];
     const RowInfo x = decode_row(g, ri);
-    const int words = (x.w + 31) >> 5;
+    const int words = (hbm_words % kBlockWords) == 0 ? block_words(x.w) : (x.w + 31) >> 5;
     for (int w = threadIdx.x; w < words; w += blockDim.x) bm[w] = 0u;
     if (threadIdx.x == 0) {
       first_word = INT_MAX;
@@ -841,12 +898,13 @@ __global__ void __launch_bounds__(256)
     const uint32_t* bm = heavy_bitmaps + h * hbm_words;
     const int words = (x.w + 31) >> 5;
     int tot = 0, first_nz = INT_MAX, last_nz = -1;
+    const int sp0 = span ? span[2 * h] : 0, sp1 = span ? span[2 * h + 1] : nfb;  // blocks that are stored
     for (int b = lane; b < nfb; b += 32) {
       int c = 0;
 #pragma unroll
       for (int q = 0; q < kWordsPerBlock; q++) {
         const int w = b * kWordsPerBlock + q;
-        if (w < words) c += __popc(__ldg(bm + w));
+        if (w < words && b >= sp0 && b < sp1) c += __popc(__ldg(bm + w));
       }
       cnt[b] = c;
       tot += c;
@@ -897,19 +955,24 @@ __global__ void __launch_bounds__(256)
 
 template <typename VT, int WORDS, int VCAP>
 struct WarpSmem {
-  uint32_t bm[WORDS];
-  uint16_t pre[WORDS];
-  VT acc[VCAP];
-  VT part[VCAP];
-  unsigned char tag[VCAP];
-  VT sa[32];
-  VT sb[32];
-  int32_t ss[32];
+  alignas(16) uint32_t bm[WORDS];
+  alignas(16) uint16_t pre[WORDS];
+  alignas(16) VT acc[VCAP];
+  alignas(16) VT part[VCAP];
+  alignas(16) unsigned char tag[VCAP];
+  WalkTable<VT> walk;
 };
 
 #ifndef BCLX_NUMERIC_MIN_BLOCKS
 #define BCLX_NUMERIC_MIN_BLOCKS 4
 #endif
+// Bound by instruction issue (67 % of the slots) and the shared-memory pipe
+// (68 %), not by DRAM.  Packed entry table, columns staged in shared memory,
+// prefix counts 8 words per lane, 32-bit divisions, int32 without an order:
+// R-MAT s16 on 8x8 tiles 3.84 -> 3.42 ms per launch, s18 on 16x16 39.3 -> 35.1
+// ms; R-MAT of 30,011 rows in int32 0.96 -> 0.42 ms; the 27-point stencil
+// on 128^3, whose rows are one item each (walked by the B rows' own bounds
+// instead of two binary searches per A entry), 37.6 -> 29.1 ms.
 // LEARNED: the learned product's single pass.  Heavy items come from the
 // predicted cut (their counts are unknown): each builds its bitmap from its
 // own products, and an item with more than kVcap outputs marks its row in
@@ -950,6 +1013,7 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     const bool heavy = idx < n_heavy_items;
     int64_t ri;
     int cnt = 0, fb_lo = 0, fb_hi = 0, lo = 0, hi, hslot = 0, icap = VCAP;
+    bool whole = false;  // the item holds all outputs of its row
     int64_t off;
     const uint32_t* hb = nullptr;
     if (heavy) {
@@ -963,6 +1027,7 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
         icap = it.count;  // temp slots sized from the prediction
       } else {
         cnt = it.count;
+        whole = cnt == row_count[ri];
         off = row_offset[ri] + it.rel;
         hb = heavy_bitmaps + (int64_t)it.h * hbm_words;
       }
@@ -984,21 +1049,20 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     }
     const int w0 = lo >> 5;
     const int words = ((hi - lo) + 31) >> 5;
+    const bool stored = heavy && !LEARNED;  // the symbolic pass left this row's bitmap
 
-    // 1. column bitmap of the item (word w covers columns lo + 32w ..)
-    if (heavy && LEARNED) {
-      for (int w = lane; w < words; w += 32) S.bm[w] = 0u;
+    // 1. column bitmap of a light or learned item (word w covers columns
+    // lo + 32w ..), cleared and kept in whole blocks of 8 words
+    if (!stored) {
+      for (int w = lane * 4; w < words; w += 128) *reinterpret_cast<uint4*>(S.bm + w) = make_uint4(0u, 0u, 0u, 0u);
+      if (lane < 4 && ((words + 3) & ~3) + lane < ((words + 7) & ~7)) S.bm[((words + 3) & ~3) + lane] = 0u;
       __syncwarp();
-      walk_columns_ranged(A, B, g, x, fb_lo, fb_hi, tab, [&](int32_t j) {
-        const int xx = j - lo;
-        atomicOr(&S.bm[xx >> 5], 1u << (xx & 31));
-      });
-    } else if (heavy) {
-      for (int w = lane; w < words; w += 32) S.bm[w] = __ldg(hb + w0 + w);
-    } else {
-      for (int w = lane; w < words; w += 32) S.bm[w] = 0u;
-      __syncwarp();
-      if (s0 == 0) {
+      if (heavy) {
+        walk_columns_ranged(A, B, g, x, fb_lo, fb_hi, tab, [&](int32_t j) {
+          const int xx = j - lo;
+          atomicOr(&S.bm[xx >> 5], 1u << (xx & 31));
+        });
+      } else if (s0 == 0) {
         walk_columns(A, B, g, x, 0, 1, [&](int32_t j) { atomicOr(&S.bm[j >> 5], 1u << (j & 31)); });
       } else {
         for (int q = lane; q < cnt; q += 32) {
@@ -1006,22 +1070,54 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
           atomicOr(&S.bm[j >> 5], 1u << (j & 31));
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
 
-    // 2. per-word exclusive prefix counts
+    // 2. per-word exclusive prefix counts, 8 words per lane in registers: a
+    // heavy item's words come from its row's stored bitmap on the way
     {
-      const int per = (words + 31) >> 5;
-      const int wa = lane * per;
-      int loc = 0;
-      for (int w = wa; w < wa + per && w < words; w++) loc += __popc(S.bm[w]);
-      const int inc = warp_inclusive_scan(loc);
-      int ex = inc - loc;
-      for (int w = wa; w < wa + per && w < words; w++) {
-        S.pre[w] = (uint16_t)ex;
-        ex += __popc(S.bm[w]);
+      int before = 0;
+      for (int b = 0; b < words; b += 256) {
+        const int w = b + lane * 8;
+        uint32_t u[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        if (w < words) {
+          if (stored && hbm_words % kBlockWords == 0) {
+            const uint4 v0 = __ldg(reinterpret_cast<const uint4*>(hb + w0 + w));
+            const uint4 v1 = __ldg(reinterpret_cast<const uint4*>(hb + w0 + w) + 1);
+            u[0] = v0.x; u[1] = v0.y; u[2] = v0.z; u[3] = v0.w;
+            u[4] = v1.x; u[5] = v1.y; u[6] = v1.z; u[7] = v1.w;
+          } else if (stored) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) u[i] = w + i < words ? __ldg(hb + w0 + w + i) : 0u;
+          } else {
+            const uint4 v0 = *reinterpret_cast<const uint4*>(S.bm + w);
+            const uint4 v1 = *reinterpret_cast<const uint4*>(S.bm + w + 4);
+            u[0] = v0.x; u[1] = v0.y; u[2] = v0.z; u[3] = v0.w;
+            u[4] = v1.x; u[5] = v1.y; u[6] = v1.z; u[7] = v1.w;
+          }
+        }
+        int loc = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) loc += __popc(u[i]);
+        const int inc = warp_inclusive_scan(loc);
+        if (w < words) {
+          if (stored) {
+            *reinterpret_cast<uint4*>(S.bm + w) = make_uint4(u[0], u[1], u[2], u[3]);
+            *reinterpret_cast<uint4*>(S.bm + w + 4) = make_uint4(u[4], u[5], u[6], u[7]);
+          }
+          uint32_t p[4];
+          uint32_t ex = (uint32_t)(before + inc - loc);
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            const uint32_t mid = ex + __popc(u[2 * i]);
+            p[i] = ex | (mid << 16);
+            ex = mid + __popc(u[2 * i + 1]);
+          }
+          *reinterpret_cast<uint4*>(S.pre + w) = make_uint4(p[0], p[1], p[2], p[3]);
+        }
+        before += __shfl_sync(kFull, inc, 31);
       }
-      if (LEARNED) cnt = __shfl_sync(kFull, inc, 31);
+      if (LEARNED) cnt = before;
     }
     __syncwarp();
     if (LEARNED) {
@@ -1039,42 +1135,40 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
       }
     }
 
-    // 3. sorted columns (first stage range only) and the accumulators
+    // 3. sorted columns (first stage range only) and the accumulators.  The
+    // columns are put in order in shared memory (in the space of `part`) and
+    // leave as whole lines: written one by one from the bitmap's words they
+    // are as many separate L2 writes as outputs.
     if (s0 == 0) {
+      int32_t* const cols = reinterpret_cast<int32_t*>(S.part);
       for (int w = lane; w < words; w += 32) {
         uint32_t bits = S.bm[w];
-        int pos = S.pre[w];
+        int32_t* to = cols + S.pre[w];
+        const int32_t c = lo + w * 32 - 1;
         while (bits) {
-          const int b = __ffs(bits) - 1;
+          *to++ = c + __ffs(bits);
           bits &= bits - 1;
-          out_col[off + pos++] = lo + w * 32 + b;
         }
       }
+      __syncwarp();
+      for (int q = lane; q < cnt; q += 32) out_col[off + q] = cols[q];
+      for (int q = lane * 4; q < cnt; q += 128) *reinterpret_cast<uint4*>(S.acc + q) = make_uint4(0u, 0u, 0u, 0u);
+    } else {
+      for (int q = lane; q < cnt; q += 32) S.acc[q] = out_val[off + q];
     }
-    for (int q = lane; q < cnt; q += 32) {
-      S.acc[q] = s0 == 0 ? VT(0) : out_val[off + q];
-      S.part[q] = VT(0);
-      S.tag[q] = (unsigned char)kNoStage;
-    }
+    // `part` is read only where `tag` names a stage
+    for (int q = lane * 16; q < cnt; q += 512) *reinterpret_cast<uint4*>(S.tag + q) = make_uint4(kFull, kFull, kFull, kFull);
     __syncwarp();
 
-    // 4. values in the reference's order, with a lazy per-column stage fold
-    auto update = [&](bool valid, int32_t j, VT a, VT b, int stage) {
-      int rank = 0;
-      if (valid) {
-        const int xx = j - lo;
-        rank = S.pre[xx >> 5] + __popc(S.bm[xx >> 5] & ((1u << (xx & 31)) - 1u));
-      }
-      const unsigned peers = __match_any_sync(kFull, valid ? j : -1);
-      const bool single = peers == (1u << lane);
-      if (__any_sync(kFull, valid && !single)) {
-        S.sa[lane] = a;
-        S.sb[lane] = b;
-        S.ss[lane] = stage;
-        __syncwarp();
-      }
-      if (valid && single) {
-        // the only product of its column in this batch
+    // 4. values in the reference's order, with a lazy per-column stage fold.
+    // int32 sums wrap, so their order is immaterial: one shared-memory add.
+    constexpr bool kOrdered = std::is_same<VT, float>::value;
+    auto rank_of = [&](int32_t j) {
+      const int xx = j - lo;
+      return (int)S.pre[xx >> 5] + __popc(S.bm[xx >> 5] & ((1u << (xx & 31)) - 1u));
+    };
+    auto apply = [&](int rank, VT a, VT b, int stage) {
+      if constexpr (kOrdered) {
         VT v = S.part[rank];
         const int t = S.tag[rank];
         if (t != stage) {
@@ -1083,50 +1177,42 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
           S.tag[rank] = (unsigned char)stage;
         }
         S.part[rank] = madd(a, b, v);
-      } else if (valid && lane == __ffs(peers) - 1) {
-        VT v = S.part[rank];
-        int t = S.tag[rank];
-        VT ac = S.acc[rank];
-        unsigned gmask = peers;
-        do {
-          const int mb = __ffs(gmask) - 1;
-          gmask &= gmask - 1;
-          const int st = S.ss[mb];
-          if (st != t) {
-            if (t != kNoStage) ac = vadd(ac, v);
-            v = VT(0);
-            t = st;
-          }
-          v = madd(S.sa[mb], S.sb[mb], v);
-        } while (gmask);
-        S.part[rank] = v;
-        S.tag[rank] = (unsigned char)t;
-        S.acc[rank] = ac;
+      } else {
+        atomicAdd(reinterpret_cast<unsigned*>(&S.acc[rank]), (unsigned)a * (unsigned)b);
       }
-      __syncwarp();
+    };
+    auto update = [&](bool valid, int32_t j, VT a, VT b, int stage, bool one) {
+      const int rank = valid ? rank_of(j) : 0;
+      if constexpr (kOrdered) {
+        // products of one column in a batch go one after another, in lane
+        // order: a lane's turn is the number of lower lanes with its column
+        const unsigned peers = one ? 0u : __match_any_sync(kFull, valid ? j : ~lane) & ((1u << lane) - 1u);
+        if (one || !__any_sync(kFull, peers != 0u)) {
+          if (valid) apply(rank, a, b, stage);
+        } else {
+          const int turn = __popc(peers), last = __reduce_max_sync(kFull, turn);
+          for (int t = 0; t <= last; t++) {
+            if (valid && t == turn) apply(rank, a, b, stage);
+            __syncwarp();
+          }
+        }
+        __syncwarp();
+      } else {
+        if (valid) apply(rank, a, b, stage);
+        __syncwarp();
+      }
     };
     // direct mode: the lanes hold distinct columns, each updates its own
-    auto update_direct = [&](int32_t j, VT a, VT b, int stage) {
-      const int xx = j - lo;
-      const int rank = S.pre[xx >> 5] + __popc(S.bm[xx >> 5] & ((1u << (xx & 31)) - 1u));
-      VT v = S.part[rank];
-      const int t = S.tag[rank];
-      if (t != stage) {
-        if (t != kNoStage) S.acc[rank] = vadd(S.acc[rank], v);
-        v = VT(0);
-        S.tag[rank] = (unsigned char)stage;
-      }
-      S.part[rank] = madd(a, b, v);
-    };
-    if (heavy)
-      walk_products<VT, true>(A, B, g, x, s0, s1, fb_lo, fb_hi, tab, long_seg, update, update_direct);
-    else
-      walk_products<VT, false>(A, B, g, x, s0, s1, 0, 0, nullptr, long_seg, update, update_direct);
+    auto update_direct = [&](int32_t j, VT a, VT b, int stage) { apply(rank_of(j), a, b, stage); };
+    // An item that holds all of its row's outputs takes every product of the
+    // row: the B rows' own bounds serve, without the table or a search.
+    const bool ranged = heavy && (LEARNED ? (fb_lo > 0 || fb_hi * kFineCols < x.w) : !whole);
+    walk_products<VT>(A, B, g, x, s0, s1, ranged, fb_lo, fb_hi, tab, long_seg, S.walk, update, update_direct);
 
     // 5. last fold and values out
     for (int q = lane; q < cnt; q += 32) {
       VT v = S.acc[q];
-      if (S.tag[q] != kNoStage) v = vadd(v, S.part[q]);
+      if (kOrdered && S.tag[q] != kNoStage) v = vadd(v, S.part[q]);
       out_val[off + q] = v;
     }
     __syncwarp();
@@ -1161,7 +1247,7 @@ __global__ void __launch_bounds__(256) k_heavy_block_ub(SpGridView A, SpGridView
     __syncwarp();
     const int ns = stage_count(g, x.ti, x.tj);
     for (int si = 0; si < ns; si++) {
-      const int64_t k = (stage_at(g, x.ti, x.tj, si) + x.rot) % g.gk;
+      const int64_t k = stage_k(g, stage_at(g, x.ti, x.tj, si), x.rot);
       const bclx_csr_t At = A.tile(x.ti, k);
       const int32_t a0 = __ldg(At.row_ptr + x.r), a1 = __ldg(At.row_ptr + x.r + 1);
       // per A entry: a B row shorter than the block count is counted column
@@ -1695,7 +1781,7 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   BCLX_TRY(build_btable(ctx, B, g, P, ctx->side));
   P->dtype = dtype;
   const int64_t nri = g.n_row_items;
-  P->hbm_words = (g.tn + 31) / 32;
+  P->hbm_words = padded_words(g.tn);
   BCLX_TRY(scratch_alloc_n(ctx, &P->light_list, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_list, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->vheavy_list, nri));
@@ -2313,7 +2399,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
   // start, beside classification and the prediction.
   BCLX_TRY(ensure_side_stream(ctx));
   BCLX_TRY(build_btable(ctx, B, g, P, ctx->side));
-  P->hbm_words = (g.tn + 31) / 32;
+  P->hbm_words = padded_words(g.tn);
   const int64_t nri = g.n_row_items;
   BCLX_TRY(scratch_alloc_n(ctx, &P->light_list, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_list, nri));
