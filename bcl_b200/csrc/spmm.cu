@@ -20,7 +20,9 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
+#include <type_traits>
 #include <vector>
 
 namespace bclx {
@@ -154,8 +156,9 @@ __device__ __forceinline__ StageLane<ST> stage_lane(const SpGridView& A, const D
   StageLane<ST> s{0, nullptr, nullptr, nullptr};
   const int64_t gk = A.gn;
   if (valid && kk < gk) {
-    const int64_t rot = SUB ? (int64_t)__ldg(B.rot_i + ti) + __ldg(B.rot_j + tj) : ti + tj;
-    const int64_t k = B.natural_order ? kk : (kk + rot) % gk;
+    // (tile and stage counts are below 2^31: a 32-bit division)
+    const uint32_t rot = SUB ? (uint32_t)__ldg(B.rot_i + ti) + (uint32_t)__ldg(B.rot_j + tj) : (uint32_t)(ti + tj);
+    const int64_t k = B.natural_order ? kk : ((uint32_t)kk + rot) % (uint32_t)gk;
     const bclx_csr_t At = A.tile(ti, k);
     const int32_t as = __ldg(At.row_ptr + r);
     s.alen = __ldg(At.row_ptr + r + 1) - as;
@@ -374,13 +377,14 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
   flush();
 }
 
-// Warp items come from a device counter (one grab per item, the next grab in
+// Tile columns [0, tjn) (k_spmm_narrow takes the others).  Warp items come
+// from a device counter (one grab per item, the next grab in
 // flight while the current item runs), so warps that draw short rows take
 // more of them: the cost of a (row group, panel) item varies by orders of
 // magnitude on power-law matrices.
 template <typename ST, bool GROUP, bool SUB>
 __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
-    k_spmm(SpGridView A, DGridView B, DGridView C, int64_t n_items, int npanels, int R, int64_t ngroups,
+    k_spmm(SpGridView A, DGridView B, DGridView C, int tjn, int64_t n_items, int npanels, int R, int64_t ngroups,
            int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag,
            unsigned long long* __restrict__ next_item) {
   constexpr int PW = 32 * Vec<ST>::N;
@@ -404,7 +408,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     }
     const int64_t t = rg / ngroups;
     const int64_t r0 = (rg - t * ngroups) * R;
-    const int64_t ti = t / C.gn, tj = t - ti * C.gn;
+    const int64_t ti = t / tjn, tj = t - ti * tjn;
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
@@ -610,7 +614,7 @@ __device__ __forceinline__ void spmm_long_row(LongSmem& S, const SpGridView& A, 
 // programmatic dependent (k_spmm under the dependent-launch schedule) launch.
 template <typename ST, bool SUB>
 __global__ void __launch_bounds__(kLongWarps * 32)
-    k_spmm_long(SpGridView A, DGridView B, DGridView C, const int64_t* __restrict__ list,
+    k_spmm_long(SpGridView A, DGridView B, DGridView C, int tjn, const int64_t* __restrict__ list,
                 const int32_t* __restrict__ count, int npanels, int row_align_ok,
                 unsigned long long* __restrict__ next_item) {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
@@ -621,7 +625,7 @@ __global__ void __launch_bounds__(kLongWarps * 32)
   const int64_t rows = A.gm * A.tm;
   const int64_t nv = count[0];
   const int64_t nl = nv + count[1];
-  const int64_t per_row = C.gn * npanels;
+  const int64_t per_row = (int64_t)tjn * npanels;
   const unsigned long long n = (unsigned long long)(nl * per_row);
   unsigned long long it = 0;
   if (lane == 0) it = atomicAdd(next_item, 1ULL);
@@ -642,6 +646,513 @@ __global__ void __launch_bounds__(kLongWarps * 32)
     }
     it = __shfl_sync(kFull, nx, 0);
   }
+}
+
+// ---- narrow and unaligned tiles ------------------------------------------------
+//
+// k_spmm gives a B-row slice of 512 bytes to a warp's 32 lanes.  A tile of a
+// few columns leaves most of those lanes idle, and one whose rows do not
+// start on 16 bytes would be read element by element, each load waited for.
+// Two kernels take those tiles:
+//  * k_spmm_narrow, the short rows: a group of L lanes per row (8 to 32), so
+//    that a warp walks 32 / L rows at once, each lane owning NV units of the
+//    row (16-byte vectors, or 4- or 2-byte words where rows start on no more);
+//  * k_spmm_chain, the long rows (32 L entries or more, over all stages): one
+//    chain of multiply-adds per column that cannot be split, only fed.  A
+//    block takes one: producer warps copy the B-row slices of the next entries
+//    into shared memory (cp.async, three buffers), one consumer warp runs 32
+//    words' chains from there and does nothing else.
+// Products with many rows list their long rows first (k_spmm_find_long) and
+// run both at once: k_spmm_narrow is launched as k_spmm_chain's programmatic
+// dependent, starts once every chain block has, and ends after it.  With
+// fewer rows (where the extra launch would show) k_spmm_narrow lists the long
+// rows it meets and k_spmm_chain follows.
+// Bound: the short rows by instruction issue (67 % of the slots; a third of a
+// warp's groups wait for its longest row) and by the latency of their loads
+// (A entry, then B row), hidden by 32 warps per SM; a long row by its chain,
+// 4.5 ns per entry (k_spmm_long: 25).  FP32 products, k_spmm before -> now:
+// R-MAT 169,343 x 47 columns (rows on 4 bytes) 3.51 -> 0.27 ms; R-MAT 400,001 x
+// 16 0.64 -> 0.27; R-MAT 300,000 x 64 0.51 -> 0.32; uniform 100,000 x 32 90 ->
+// 54 us; BF16, R-MAT 50,000 x 135 (rows on 2 bytes) 2.5 -> 0.37 ms.
+constexpr int kNarrowWarps = 8;
+constexpr int kNarrowUnroll = 4;          // entries per lane group whose loads are in flight
+// A row is long from this many steps of L entries (or BCLX_TUNE_SPMM_LONG_ROW):
+// fewer make k_spmm_chain's set-up per row (3.5 us of a block) show, more leave
+// a warp its longest row (R-MAT 50,000 x 8: 82 us with 16 steps, 83 with 32, 111
+// with 64; R-MAT 300,000 x 32 BF16: 284, 264, 289).
+constexpr int kNarrowLongSteps = 32;
+// Widest row of an aligned tile that k_spmm_narrow takes: two 128-byte lines
+// (one warp then walks two rows).  At 256 bytes: R-MAT 300,000 x 64 FP32 0.32
+// ms against 0.51 with k_spmm, uniform 100,000 x 128 BF16 93 us against 108.
+constexpr int64_t kNarrowMaxBytes = 256;
+constexpr int kChainWarps = 8;            // one applies, the others copy
+constexpr int kChainPanelWords = 32;      // words of a long row that a block takes at once: one per consumer lane
+constexpr int kChainBuffers = 3;
+constexpr int kChainBytes = 92 * 1024;    // shared memory for their slices and values (two blocks per SM)
+
+// First lane whose inclusive prefix exceeds e (32 when none does).
+__device__ __forceinline__ int warp_search_lanes(int32_t incl, int32_t e) {
+  int src = 0;
+#pragma unroll
+  for (int step = 16; step >= 1; step >>= 1) {
+    const int32_t t = __shfl_sync(kFull, incl, src + step - 1);
+    if (t <= e) src += step;
+  }
+  return src;
+}
+
+// A unit of U bytes of a row of ST: load, store and the chain step.
+template <typename ST, int U>
+struct Unit {
+  static constexpr int N = U / (int)sizeof(ST);  // columns
+  using R = std::conditional_t<U == 16, uint4, std::conditional_t<U == 4, uint32_t, uint16_t>>;
+  __device__ __forceinline__ static R load(const ST* p, int u) { return __ldg(reinterpret_cast<const R*>(p) + u); }
+  __device__ __forceinline__ static R load_c(const ST* p, int u) { return reinterpret_cast<const R*>(p)[u]; }
+  __device__ __forceinline__ static void store(ST* p, int u, R v) { reinterpret_cast<R*>(p)[u] = v; }
+  __device__ __forceinline__ static void unpack(R v, float* o) {
+    if constexpr (U == 16) {
+      Vec<ST>::unpack_raw(v, o);
+    } else if constexpr (sizeof(ST) == 4) {
+      o[0] = __uint_as_float(v);
+    } else {
+      o[0] = __uint_as_float((uint32_t)v << 16);
+      if constexpr (U == 4) o[1] = __uint_as_float(v & 0xffff0000u);
+    }
+  }
+  __device__ __forceinline__ static uint32_t bf16_bits(float x) {
+    return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x));
+  }
+  __device__ __forceinline__ static R pack(const float* i) {
+    if constexpr (U == 16 && sizeof(ST) == 4) {
+      return make_uint4(__float_as_uint(i[0]), __float_as_uint(i[1]), __float_as_uint(i[2]), __float_as_uint(i[3]));
+    } else if constexpr (U == 16) {
+      return make_uint4(bf16_bits(i[0]) | bf16_bits(i[1]) << 16, bf16_bits(i[2]) | bf16_bits(i[3]) << 16,
+                        bf16_bits(i[4]) | bf16_bits(i[5]) << 16, bf16_bits(i[6]) | bf16_bits(i[7]) << 16);
+    } else if constexpr (sizeof(ST) == 4) {
+      return __float_as_uint(i[0]);
+    } else if constexpr (U == 4) {
+      return bf16_bits(i[0]) | bf16_bits(i[1]) << 16;
+    } else {
+      return (uint16_t)bf16_bits(i[0]);
+    }
+  }
+};
+
+// Every row slice of C tile (ti, tj) and of its B tiles starts on U bytes and
+// is a whole number of them.
+template <typename ST, int U>
+__device__ __forceinline__ bool tile_on(const DGridView& B, const DGridView& C, int64_t ti, int64_t tj, int W) {
+  uint32_t low = (uint32_t)reinterpret_cast<uintptr_t>(C.tile(ti, tj)) | (uint32_t)(B.ld * sizeof(ST)) |
+                 (uint32_t)(C.ld * sizeof(ST)) | (uint32_t)(W * sizeof(ST));
+  for (int64_t k = lane_id(); k < B.gm; k += 32) low |= (uint32_t)reinterpret_cast<uintptr_t>(B.tile(k, tj));
+  return __reduce_or_sync(kFull, low & (uint32_t)(U - 1)) == 0u;
+}
+
+// Rows [r0, r0 + 32/L) of C tile (ti, tj), columns [c0, c0 + W): the group of
+// L lanes g walks row r0 + g, L entries at a time: each lane finds and loads
+// one A entry (the next L are in flight meanwhile) and the group's lanes then
+// take the B rows kNarrowUnroll at a time.  32/L * gk <= 32: one lane per
+// (row, stage) holds that segment; with L == 32 the stages go 32 at a time.
+// Rows of long_row entries or more are left out; their mask (by group) is
+// returned.
+template <typename ST, int U, int NV, bool SUB>
+__device__ __forceinline__ unsigned narrow_rows(const SpGridView& A, const DGridView& B, const DGridView& C,
+                                                int64_t ti, int64_t tj, int64_t r0, int L, int c0, int W,
+                                                int long_row) {
+  using UN = Unit<ST, U>;
+  constexpr int N = UN::N;
+  const int lane = lane_id();
+  const int gk = (int)A.gn;
+  const int grp = lane / L, li = lane & (L - 1);
+  const int rows = 32 / L;
+  const int64_t nrows = min((int64_t)rows, C.rows_of(ti) - r0);
+  ST* __restrict__ crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + (r0 + grp) * C.ld + c0;
+  const int units = W / N;
+  float acc[NV][N];
+  bool have = false;  // the row's chain is in acc
+  unsigned left = 0u;
+  for (int g0 = 0; g0 < gk; g0 += 32) {
+    const int sq = L == 32 ? 0 : lane / gk;
+    const int64_t kk = L == 32 ? g0 + lane : lane - sq * gk;
+    const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r0 + sq, kk, sq < nrows);
+    const int32_t aincl = warp_inclusive_scan(sl.alen);
+    const int32_t aexcl = aincl - sl.alen;
+    const int f = L == 32 ? 0 : grp * gk, l = L == 32 ? 31 : min(grp * gk + gk - 1, 31);
+    const int32_t first = __shfl_sync(kFull, aexcl, min(f, 31));
+    int32_t T = __shfl_sync(kFull, aincl, l) - first;  // this group's entries
+    if (grp >= nrows) T = 0;
+    if (T >= long_row) {
+      left = 1u << grp;
+      T = 0;
+    }
+    const int32_t most = __reduce_max_sync(kFull, T);
+    if (most == 0) continue;
+    if (T > 0 && !have) {
+      have = true;
+#pragma unroll
+      for (int i = 0; i < NV; i++)
+        if (li + L * i < units) UN::unpack(UN::load_c(crow, li + L * i), acc[i]);
+    }
+    int32_t nc = 0;
+    float nv = 0.f;
+    const ST* nbt = nullptr;
+    auto fetch = [&](int32_t p) {  // A entry p + li of the group's row
+      const int32_t e = first + p + li;
+      const int src = min(warp_search_lanes(aincl, e), 31);
+      const int32_t off = e - __shfl_sync(kFull, aexcl, src);
+      const int32_t* sacol = reinterpret_cast<const int32_t*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
+      const float* saval = reinterpret_cast<const float*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
+      nbt = reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), src));
+      if (p + li < T) {
+        nc = __ldg(sacol + off);
+        nv = __ldg(saval + off);
+      }
+    };
+    fetch(0);
+    for (int32_t p = 0; p < most; p += L) {
+      const float v = nv;
+      const unsigned long long baddr = reinterpret_cast<unsigned long long>(nbt + (int64_t)nc * B.ld + c0);
+      if (p + L < most) fetch(p + L);
+      const int here = min(L, most - p);  // (uniform)
+      for (int u0 = 0; u0 < here; u0 += kNarrowUnroll) {
+        float vs[kNarrowUnroll];
+        const ST* br[kNarrowUnroll];
+#pragma unroll
+        for (int k = 0; k < kNarrowUnroll; k++) {
+          br[k] = reinterpret_cast<const ST*>(__shfl_sync(kFull, baddr, u0 + k, L));
+          vs[k] = __shfl_sync(kFull, v, u0 + k, L);
+        }
+        typename UN::R raw[kNarrowUnroll][NV];
+#pragma unroll
+        for (int k = 0; k < kNarrowUnroll; k++)
+#pragma unroll
+          for (int i = 0; i < NV; i++)
+            if (p + u0 + k < T && li + L * i < units) raw[k][i] = UN::load(br[k], li + L * i);
+#pragma unroll
+        for (int k = 0; k < kNarrowUnroll; k++)
+          if (p + u0 + k < T) {
+#pragma unroll
+            for (int i = 0; i < NV; i++) {
+              float b[N];
+              UN::unpack(raw[k][i], b);
+#pragma unroll
+              for (int x = 0; x < N; x++) acc[i][x] = __fmaf_rn(vs[k], b[x], acc[i][x]);
+            }
+          }
+      }
+    }
+  }
+  if (have) {
+#pragma unroll
+    for (int i = 0; i < NV; i++)
+      if (li + L * i < units) UN::store(crow, li + L * i, UN::pack(acc[i]));
+  }
+  return __reduce_or_sync(kFull, left);
+}
+
+// Rows [r0, r1) of C tile (ti, tj), columns [c0, c1), one column per lane and
+// one entry at a time: tiles whose base is off the launch's unit (the host
+// sees their leading dimensions and widths, not the device array of bases).
+template <typename ST, bool SUB>
+__device__ __forceinline__ void elem_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
+                                          int64_t tj, int64_t r0, int64_t r1, int c0, int c1, int long_row) {
+  for (int64_t r = r0; r < r1; r++) {
+    int64_t total = 0;
+    for (int64_t k = 0; k < A.gn; k++) {
+      const int32_t* rp = A.tile(ti, k).row_ptr + r;
+      total += __ldg(rp + 1) - __ldg(rp);
+    }
+    if (total == 0 || total >= long_row) continue;
+    ST* crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld;
+    for (int c = c0 + lane_id(); c < c1; c += 32) {
+      float acc = Vec<ST>::to_f(crow[c]);
+      for (int64_t kk = 0; kk < A.gn; kk++) {
+        const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, kk, true);
+        for (int32_t e = 0; e < sl.alen; e++)
+          acc = __fmaf_rn(__ldg(sl.aval + e), Vec<ST>::to_f(sl.bt[(int64_t)__ldg(sl.acol + e) * B.ld + c]), acc);
+      }
+      crow[c] = Vec<ST>::from_f(acc);
+    }
+  }
+}
+
+// The chains of n entries in a buffer: this lane's word of each slice at `sw`
+// (slices STRIDE words apart), the A values at `sv`.  The next eight entries'
+// words are loaded before the current eight are applied, so that a chain step
+// waits for its multiply-add alone.
+template <typename ST, int STRIDE>
+__device__ __forceinline__ void chain_apply(const uint32_t* sw, const float* sv, int n, float* acc) {
+  constexpr int CN = 4 / (int)sizeof(ST);
+  struct Eight {
+    uint32_t x[8];
+    float v[8];
+  };
+  auto load = [&](Eight& t, int u) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) t.x[k] = sw[(u + k) * STRIDE];
+    const float4 a = *reinterpret_cast<const float4*>(sv + u), b = *reinterpret_cast<const float4*>(sv + u + 4);
+    t.v[0] = a.x; t.v[1] = a.y; t.v[2] = a.z; t.v[3] = a.w;
+    t.v[4] = b.x; t.v[5] = b.y; t.v[6] = b.z; t.v[7] = b.w;
+  };
+  auto step = [&](uint32_t x, float v) {
+    float o[CN];
+    Unit<ST, 4>::unpack(x, o);
+#pragma unroll
+    for (int c = 0; c < CN; c++) acc[c] = __fmaf_rn(v, o[c], acc[c]);
+  };
+  auto apply = [&](const Eight& t) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) step(t.x[k], t.v[k]);
+  };
+  int u = 0;
+  if (n >= 8) {
+    Eight t0, t1;
+    load(t0, 0);
+    for (; u + 24 <= n; u += 16) {
+      load(t1, u + 8);
+      apply(t0);
+      load(t0, u + 16);
+      apply(t1);
+    }
+    if (u + 16 <= n) {
+      load(t1, u + 8);
+      apply(t0);
+      apply(t1);
+      u += 16;
+    } else {
+      apply(t0);
+      u += 8;
+    }
+  }
+  for (; u < n; u++) step(sw[u * STRIDE], sv[u]);
+}
+
+// One long row r of C tile (ti, tj), columns [c0, c0 + W) (at most
+// kChainPanelWords words), by the whole block: warp 0 applies, the others
+// copy, `each` entries of a batch per producer warp.  While batch b is
+// applied from its buffer, batches b + 1 and b + 2 are in flight.  One barrier
+// per batch: past it batch b has landed (each producer waited for its own
+// copies) and batch b - 1, whose buffer batch b + 2 overwrites, has been
+// applied.  At most 32 stages.  Buffers: slices of `stride` words, then the
+// values.
+template <typename ST, bool SUB>
+__device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int stride, int each, const SpGridView& A,
+                                          const DGridView& B, const DGridView& C, int64_t ti, int64_t tj, int64_t r,
+                                          int c0, int W, int unit) {
+  constexpr int CN = 4 / (int)sizeof(ST);  // columns per word
+  const int lane = lane_id();
+  const int prod = (int)(threadIdx.x >> 5) - 1;  // producer number; -1: the consumer
+  const int nw = (W * (int)sizeof(ST) + 3) >> 2;
+  const int batch = each * (kChainWarps - 1);
+  ST* __restrict__ crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld + c0;
+  const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, lane, true);
+  const int32_t aincl = warp_inclusive_scan(sl.alen);
+  const int32_t atot = __shfl_sync(kFull, aincl, 31);
+  const int32_t aexcl = aincl - sl.alen;
+  const int32_t nb = (atot + batch - 1) / batch;
+  if (prod < 0) {
+    // the lane's columns 2 lane and 2 lane + 1 (BF16) or lane (FP32)
+    float acc[CN];
+#pragma unroll
+    for (int x = 0; x < CN; x++) acc[x] = lane < nw && lane * CN + x < W ? Vec<ST>::to_f(crow[lane * CN + x]) : 0.f;
+    for (int32_t b = 0; b < nb; b++) {
+      __syncthreads();
+      const int n = min(batch, atot - b * batch);
+      const int base = (b % kChainBuffers) * batch;
+      const uint32_t* sw = slices + base * stride + lane;
+      const float* sv = vals + base;
+      if (stride == 4) chain_apply<ST, 4>(sw, sv, n, acc);
+      else if (stride == 8) chain_apply<ST, 8>(sw, sv, n, acc);
+      else if (stride == 16) chain_apply<ST, 16>(sw, sv, n, acc);
+      else chain_apply<ST, 32>(sw, sv, n, acc);
+    }
+#pragma unroll
+    for (int x = 0; x < CN; x++)
+      if (lane < nw && lane * CN + x < W) crow[lane * CN + x] = Vec<ST>::from_f(acc[x]);
+  } else {
+    const int n_unit = W * (int)sizeof(ST) / unit;  // copies per slice
+    const int trips = (each * n_unit + 31) >> 5;
+    const int u_first = lane / n_unit, q_first = lane - u_first * n_unit;
+    const int u_step = 32 / n_unit, q_step = 32 - u_step * n_unit;
+    int32_t nc = 0;  // the pending A entry: its column, value and B tile
+    float nv = 0.f;
+    const ST* nbt = nullptr;
+    auto fetch = [&](int32_t x) {
+      if (x >= nb) return;
+      const int32_t e = x * batch + prod * each + lane;
+      const int src = min(warp_search_lanes(aincl, e), 31);
+      const int32_t off = e - __shfl_sync(kFull, aexcl, src);
+      const int32_t* sacol = reinterpret_cast<const int32_t*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
+      const float* saval = reinterpret_cast<const float*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
+      nbt = reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), src));
+      if (lane < each && e < atot) {
+        nc = __ldg(sacol + off);
+        nv = __ldg(saval + off);
+      }
+    };
+    auto issue = [&](int32_t x) {  // batch x: its A entries are in nc, nv, nbt
+      if (x < nb) {
+        const int base = (x % kChainBuffers) * batch + prod * each;
+        const int left = min(each, atot - x * batch - prod * each);  // entries of this warp (or none)
+        const unsigned long long addr = reinterpret_cast<unsigned long long>(nbt + (int64_t)nc * B.ld + c0);
+        if (lane < each) vals[base + lane] = nv;
+        char* to = reinterpret_cast<char*>(slices + base * stride);
+        int u = u_first, q = q_first;
+        auto next = [&]() {
+          u += u_step;
+          q += q_step;
+          if (q >= n_unit) {
+            q -= n_unit;
+            u++;
+          }
+        };
+        if (left <= 0) {
+        } else if (unit != 2) {
+#pragma unroll 4
+          for (int i = 0; i < trips; i++) {
+            const char* from = reinterpret_cast<const char*>(__shfl_sync(kFull, addr, u & 31)) + q * unit;
+            char* dst = to + u * stride * 4 + q * unit;
+            if (u < left) {
+              if (unit == 16) cp_async16_nb(dst, from);
+              else cp_async4_nb(dst, from);
+            }
+            next();
+          }
+        } else {  // no asynchronous copy of 2 bytes: eight loads in flight
+          for (int i0 = 0; i0 < trips; i0 += 8) {
+            uint16_t h[8];
+            int at[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+              const uint16_t* from = reinterpret_cast<const uint16_t*>(__shfl_sync(kFull, addr, u & 31)) + q;
+              at[k] = u < left ? u * stride * 2 + q : -1;
+              if (at[k] >= 0) h[k] = __ldg(from);
+              next();
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+              if (at[k] >= 0) reinterpret_cast<uint16_t*>(to)[at[k]] = h[k];
+          }
+        }
+      }
+      cp_async_commit();
+    };
+    fetch(0);
+    issue(0);
+    fetch(1);
+    issue(1);
+    fetch(2);
+    for (int32_t b = 0; b < nb; b++) {
+      cp_async_wait_group<1>();  // this warp's part of batch b has landed
+      __syncthreads();
+      issue(b + 2);
+      fetch(b + 3);
+    }
+    cp_async_wait_all();
+  }
+  __syncthreads();  // the buffers are free again
+}
+
+// Long rows of tile columns [tj0, tj0 + tjn), a block per (row, tile column,
+// panel).  `met`: list[0, count[0]) holds row * tjn + tile column of the rows
+// that k_spmm_narrow met (its programmatic dependent: it waits for it);
+// otherwise the rows k_spmm_find_long listed, and k_spmm_narrow may start.
+template <typename ST, bool SUB>
+__global__ void __launch_bounds__(kChainWarps * 32, 2)
+    k_spmm_chain(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int npanels, int stride, int each, bool met,
+                 const int64_t* __restrict__ list, const int32_t* __restrict__ count,
+                 unsigned long long* __restrict__ next_item) {
+  if (met) asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  else asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  extern __shared__ __align__(16) unsigned char chain_smem[];
+  __shared__ int64_t item[2], code[2];
+  uint32_t* slices = reinterpret_cast<uint32_t*>(chain_smem);
+  float* vals = reinterpret_cast<float*>(slices + kChainBuffers * (kChainWarps - 1) * each * stride + kChainPanelWords);
+  constexpr int PW = kChainPanelWords * 4 / (int)sizeof(ST);
+  const int64_t rows = A.gm * A.tm;
+  const int64_t nv = count[0], nl = nv + (met ? 0 : count[1]);
+  const int64_t per = (met ? 1 : tjn) * (int64_t)npanels;
+  const int64_t n = nl * per;
+  // thread 0 takes an item and reads its row ahead, while the block works on
+  // the one before
+  auto take = [&](int slot) {
+    const int64_t it = (int64_t)atomicAdd(next_item, 1ULL);
+    item[slot] = it < n ? it : -1;
+    if (it < n) {
+      const int64_t q = it / per;
+      code[slot] = q < nv ? list[q] : list[rows - 1 - (q - nv)];
+    }
+  };
+  if (threadIdx.x == 0) take(0);
+  __syncthreads();
+  for (int slot = 0;; slot ^= 1) {
+    const int64_t it = item[slot];
+    if (it < 0) break;
+    const int64_t x = met ? code[slot] / tjn : code[slot];  // the row, over all tile rows
+    const int pt = (int)(it % per);
+    const int64_t tj = tj0 + (met ? code[slot] - x * tjn : pt / npanels);
+    const int64_t ti = x / A.tm;
+    const int W = (int)C.cols_of(tj), c0 = pt % npanels * PW;
+    if (threadIdx.x == 0) take(slot ^ 1);
+    if (c0 < W) {
+      const int unit = tile_on<ST, 16>(B, C, ti, tj, W) ? 16 : (tile_on<ST, 4>(B, C, ti, tj, W) ? 4 : 2);
+      chain_row<ST, SUB>(slices, vals, stride, each, A, B, C, ti, tj, x - ti * A.tm, c0, min(PW, W - c0), unit);
+    } else {
+      __syncthreads();  // (chain_row ends with a barrier)
+    }
+  }
+}
+
+// Short rows of tile columns [tj0, tj0 + tjn).  With `met` the long rows go to
+// that list (met_count their number), otherwise they are left to k_spmm_chain.
+template <typename ST, int U, int NV, bool SUB>
+__global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
+    k_spmm_narrow(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int L, int npanels, int64_t n_items,
+                  int64_t ngroups, int long_row, int64_t* __restrict__ met, int32_t* __restrict__ met_count,
+                  unsigned long long* __restrict__ next_item) {
+  constexpr int PW = 32 * NV * Unit<ST, U>::N;  // columns of a panel
+  const int lane = lane_id();
+  unsigned long long it = 0;
+  if (lane == 0) it = atomicAdd(next_item, 1ULL);
+  it = __shfl_sync(kFull, it, 0);
+  int64_t at = -1, ti = 0, tj = 0;  // the C tile of the last item
+  bool on = false;
+  while ((int64_t)it < n_items) {
+    unsigned long long nx = 0;
+    if (lane == 0) nx = atomicAdd(next_item, 1ULL);
+    const int64_t rg = npanels == 1 ? (int64_t)it : (int64_t)it / npanels;
+    const int panel = (int)((int64_t)it - rg * npanels);
+    const int64_t t = rg / ngroups;
+    const int64_t r0 = (rg - t * ngroups) * (32 / L);
+    if (t != at) {
+      at = t;
+      ti = t / tjn;
+      tj = tj0 + (t - ti * tjn);
+      on = tile_on<ST, U>(B, C, ti, tj, (int)C.cols_of(tj));
+    }
+    const int W = (int)C.cols_of(tj);
+    const int c0 = panel * PW;
+    if (r0 < C.rows_of(ti) && c0 < W) {
+      const int c1 = min(W, c0 + PW);
+      if (on) {
+        unsigned left = narrow_rows<ST, U, NV, SUB>(A, B, C, ti, tj, r0, L, c0, c1 - c0, long_row);
+        if (met && panel == 0 && lane == 0)
+          for (; left; left &= left - 1)
+            met[atomicAdd(met_count, 1)] = (ti * A.tm + r0 + __ffs(left) - 1) * tjn + (tj - tj0);
+      } else {
+        // (met: none is left to k_spmm_chain, whose list this kernel fills by rows on the unit)
+        elem_rows<ST, SUB>(A, B, C, ti, tj, r0, min(r0 + 32 / L, C.rows_of(ti)), c0, c1, met ? INT_MAX : long_row);
+      }
+    }
+    it = __shfl_sync(kFull, nx, 0);
+  }
+  // launched as k_spmm_chain's programmatic dependent: finish only after it
+  // (a normal launch returns here at once)
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 // Launch delay of the short-row kernel under the side-stream schedule: a
@@ -680,13 +1191,13 @@ static int64_t spmm_long_min_rows() {
 // Rows per k_spmm warp item: grouping short rows shares one prologue (tile
 // descriptors, row pointers, A loads) among them, while the items still
 // cover every resident warp.  BCLX_TUNE_SPMM_ROWS (1, 2, 4) overrides.
-static int spmm_rows_per_item(const Context* ctx, const DGridView& C, int64_t gk, int npanels) {
+static int spmm_rows_per_item(const Context* ctx, const DGridView& C, int64_t tjn, int64_t gk, int npanels) {
   auto fits = [&](int r) { return r <= kSpmmMaxRows && r * gk <= 32; };
   const int want = (int)tuning(ctx, BCLX_TUNE_SPMM_ROWS);
   if ((want == 1 || want == 2 || want == 4) && fits(want)) return want;
   const int64_t resident = (int64_t)ctx->num_sms * 4 * kSpmmWarps;
   int r = 1;
-  while (fits(2 * r) && C.gm * C.gn * ceil_div(C.tm, (int64_t)(2 * r)) * npanels >= resident) r *= 2;
+  while (fits(2 * r) && C.gm * tjn * ceil_div(C.tm, (int64_t)(2 * r)) * npanels >= resident) r *= 2;
   return r;
 }
 
@@ -706,12 +1217,12 @@ static int spmm_rows_per_item(const Context* ctx, const DGridView& C, int64_t gk
 // mbarrier, in place of the per-lane copies: 6.8 ms for k_spmm_long alone
 // against 1.9.
 template <typename ST, bool SUB>
-static int launch_spmm(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int align_ok) {
+static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int tjn, int align_ok) {
   constexpr int VN = Vec<ST>::N;
   const int npanels = (int)ceil_div(C.tn, 32 * VN);
-  const int R = spmm_rows_per_item(ctx, C, A.gn, npanels);
+  const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, npanels);
   const int64_t ngroups = ceil_div(C.tm, (int64_t)R);
-  const int64_t n_items = C.gm * C.gn * ngroups * npanels;
+  const int64_t n_items = C.gm * tjn * ngroups * npanels;
   if (n_items == 0) return BCLX_OK;
   const int64_t want = ceil_div(n_items, kSpmmWarps);
   const int64_t cap = (int64_t)ctx->num_sms * 4;  // resident blocks: warps take items from a counter
@@ -747,7 +1258,7 @@ static int launch_spmm(Context* ctx, const SpGridView& A, const DGridView& B, co
     if (!dependent) BCLX_CK(cudaEventRecord(ctx->fork2_ev, ctx->side));
     const size_t lsmem = sizeof(LongSmem) * kLongWarps;
     BCLX_CK(cudaFuncSetAttribute(k_spmm_long<ST, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem));
-    k_spmm_long<ST, SUB><<<(unsigned)spmm_long_blocks(ctx, npanels), kLongWarps * 32, lsmem, ls>>>(A, B, C, list, cnt, npanels,
+    k_spmm_long<ST, SUB><<<(unsigned)spmm_long_blocks(ctx, npanels), kLongWarps * 32, lsmem, ls>>>(A, B, C, tjn, list, cnt, npanels,
                                                                                     align_ok, ctr + 1);
     note_launch();
     BCLX_CK_LAUNCH();
@@ -773,10 +1284,10 @@ static int launch_spmm(Context* ctx, const SpGridView& A, const DGridView& B, co
   const uint8_t* lflag = flag;
   const int pmajor = (int)tuning(ctx, BCLX_TUNE_SPMM_PANEL_MAJOR);
   if (R > 1)
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB>, A, B, C, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
                                ctr));
   else
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB>, A, B, C, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
                                ctr));
   note_launch();
   BCLX_CK_LAUNCH();
@@ -787,6 +1298,139 @@ static int launch_spmm(Context* ctx, const SpGridView& A, const DGridView& B, co
   }
   scratch_free(ctx, ctr);
   return BCLX_OK;
+}
+
+// Launch `kern` so that it may start before the kernel ahead of it in the
+// stream has finished (`early`; not inside a capture, where launches stay in
+// plain order).
+template <typename... KP, typename... AP>
+static int launch_after(Context* ctx, bool early, unsigned grid, unsigned threads, size_t smem, void (*kern)(KP...),
+                        AP... args) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (early) BCLX_CK(cudaStreamIsCapturing(ctx->stream, &cap));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early && cap == cudaStreamCaptureStatusNone ? 1 : 0;
+  BCLX_CK(cudaLaunchKernelEx(&cfg, kern, KP(args)...));
+  note_launch();
+  return BCLX_OK;
+}
+
+// k_spmm_narrow and k_spmm_chain over tile columns [tj0, tj0 + tjn), `width`
+// columns each (the last may have fewer), rows on U bytes.
+template <typename ST, int U, int NV, bool SUB>
+static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int tj0,
+                            int tjn, int64_t width, int L) {
+  constexpr int PW = 32 * NV * Unit<ST, U>::N;
+  const int npanels = (int)ceil_div(width, PW);
+  const int64_t ngroups = ceil_div(C.tm, (int64_t)(32 / L));
+  const int64_t n_items = C.gm * tjn * ngroups * npanels;
+  if (n_items == 0) return BCLX_OK;
+  // long rows: slices a power of two of words apart, batches of as many
+  // entries as three buffers hold, a whole number of eights per producer warp
+  int stride = 4;
+  while (stride < kChainPanelWords && stride * 4 < width * (int64_t)sizeof(ST)) stride *= 2;
+  const int fit = kChainBytes / (kChainBuffers * (kChainWarps - 1) * (stride + 1) * 4);
+  const int each = std::min(32, fit / 8 * 8);
+  const size_t smem = 4 * (size_t)(kChainBuffers * (kChainWarps - 1) * each * (stride + 1) + kChainPanelWords);
+  const int64_t arows = A.gm * A.tm;
+  const bool chains = A.gn <= 32;  // one lane per stage
+  const bool listed = chains && arows >= spmm_long_min_rows();
+  int long_row = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_ROW);
+  if (long_row <= 0) long_row = kNarrowLongSteps * L;
+  if (!chains) long_row = INT_MAX;
+  // counters: [0] row groups taken, [1] long rows taken, [2] listed very long / other long rows (2 x int32)
+  unsigned long long* ctr = nullptr;
+  uint8_t* flag = nullptr;
+  int64_t* list = nullptr;
+  BCLX_TRY(scratch_alloc_n(ctx, &ctr, 3));
+  BCLX_CK(cudaMemsetAsync(ctr, 0, 3 * sizeof(unsigned long long), ctx->stream));
+  int32_t* cnt = reinterpret_cast<int32_t*>(ctr + 2);
+  if (chains) BCLX_TRY(scratch_alloc_n(ctx, &list, (size_t)arows * (listed ? 1 : tjn)));
+  if (listed) {
+    BCLX_TRY(scratch_alloc_n(ctx, &flag, (size_t)arows));
+    k_spmm_find_long<<<(unsigned)std::min<int64_t>(ceil_div(arows, 256), (int64_t)ctx->num_sms * 16), 256, 0,
+                       ctx->stream>>>(A, long_row, (int)std::min<int64_t>((int64_t)long_row * 8, INT32_MAX), flag, list, cnt);
+    note_launch();
+    BCLX_CK_LAUNCH();
+  }
+  auto narrow = [&]() {
+    const int64_t blocks = std::min(ceil_div(n_items, kNarrowWarps), (int64_t)ctx->num_sms * 4);
+    return launch_after(ctx, listed, (unsigned)blocks, kNarrowWarps * 32, 0, k_spmm_narrow<ST, U, NV, SUB>, A, B, C,
+                        tj0, tjn, L, npanels, n_items, ngroups, long_row, listed ? nullptr : list, cnt, ctr);
+  };
+  if (!listed) BCLX_TRY(narrow());
+  if (chains) {
+    auto kern = k_spmm_chain<ST, SUB>;
+    BCLX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // one block per SM beside k_spmm_narrow, two where it has finished
+    const int64_t blocks = std::min<int64_t>(arows * tjn, (int64_t)ctx->num_sms * (listed ? 1 : 2));
+    BCLX_TRY(launch_after(ctx, !listed, (unsigned)blocks, kChainWarps * 32, smem, kern, A, B, C, tj0, tjn,
+                          (int)ceil_div(width * (int64_t)sizeof(ST), 4 * kChainPanelWords), stride, each, !listed, list,
+                          cnt, ctr + 1));
+  }
+  if (listed) BCLX_TRY(narrow());
+  scratch_free(ctx, flag);
+  scratch_free(ctx, list);
+  scratch_free(ctx, ctr);
+  return BCLX_OK;
+}
+
+// Lanes per row: one 16-byte vector per lane, or up to four words (each lane
+// then loads as many bytes); at least as many as stages, so that a warp's
+// (row, stage) segments fit its lanes.
+template <typename ST, int U, bool SUB>
+static int launch_narrow_u(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int64_t tj0,
+                           int64_t tjn, int64_t width) {
+  const int64_t units = ceil_div(width * (int64_t)sizeof(ST), U);
+  const int per = U == 16 ? 1 : 4;
+  int L = 8;
+  while (L < 32 && (L * per < units || L < A.gn)) L *= 2;
+  const int64_t nv = ceil_div(std::min<int64_t>(units, 32 * per), L);
+  if constexpr (U != 16) {
+    if (nv > 2) return launch_narrow_nv<ST, U, 4, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
+    if (nv > 1) return launch_narrow_nv<ST, U, 2, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
+  }
+  return launch_narrow_nv<ST, U, 1, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
+}
+
+template <typename ST, bool SUB>
+static int launch_narrow(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int64_t tj0,
+                         int64_t tjn, int64_t width) {
+  const int64_t es = (int64_t)sizeof(ST);
+  const int64_t low = (B.ld * es) | (C.ld * es) | (width * es) |
+                      (B.tiles ? 0 : (int64_t)(reinterpret_cast<uintptr_t>(B.single) | reinterpret_cast<uintptr_t>(C.single)));
+  if (low % 16 == 0) return launch_narrow_u<ST, 16, SUB>(ctx, A, B, C, tj0, tjn, width);
+  if constexpr (sizeof(ST) == 2) {
+    if (low % 4 != 0) return launch_narrow_u<ST, 2, SUB>(ctx, A, B, C, tj0, tjn, width);
+  }
+  return launch_narrow_u<ST, 4, SUB>(ctx, A, B, C, tj0, tjn, width);
+}
+
+// Which kernel takes which tile columns: k_spmm_narrow those whose rows are
+// narrow (at most kNarrowMaxBytes) or not whole 16-byte vectors, k_spmm (with
+// k_spmm_long) the others.  The last tile column may be narrower than the rest.
+template <typename ST, bool SUB>
+static int launch_spmm(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int align_ok) {
+  if (C.gn == 0 || C.gm == 0) return BCLX_OK;
+  const int64_t last = C.n - (C.gn - 1) * C.tn;
+  const bool narrow = !align_ok || C.tn * (int64_t)sizeof(ST) <= kNarrowMaxBytes;
+  const bool split = C.gn > 1 ? last % Vec<ST>::N != 0 : false;
+  if (C.gn == 1) {
+    if (narrow || last % Vec<ST>::N != 0) return launch_narrow<ST, SUB>(ctx, A, B, C, 0, 1, last);
+    return launch_wide<ST, SUB>(ctx, A, B, C, 1, align_ok);
+  }
+  const int64_t tjn = split ? C.gn - 1 : C.gn;
+  if (narrow) BCLX_TRY((launch_narrow<ST, SUB>(ctx, A, B, C, 0, tjn, C.tn)));
+  else BCLX_TRY((launch_wide<ST, SUB>(ctx, A, B, C, (int)tjn, align_ok)));
+  return split ? launch_narrow<ST, SUB>(ctx, A, B, C, tjn, 1, last) : BCLX_OK;
 }
 
 static int run_spmm(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int dtype) {
