@@ -102,6 +102,7 @@ SIGNATURES = {
     "bclx_dmatrix_sum": [vp, ctypes.POINTER(DGrid), vp],
     "bclx_spmatrix_binary_op": [vp, ctypes.POINTER(SpGrid), ctypes.POINTER(DGrid), i32],
     "bclx_csr_to_tiles": [vp, ctypes.POINTER(CSRDesc), ctypes.POINTER(SpGridOut)],
+    "bclx_spgrid_describe": [vp, ctypes.POINTER(SpGridOut), vp],
     "bclx_tiles_to_csr": [vp, ctypes.POINTER(SpGrid), vp, vp, vp],
 }
 _RESTYPES = {"bclx_last_error": ctypes.c_char_p, "bclx_launch_count": ctypes.c_longlong}

@@ -255,7 +255,7 @@ class SPMatrix:
         np_dtype = np.dtype(np.float32) if vals.dtype == torch.float32 else np.dtype(np.int32)
         dt = _NP_TO_DT[np_dtype]
         trp = torch.empty((gm * gn, tm + 1), dtype=torch.int32, device=td)
-        toff = torch.zeros(gm * gn + 1, dtype=torch.int64, device=td)
+        toff = (torch.empty if gm * gn else torch.zeros)(gm * gn + 1, dtype=torch.int64, device=td)
         oci = torch.empty(max(nnz, 1), dtype=torch.int32, device=td)
         ov = torch.empty(max(nnz, 1), dtype=vals.dtype, device=td)
         desc = CSRDesc(m, n, nnz, row_ptr.data_ptr(), col_ind.data_ptr() if nnz else 0,
@@ -287,22 +287,30 @@ class SPMatrix:
                    torch.zeros(0, dtype=_TORCH_OF[_NP_TO_DT[np.dtype(dtype)]], device=td))
 
     def _build_desc(self):
-        """Device array of bclx_csr_t, one per tile, computed on the device."""
+        """Device array of bclx_csr_t, one per tile, computed on the device
+        (bclx_spgrid_describe; with torch for host tensors)."""
         ntiles = self.gm * self.gn
         td = self.tile_row_ptr.device
+        if td.type == "cuda":
+            self.desc = torch.empty((ntiles, 7), dtype=torch.int64, device=td)
+            g = SpGridOut(self.m, self.n, self.tm, self.tn, self.gm, self.gn, self.tile_row_ptr.data_ptr(),
+                          self.tile_offset.data_ptr(), self.col_ind.data_ptr(), self.vals.data_ptr(),
+                          _NP_TO_DT[self.dtype], 0)
+            call("bclx_spgrid_describe", context(self.device).use_current_stream(), ctypes.byref(g),
+                 ctypes.c_void_p(self.desc.data_ptr()))
+            self._offsets_host = None
+            return
         ti = torch.arange(self.gm, device=td).repeat_interleave(self.gn)
         tj = torch.arange(self.gn, device=td).repeat(self.gm)
-        d = torch.empty((ntiles, 6), dtype=torch.int64, device=td)
+        d = torch.empty((ntiles, 7), dtype=torch.int64, device=td)
         d[:, 0] = torch.clamp(self.m - ti * self.tm, max=self.tm)
         d[:, 1] = torch.clamp(self.n - tj * self.tn, max=self.tn)
         d[:, 2] = self.tile_offset[1:] - self.tile_offset[:-1]
         d[:, 3] = self.tile_row_ptr.data_ptr() + torch.arange(ntiles, device=td) * (self.tm + 1) * 4
         d[:, 4] = self.col_ind.data_ptr() + self.tile_offset[:-1] * 4
         d[:, 5] = self.vals.data_ptr() + self.tile_offset[:-1] * self.vals.element_size()
-        self.desc = torch.empty((ntiles, 7), dtype=torch.int64, device=td)
-        self.desc[:, :6] = d
-        self.desc[:, 6] = _NP_TO_DT[self.dtype]  # dtype (low 32 bits) and pad
-        self.desc = self.desc.contiguous()
+        d[:, 6] = _NP_TO_DT[self.dtype]  # dtype (low 32 bits) and pad
+        self.desc = d
         self._offsets_host = None
 
     # -- the reference's accessors
