@@ -3,7 +3,7 @@
 SpGEMM: the light-row bound of the row classification (a context knob, so
 each candidate runs the whole product), then the numeric pass's plan
 parameters (work items a warp takes from the device queue at a time, blocks
-per SM, the B-segment length from which a segment is walked lane-parallel),
+per SM, the B-segment length from which segments are walked one by one),
 grid-searched on one plan.  SpMM: rows per warp item, the long-row
 threshold, the long-row kernel's block count, the schedule of the
 long-row and short-row kernels and the order of column panels, by coordinate descent (one knob at a time, the
@@ -30,9 +30,9 @@ SPGEMM_LIGHT_UB = (128, 256, 512)
 CANDIDATES = {
     "grab": (1, 2, 4, 8),
     "blocks_per_sm": (3, 4),
-    "long_seg": (32, 48, 64, 1 << 30),
+    "long_seg": (6, 14, 28, 1 << 30),
 }
-DEFAULT = (1, 4, 64)
+DEFAULT = (1, 4, 14)
 SPMM_CANDIDATES = {
     "spmm_rows": (0, 1, 2, 4),
     "spmm_long_row": (0, 512, 1024, 2048),

@@ -662,7 +662,7 @@ def spgemm(a: SPMatrix, b: SPMatrix, stages: str = "fused", keep_plan: bool = Fa
     else:
         plan, out, trp, toff, nnz = spgemm_symbolic(a, b)
     if params:
-        plan.tune(params.get("grab", 1), params.get("blocks_per_sm", 4), params.get("long_seg", 64))
+        plan.tune(params.get("grab", 1), params.get("blocks_per_sm", 4), params.get("long_seg", 14))
     td = a.tile_row_ptr.device
     ci = torch.empty(max(nnz, 1), dtype=torch.int32, device=td)
     v = torch.empty(max(nnz, 1), dtype=_TORCH_OF[_NP_TO_DT[a.dtype]], device=td)

@@ -59,11 +59,11 @@ constexpr int kMaxCols = kMaxWords * 32;
 constexpr int kWarpsSym = 8;
 constexpr int kWarpsNum = 8;
 constexpr int kNoStage = 0xff;
-// B segments at least this long are walked in direct mode.  A shorter bound
-// ends more packed batches before they are full (a segment's products follow
-// those before it): R-MAT s16 numeric pass 3.54 ms with 32, 3.42 with 64, 3.44
-// with 96; R-MAT s18 37.0, 35.1 and 34.9.
-constexpr int kLongSegDefault = 64;
+// FP32 chunks whose B segments average fewer products are walked packed (see
+// walk_products).  Numeric pass with 1 (every chunk entry by entry), 6, 14, 28
+// and no bound: R-MAT s16 3.20, 2.92, 2.85, 2.88, 2.99 ms; R-MAT s18 34.0, 30.5,
+// 30.3, 30.4, 30.6; graph x sparse features 983, 492, 494, 502, 498 us.
+constexpr int kLongSegDefault = 14;
 constexpr int kQueueSlots = 256;          // work-queue heads in a plan (one per stage launch)
 constexpr int64_t kVeryHeavyUb = 32768;  // rows above this many products get a whole block in the symbolic pass
 
@@ -186,6 +186,13 @@ __device__ __forceinline__ int warp_search(int32_t incl, int32_t q) {
   return src;
 }
 
+// 1 << d, or 0 where d is negative or above 31 (the PTX shift clamps).
+__device__ __forceinline__ unsigned bit_or_none(int32_t d) {
+  unsigned r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(d));
+  return r;
+}
+
 template <typename P>
 __device__ __forceinline__ P* shfl_ptr(P* p, int src) {
   unsigned long long u = reinterpret_cast<unsigned long long>(p);
@@ -193,13 +200,14 @@ __device__ __forceinline__ P* shfl_ptr(P* p, int src) {
   return reinterpret_cast<P*>(u);
 }
 
-// Shared-memory table of one warp's walk: the entries of a packed run.
+// Shared-memory table of one warp's walk: the non-empty entries of a chunk.
 template <typename VT>
 struct WalkTable {
-  ulonglong2 seg[32];  // column and value addresses of product 0 of the run, as this entry's segment continues them
+  ulonglong2 seg[32];  // column and value addresses of the entry's segment (packed: of product 0 of the chunk,
+                       // as this segment continues them)
   struct {
     VT a;
-    int32_t stage;
+    uint32_t len_stage;  // segment length << 8 | stage
   } av[32];
 };
 
@@ -209,23 +217,26 @@ struct WalkTable {
 //
 // One lane per stage first reads that stage's A-row segment and B-tile
 // pointers.  The A entries of the row (all stages, flattened) are then taken
-// 32 at a time, one per lane, each finding its B segment.  An entry whose B
-// segment has at least long_seg products is walked in "direct" mode: lanes
-// stride over the segment and each lane calls fd(j, a, b, stage) for its own
-// products (the columns of one B row are distinct, so lanes never touch the
-// same column; a __syncwarp follows the segment).  Runs of shorter entries
-// are packed 32 products per batch and every lane calls f(valid, j, a, b,
-// stage, one) once per batch (warp-uniform); valid lanes form a prefix of the
-// warp and lane order is product order; `one`: the batch is 32 products of
-// one entry.  The loads of batch n+1 are issued before f runs on batch n.
+// 32 at a time (a chunk), one per lane, each finding its B segment; the
+// non-empty ones go to `tbl`, compacted.  The chunk's products are walked
+// in one of two ways:
+//  * entry by entry, 32 products of one segment at a time: the columns of one
+//    B row are distinct, so the lanes never touch the same column, and each
+//    calls fd(on, j, a, b, stage) for its own product;
+//  * packed 32 products per batch whatever entries they belong to: every lane
+//    calls f(on, j, a, b, stage, one) once per batch (warp-uniform); `on`
+//    lanes form a prefix of the warp and lane order is product order; `one`:
+//    the batch is 32 products of one entry.
+// Either way a __syncwarp follows and the next loads are issued before f or
+// fd runs.  A batch costs about four steps (finding each product's entry and
+// ordering equal columns: some 170 instructions against 40), so a chunk is
+// packed where its segments average fewer than long_seg products.
 //
-// The run's non-empty entries go to `tbl`, compacted, with their segment
-// addresses moved back by the entry's first product, so that product q is at
-// seg + q whatever its entry.  Which entry a lane's product belongs to is
-// the number of entries that begin at or before it: each entry sets the bit
-// of its first product in the batch, the bits are or-ed over the warp, and a
-// population count gives the entry (one warp reduction and one broadcast-like
-// 16-byte shared load in place of a five-step search and seven shuffles).
+// Packed, the table's addresses are moved back by the entry's first product,
+// so that product q is at seg + q whatever its entry.  Which entry a lane's
+// product belongs to is the number of entries that begin at or before it: each
+// entry sets the bit of its first product in the batch, the bits are or-ed
+// over the warp, and a population count gives the entry.
 template <typename VT, typename F, typename FD>
 __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridView& B, const Geom& g,
                                               const RowInfo& x, int s0, int s1, bool ranged, int fb_lo, int fb_hi,
@@ -241,6 +252,8 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
   const bool search = ranged && !table;
   int w0, w1;
   stage_window(g, x.ti, x.tj, s0, s1, w0, w1);
+  w0 = __reduce_max_sync(kFull, w0);
+  w1 = __reduce_max_sync(kFull, w1);
   for (int g0 = w0; g0 < w1; g0 += 32) {
     // one lane per stage: its A-row segment and its B tile
     const int si = g0 + lane;
@@ -265,7 +278,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       bva = reinterpret_cast<const VT*>(Bt.vals);
     }
     const int32_t aincl = warp_inclusive_scan(alen);
-    const int32_t atot = __shfl_sync(kFull, aincl, 31);
+    const int32_t atot = __reduce_add_sync(kFull, alen);
     const int32_t aexcl = aincl - alen;
     for (int32_t e0 = 0; e0 < atot; e0 += 32) {
       // one lane per A entry of the flattened stage stream
@@ -293,78 +306,77 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
         }
         len = be - bs;
       }
-      const int nent = min(32, atot - e0);
-      const unsigned longm = __ballot_sync(kFull, len >= long_seg);
-      int e_start = 0;
-      while (e_start < nent) {
-        const unsigned lm = longm & (kFull << e_start);
-        const int e_long = lm ? __ffs(lm) - 1 : nent;
-        const int32_t lenm = (lane >= e_start && lane < e_long) ? len : 0;
-        const unsigned full = __ballot_sync(kFull, lenm > 0);  // the run's non-empty entries
-        if (full) {
-          // packed batches over the short entries [e_start, e_long), software pipelined
-          const int32_t incl = warp_inclusive_scan(lenm);
-          const int32_t total = __shfl_sync(kFull, incl, 31);
-          const int32_t excl = incl - lenm;
-          if (lenm > 0) {
-            const int at = __popc(full & below);
-            tbl.seg[at] = make_ulonglong2(reinterpret_cast<unsigned long long>(sbci + bs) - 4ull * (unsigned)excl,
-                                          reinterpret_cast<unsigned long long>(sbva + bs) - 4ull * (unsigned)excl);
-            tbl.av[at].a = av;
-            tbl.av[at].stage = stage;
-          }
-          __syncwarp();
-          const int32_t begins = lenm > 0 ? excl : INT_MAX;  // this entry's first product
-          int ahead = -1;                                    // entries begun before the batch, less one
-          int32_t nj = -1;
-          VT na = VT(0), nb = VT(0);
-          int nst = 0;
-          bool none = false;
-          auto fetch = [&](int32_t base) {
-            const int32_t d = begins - base;
-            const unsigned heads = __reduce_or_sync(kFull, (unsigned)d < 32u ? 1u << d : 0u);
-            const int src = ahead + __popc(heads & upto);
-            ahead += __popc(heads);
-            none = (heads & ~1u) == 0u;  // no entry begins after the batch's first product
-            const int32_t q = base + lane;
-            const ulonglong2 sg = tbl.seg[src];
-            na = tbl.av[src].a;
-            nst = tbl.av[src].stage;
-            nj = -1;
-            nb = VT(0);
-            if (q < total) {
-              nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * (unsigned)q));
-              nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * (unsigned)q));
-            }
-          };
-          fetch(0);
-          for (int32_t base = 0; base < total; base += 32) {
-            const int32_t j = nj;
-            const VT a = na, b = nb;
-            const int st = nst;
-            const bool one = none && base + 32 <= total;
-            if (base + 32 < total) fetch(base + 32);
-            f(j >= 0, j, a, b, st, one);
-          }
+      const unsigned full = __ballot_sync(kFull, len > 0);
+      if (full == 0u) continue;
+      const int32_t total = __reduce_add_sync(kFull, len);
+      // (int32 sums need no order: a batch costs as little as a step)
+      const bool packed = !std::is_same<VT, float>::value || total < (int64_t)long_seg * __popc(full);
+      int32_t excl = 0;
+      if (packed) excl = warp_inclusive_scan(len) - len;
+      if (len > 0) {
+        const int at = __popc(full & below);
+        tbl.seg[at] = make_ulonglong2(reinterpret_cast<unsigned long long>(sbci + bs) - 4ull * (unsigned)excl,
+                                      reinterpret_cast<unsigned long long>(sbva + bs) - 4ull * (unsigned)excl);
+        tbl.av[at].a = av;
+        tbl.av[at].len_stage = (uint32_t)len << 8 | (uint32_t)stage;
+      }
+      __syncwarp();
+      // (straight-line loads: lanes past the end repeat the last product)
+      int32_t nj;
+      VT na, nb;
+      uint32_t nls;
+      if (packed) {
+        const int32_t begins = len > 0 ? excl : INT_MAX;  // this entry's first product
+        int ahead = -1;                                   // entries begun before the batch, less one
+        const uint32_t end = (uint32_t)total - 1u;
+        unsigned heads;
+        auto fetch = [&](int32_t base) {
+          heads = __reduce_or_sync(kFull, bit_or_none(begins - base));
+          const int src = ahead + __popc(heads & upto);
+          ahead += __popc(heads);
+          const uint32_t q = min((uint32_t)(base + lane), end);
+          const ulonglong2 sg = tbl.seg[src];
+          na = tbl.av[src].a;
+          nls = tbl.av[src].len_stage;
+          nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * q));
+          nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * q));
+        };
+        fetch(0);
+        for (int32_t base = 0; base < total; base += 32) {
+          const int32_t j = nj;
+          const VT a = na, b = nb;
+          const int st = (int)(nls & 255u);
+          const bool one = (heads & ~1u) == 0u && base + 32 <= total;  // no entry begins after the first product
+          if (base + 32 < total) fetch(base + 32);
+          f(base + lane < total, j, a, b, st, one);
         }
-        if (e_long < nent) {
-          // direct mode over one long segment
-          const int32_t dl = __shfl_sync(kFull, len, e_long);
-          const int32_t* dcol = shfl_ptr(sbci + bs, e_long);
-          const VT* dval = shfl_ptr(sbva + bs, e_long);
-          const VT da = __shfl_sync(kFull, av, e_long);
-          const int dst = __shfl_sync(kFull, stage, e_long);
-          int32_t q = lane;
-          for (; q + 32 < dl; q += 64) {
-            const int32_t j0 = __ldg(dcol + q), j1 = __ldg(dcol + q + 32);
-            const VT b0 = __ldg(dval + q), b1 = __ldg(dval + q + 32);
-            fd(j0, da, b0, dst);
-            fd(j1, da, b1, dst);
+      } else {
+        const int steps = __reduce_add_sync(kFull, (len + 31) >> 5);
+        int ent = 0;
+        uint32_t off = 0;  // the step's first product in its segment
+        auto fetch = [&]() {
+          const ulonglong2 sg = tbl.seg[ent];
+          na = tbl.av[ent].a;
+          nls = tbl.av[ent].len_stage;
+          const uint32_t q = min(off + (uint32_t)lane, (nls >> 8) - 1u);
+          nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * q));
+          nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * q));
+        };
+        fetch();
+        for (int i = 0; i < steps; i++) {
+          const int32_t j = nj;
+          const VT a = na, b = nb;
+          const int st = (int)(nls & 255u);
+          const bool on = off + (uint32_t)lane < (nls >> 8);
+          off += 32;
+          if (off >= (nls >> 8)) {
+            off = 0;
+            ent++;
           }
-          if (q < dl) fd(__ldg(dcol + q), da, __ldg(dval + q), dst);
+          if (i + 1 < steps) fetch();
+          fd(on, j, a, b, st);
           __syncwarp();
         }
-        e_start = e_long + 1;
       }
     }
   }
@@ -855,7 +867,8 @@ __global__ void k_tile_ptrs(Geom g, const int64_t* __restrict__ row_offset, int3
 // Heavy rows are cut at fine-block boundaries into items of <= vcap outputs
 // (greedy left to right; leading empty blocks are skipped).  One warp per
 // heavy row (blocks of 256 threads): lanes count the fine blocks' outputs
-// from the row's bitmap, lane 0 cuts.  FILL = false counts the items,
+// from the row's bitmap, lane 0 cuts.  The first n_half rows' items hold half
+// as many outputs (see half_rows).  FILL = false counts the items,
 // FILL = true writes them.
 struct HeavyItem {
   int32_t h;       // heavy slot
@@ -869,7 +882,7 @@ template <bool FILL>
 __global__ void __launch_bounds__(256)
     k_cut_heavy(Geom g, const int32_t* __restrict__ heavy_list, int n_heavy,
                 const uint32_t* __restrict__ heavy_bitmaps, int64_t hbm_words, int32_t* __restrict__ n_items,
-                const int64_t* __restrict__ first, HeavyItem* __restrict__ items, int vcap,
+                const int64_t* __restrict__ first, HeavyItem* __restrict__ items, int vcap_most, int n_half,
                 const int32_t* __restrict__ row_count = nullptr, const int16_t* __restrict__ span = nullptr) {
   __shared__ int32_t cnt_all[8][kMaxCols / kFineCols];
   int32_t* cnt = cnt_all[threadIdx.x >> 5];
@@ -881,6 +894,7 @@ __global__ void __launch_bounds__(256)
     const int64_t ri = heavy_list[h];
     const RowInfo x = decode_row(g, ri);
     const int nfb = (x.w + kFineCols - 1) / kFineCols;
+    const int vcap = h < n_half ? vcap_most / 2 : vcap_most;
     if (span && row_count) {
       // counted by the symbolic pass: a row whose outputs fit one item needs
       // no look at its bitmap; the item spans its first to its last block
@@ -967,12 +981,13 @@ struct WarpSmem {
 #define BCLX_NUMERIC_MIN_BLOCKS 4
 #endif
 // Bound by instruction issue (67 % of the slots) and the shared-memory pipe
-// (68 %), not by DRAM.  Packed entry table, columns staged in shared memory,
-// prefix counts 8 words per lane, 32-bit divisions, int32 without an order:
-// R-MAT s16 on 8x8 tiles 3.84 -> 3.42 ms per launch, s18 on 16x16 39.3 -> 35.1
-// ms; R-MAT of 30,011 rows in int32 0.96 -> 0.42 ms; the 27-point stencil
-// on 128^3, whose rows are one item each (walked by the B rows' own bounds
-// instead of two binary searches per A entry), 37.6 -> 29.1 ms.
+// (66 %), not by DRAM: at R-MAT s16 2.3e9 warp instructions, of which an item's
+// set-up and output 27 %, the A-entry walk 13 %, the products the rest.
+// Per launch, before this walk -> now: R-MAT s16 on 8x8 tiles 3.84 -> 2.85 ms,
+// s18 on 16x16 39.3 -> 30.3; R-MAT of 30,011 rows in int32 0.96 -> 0.37; graph x
+// sparse features 0.69 -> 0.39; the 27-point stencil on 128^3, whose rows are
+// one item each (walked by the B rows' own bounds instead of two binary
+// searches per A entry), 37.6 -> 24.8.
 // LEARNED: the learned product's single pass.  Heavy items come from the
 // predicted cut (their counts are unknown): each builds its bitmap from its
 // own products, and an item with more than kVcap outputs marks its row in
@@ -998,17 +1013,17 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
   const int lane = lane_id();
   const int64_t n_total = n_heavy_items + n_light;
   // persistent warps: take `grab` consecutive items at a time from the queue
-  int64_t next = 0, stop = 0;
+  uint32_t next = 0, stop = 0;
   for (;;) {
     if (next >= stop) {
-      unsigned long long b = 0;
-      if (lane == 0) b = atomicAdd(queue, (unsigned long long)grab);
-      b = __shfl_sync(kFull, b, 0);
-      if ((int64_t)b >= n_total) break;
-      next = (int64_t)b;
-      stop = min((int64_t)b + grab, n_total);
+      uint32_t b = 0;
+      if (lane == 0) b = (uint32_t)min(atomicAdd(queue, (unsigned long long)grab), (unsigned long long)n_total);
+      b = __reduce_max_sync(kFull, b);
+      if ((int64_t)b >= n_total) break;  // (items are fewer than rows plus outputs / 256: below 2^32)
+      next = b;
+      stop = min(b + (uint32_t)grab, (uint32_t)n_total);
     }
-    const int64_t idx = next++;
+    const uint32_t idx = next++;
     // heavy items first (they are the larger ones)
     const bool heavy = idx < n_heavy_items;
     int64_t ri;
@@ -1167,43 +1182,41 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
       const int xx = j - lo;
       return (int)S.pre[xx >> 5] + __popc(S.bm[xx >> 5] & ((1u << (xx & 31)) - 1u));
     };
-    auto apply = [&](int rank, VT a, VT b, int stage) {
+    // one product per lane where `on`, straight-line: every lane reads its
+    // column's slots and the stores alone are conditional
+    auto apply = [&](bool on, int rank, VT a, VT b, int stage) {
       if constexpr (kOrdered) {
-        VT v = S.part[rank];
+        const VT v = S.part[rank];
         const int t = S.tag[rank];
-        if (t != stage) {
-          if (t != kNoStage) S.acc[rank] = vadd(S.acc[rank], v);
-          v = VT(0);
-          S.tag[rank] = (unsigned char)stage;
-        }
-        S.part[rank] = madd(a, b, v);
+        const bool next = on && t != stage;  // first product of this stage
+        const bool fold = next && t != kNoStage;
+        const VT ac = S.acc[rank];
+        if (on) S.part[rank] = madd(a, b, t != stage ? VT(0) : v);
+        if (next) S.tag[rank] = (unsigned char)stage;
+        if (fold) S.acc[rank] = vadd(ac, v);
       } else {
-        atomicAdd(reinterpret_cast<unsigned*>(&S.acc[rank]), (unsigned)a * (unsigned)b);
+        if (on) atomicAdd(reinterpret_cast<unsigned*>(&S.acc[rank]), (unsigned)a * (unsigned)b);
       }
     };
     auto update = [&](bool valid, int32_t j, VT a, VT b, int stage, bool one) {
-      const int rank = valid ? rank_of(j) : 0;
-      if constexpr (kOrdered) {
+      const int rank = rank_of(j);
+      if (!kOrdered || one) {
+        apply(valid, rank, a, b, stage);
+      } else {
         // products of one column in a batch go one after another, in lane
         // order: a lane's turn is the number of lower lanes with its column
-        const unsigned peers = one ? 0u : __match_any_sync(kFull, valid ? j : ~lane) & ((1u << lane) - 1u);
-        if (one || !__any_sync(kFull, peers != 0u)) {
-          if (valid) apply(rank, a, b, stage);
-        } else {
-          const int turn = __popc(peers), last = __reduce_max_sync(kFull, turn);
-          for (int t = 0; t <= last; t++) {
-            if (valid && t == turn) apply(rank, a, b, stage);
-            __syncwarp();
-          }
+        const int turn = __popc(__match_any_sync(kFull, valid ? j : ~lane) & ((1u << lane) - 1u));
+        const int last = __reduce_max_sync(kFull, turn);
+        apply(valid && turn == 0, rank, a, b, stage);
+        for (int t = 1; t <= last; t++) {
+          __syncwarp();
+          apply(valid && turn == t, rank, a, b, stage);
         }
-        __syncwarp();
-      } else {
-        if (valid) apply(rank, a, b, stage);
-        __syncwarp();
       }
+      __syncwarp();
     };
-    // direct mode: the lanes hold distinct columns, each updates its own
-    auto update_direct = [&](int32_t j, VT a, VT b, int stage) { apply(rank_of(j), a, b, stage); };
+    // entry by entry: the lanes hold distinct columns, each updates its own
+    auto update_direct = [&](bool on, int32_t j, VT a, VT b, int stage) { apply(on, rank_of(j), a, b, stage); };
     // An item that holds all of its row's outputs takes every product of the
     // row: the B rows' own bounds serve, without the table or a search.
     const bool ranged = heavy && (LEARNED ? (fb_lo > 0 || fb_hi * kFineCols < x.w) : !whole);
@@ -1770,6 +1783,16 @@ static int build_btable(Context* ctx, const SpGridView& B, const Geom& g, bclx_s
   return BCLX_OK;
 }
 
+// Very heavy rows whose items hold half as many outputs: all of them where
+// there are no more than SMs.  An item is one warp's serial walk, and such a
+// product's numeric pass ends with the longest (graph x sparse features, 17
+// very heavy rows: 503 us with whole items, 394 with half; R-MAT s16, 1,108 of
+// them: 2.85 ms with whole items, 3.05 with half, as each item walks its
+// row's A entries again).
+static int half_rows(const Context* ctx, const bclx_spgemm_plan_s* P) {
+  return P->n_vheavy <= ctx->num_sms ? (int)P->n_vheavy : 0;
+}
+
 // Classification, symbolic, row offsets and the heavy-row cut.
 static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B, Geom g, int dtype,
                          int32_t* tile_row_ptr, int64_t* tile_offset, bclx_spgemm_plan_s* P) {
@@ -1845,7 +1868,7 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     const unsigned blocks = grid_for(ctx, P->n_heavy, 8, 8);
     k_cut_heavy<false><<<blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
                                                         P->hbm_words, P->heavy_nitems, nullptr, nullptr, P->vcap,
-                                                        P->row_count, P->heavy_span);
+                                                        half_rows(ctx, P), P->row_count, P->heavy_span);
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -1865,7 +1888,7 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     const unsigned blocks = grid_for(ctx, P->n_heavy, 8, 8);
     k_cut_heavy<true><<<blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
                                                        P->hbm_words, nullptr, P->heavy_first, P->heavy_items, P->vcap,
-                                                       P->row_count, P->heavy_span);
+                                                       half_rows(ctx, P), P->row_count, P->heavy_span);
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -2282,7 +2305,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
   BCLX_CK_LAUNCH();
   if (P.n_heavy > 0) {
     k_cut_heavy<false><<<grid_for(ctx, P.n_heavy, 8, 8), 256, 0, ctx->stream>>>(
-        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, P.heavy_nitems, nullptr, nullptr, P.vcap);
+        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, P.heavy_nitems, nullptr, nullptr, P.vcap, 0);
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -2317,7 +2340,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
     if (probe.ok) ar = probe;
     else P.tab = nullptr;
     k_cut_heavy<true><<<grid_for(ctx, P.n_heavy, 8, 8), 256, 0, ctx->stream>>>(
-        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, nullptr, P.heavy_first, P.heavy_items, P.vcap);
+        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, nullptr, P.heavy_first, P.heavy_items, P.vcap, 0);
     note_launch();
     BCLX_CK_LAUNCH();
     if (P.tab && g.tk > 0) {
@@ -2571,7 +2594,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->row_offset = P->redo_off;  // borrowed
     const unsigned rb = grid_for(ctx, nf, 8, 8);
     k_cut_heavy<false><<<rb, 256, 0, ctx->stream>>>(g, R->heavy_list, nf, R->heavy_bitmaps, R->hbm_words,
-                                                    R->heavy_nitems, nullptr, nullptr, R->vcap);
+                                                    R->heavy_nitems, nullptr, nullptr, R->vcap, 0);
     note_launch();
     BCLX_CK_LAUNCH();
     BCLX_TRY(exclusive_scan_i32(ctx, R->heavy_nitems, R->heavy_first, nf));
@@ -2582,7 +2605,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->n_heavy_items = rt[0];
     BCLX_TRY(scratch_alloc_n(ctx, &R->heavy_items, R->n_heavy_items));
     k_cut_heavy<true><<<rb, 256, 0, ctx->stream>>>(g, R->heavy_list, nf, R->heavy_bitmaps, R->hbm_words, nullptr,
-                                                   R->heavy_first, R->heavy_items, R->vcap);
+                                                   R->heavy_first, R->heavy_items, R->vcap, 0);
     note_launch();
     BCLX_CK_LAUNCH();
     R->tab = P->tab;  // borrowed

@@ -1,5 +1,5 @@
 """The numeric pass's product walk at the lengths where it can go wrong:
-B segments around one batch (32 products) and around the direct-mode bound,
+B segments around one batch (32 products), chunks on either side of the packed bound,
 empty segments between them, columns shared by neighbouring segments, tiles
 whose width is no whole number of 256-column blocks, and heavy rows that are
 one item (walked by the B rows' own bounds) or several.  Exact arithmetic
@@ -75,10 +75,31 @@ def test_walk_vs_oracle(n, span, tiles, value_type, mode):
     assert_csr_identical(spgemm(A, B, stages=mode).get(), rp, ci, cv)
 
 
-@pytest.mark.parametrize("long_seg", [1, 32, 33, 64, 1 << 20])
-def test_direct_mode_bound_does_not_change_results(long_seg):
+@pytest.mark.parametrize("long_seg", [1, 8, 14, 33, 1 << 20])
+def test_packed_bound_does_not_change_results(long_seg):
     from bcl_b200.containers import BlockCustom, SPMatrix, spgemm
     a, b = _operands(1000, 700, "f32", 5)
     A, B = SPMatrix.from_csr(a, BlockCustom((64, 40))), SPMatrix.from_csr(b, BlockCustom((40, 1000)))
     rp, ci, cv = O.gemm_tiled(a, b, 64, 40, 1000)
     assert_csr_identical(spgemm(A, B, tuning=(1, 4, long_seg)).get(), rp, ci, cv)
+
+
+@pytest.mark.parametrize("value_type", ["f32", "i32"])
+@pytest.mark.parametrize("n,tile", [(3001, 3001), (2900, 700)])
+def test_few_very_heavy_rows_cut_finer(n, tile, value_type):
+    """Two rows of 32768 products or more (items of half as many outputs), one
+    just below, among light ones."""
+    from bcl_b200.containers import BlockCustom, SPMatrix, spgemm
+    rng = np.random.default_rng(n)
+    k, per = 900, 64 * (n // tile + 1)
+
+    def vals(count):
+        return (rng.uniform(-1, 1, count).astype(np.float32) if value_type == "f32"
+                else rng.integers(-99, 99, count).astype(np.int32))
+
+    b = _csr(k, n, [np.sort(rng.choice(n, per, replace=False)) for _ in range(k)], vals)
+    lens = [3] * 20 + [900, 600, 500] + [7] * 20
+    a = _csr(len(lens), k, [np.sort(rng.choice(k, c, replace=False)) for c in lens], vals)
+    A, B = SPMatrix.from_csr(a, BlockCustom((16, 300))), SPMatrix.from_csr(b, BlockCustom((300, tile)))
+    rp, ci, cv = O.gemm_tiled(a, b, 16, 300, tile, mode=value_type)
+    assert_csr_identical(spgemm(A, B).get(), rp, ci, cv)
