@@ -64,7 +64,8 @@ constexpr int kNoStage = 0xff;
 // and no bound: R-MAT s16 3.20, 2.92, 2.85, 2.88, 2.99 ms; R-MAT s18 34.0, 30.5,
 // 30.3, 30.4, 30.6; graph x sparse features 983, 492, 494, 502, 498 us.
 constexpr int kLongSegDefault = 14;
-constexpr int kQueueSlots = 256;          // work-queue heads in a plan (one per stage launch)
+constexpr int kQueueSlots = 256;          // work-queue heads in a plan: one per stage launch (at most 254), and
+constexpr int kClassifySlot = 254, kSymbolicSlot = 255;  // the planning passes' (each used once)
 constexpr int64_t kVeryHeavyUb = 32768;  // rows above this many products get a whole block in the symbolic pass
 
 constexpr int kBlockWords = kFineCols / 32;  // bitmap words of a fine block
@@ -383,103 +384,86 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
 }
 
 // Order-free walk for the symbolic pass: calls fs(j) for every product
-// column of C-tile row `x` (all stages).  Short B segments are looped over by
-// their own lane, long ones by the whole warp.  With nparts walkers (the warps
-// of a block): when the row has at least 2 * nparts chunks of 32 A entries,
-// each walker takes every nparts-th chunk whole (short and long segments);
-// otherwise every walker reads every chunk and takes every nparts-th chunk of
-// short segments and an interleaved share of every long segment.
+// column of C-tile row `x` (all stages), packed 32 products per batch as in
+// walk_products (`tbl`: 32 entries of shared memory of this warp), four
+// batches' loads in flight.  With nparts walkers (the warps of a block): when
+// the row has at least 2 * nparts chunks of 32 A entries, each walker takes
+// every nparts-th chunk whole; otherwise every walker reads every chunk and
+// takes every nparts-th batch.
 template <typename FS>
 __device__ __forceinline__ void walk_columns(const SpGridView& A, const SpGridView& B, const Geom& g,
-                                             const RowInfo& x, int part, int nparts, FS&& fs) {
+                                             const RowInfo& x, int part, int nparts, unsigned long long* tbl, FS&& fs) {
+  constexpr int kAhead = 4;
   const int lane = lane_id();
+  const unsigned below = (1u << lane) - 1u, upto = below | (1u << lane);
   const int ns = stage_count(g, x.ti, x.tj);
   for (int g0 = 0; g0 < ns; g0 += 32) {
     const int si = g0 + lane;
-    int32_t as = 0, alen = 0;
+    int32_t alen = 0;
     const int32_t* acol = nullptr;
     const int32_t* brp = nullptr;
     const int32_t* bci = nullptr;
     if (si < ns) {
       const int64_t k = stage_k(g, stage_at(g, x.ti, x.tj, si), x.rot);
       const bclx_csr_t At = A.tile(x.ti, k);
-      as = __ldg(At.row_ptr + x.r);
+      const int32_t as = __ldg(At.row_ptr + x.r);
       alen = __ldg(At.row_ptr + x.r + 1) - as;
-      acol = At.col_ind;
+      acol = At.col_ind + as;
       const bclx_csr_t Bt = B.tile(k, x.tj);
       brp = Bt.row_ptr;
       bci = Bt.col_ind;
     }
     const int32_t aincl = warp_inclusive_scan(alen);
-    const int32_t atot = __shfl_sync(kFull, aincl, 31);
+    const int32_t atot = __reduce_add_sync(kFull, alen);
     const int32_t aexcl = aincl - alen;
-    // chunk x's A column (one entry per lane) and its B tile, loaded one
-    // chunk ahead so the column load of the next chunk is in flight while
-    // the current chunk's B rows are read
-    struct Ent {
-      int32_t kc;
-      const int32_t* brp;
-      const int32_t* bci;
-    };
-    auto load_ent = [&](int32_t e0) {
-      Ent t{0, nullptr, nullptr};
-      const int32_t e = e0 + lane;
-      const int sl = warp_search(aincl, e);
-      const int32_t sas = __shfl_sync(kFull, as, sl);
-      const int32_t sax = __shfl_sync(kFull, aexcl, sl);
-      const int32_t* sacol = shfl_ptr(acol, sl);
-      t.brp = shfl_ptr(brp, sl);
-      t.bci = shfl_ptr(bci, sl);
-      if (e < atot) t.kc = __ldg(sacol + sas + (e - sax));
-      return t;
-    };
     // whole chunks per walker, or every chunk read by every walker
     const bool own = nparts > 1 && atot >= 64 * nparts;
     const int32_t first = own ? 32 * part : 0;
     const int32_t stride = own ? 32 * nparts : 32;
-    const int wpart = own ? 0 : part;  // this walker's share within a chunk
-    const int wparts = own ? 1 : nparts;
-    Ent nxt = first < atot ? load_ent(first) : Ent{0, nullptr, nullptr};
-    for (int32_t e0 = first, chunk = 0; e0 < atot; e0 += stride, chunk++) {
-      const Ent cur = nxt;
+    const int32_t b_first = own ? 0 : 32 * part;  // this walker's batches within a chunk
+    const int32_t b_step = own ? 32 : 32 * nparts;
+    // a chunk's A columns (one entry per lane) are loaded one chunk ahead
+    int nsl = 0;
+    int32_t nkc = 0;
+    auto fetch_a = [&](int32_t e0) {
       const int32_t e = e0 + lane;
-      if (e0 + stride < atot) nxt = load_ent(e0 + stride);
-      const int32_t* sbci = cur.bci;
-      int32_t bs = 0, be = 0;
-      if (e < atot) {
-        bs = __ldg(cur.brp + cur.kc);
-        be = __ldg(cur.brp + cur.kc + 1);
+      nsl = warp_search(aincl, e);
+      const int32_t off = e - __shfl_sync(kFull, aexcl, nsl);
+      const int32_t* sacol = shfl_ptr(acol, nsl);
+      if (e < atot) nkc = __ldg(sacol + off);
+    };
+    if (first < atot) fetch_a(first);
+    for (int32_t e0 = first; e0 < atot; e0 += stride) {
+      const int32_t* sbrp = shfl_ptr(brp, nsl);
+      const int32_t* sbci = shfl_ptr(bci, nsl);
+      int32_t len = 0;
+      if (e0 + lane < atot) {
+        const int32_t bs = __ldg(sbrp + nkc);
+        len = __ldg(sbrp + nkc + 1) - bs;
+        sbci += bs;
       }
-      const bool lng = be - bs >= 32;
-      if (!lng && chunk % wparts == wpart) {
-        int32_t q = bs;
-        for (; q + 4 <= be; q += 4) {  // four column loads in flight
-          const int32_t j0 = __ldg(sbci + q), j1 = __ldg(sbci + q + 1);
-          const int32_t j2 = __ldg(sbci + q + 2), j3 = __ldg(sbci + q + 3);
-          fs(j0);
-          fs(j1);
-          fs(j2);
-          fs(j3);
+      if (e0 + stride < atot) fetch_a(e0 + stride);
+      const unsigned full = __ballot_sync(kFull, len > 0);
+      if (full == 0u) continue;
+      const int32_t total = __reduce_add_sync(kFull, len);
+      const int32_t excl = warp_inclusive_scan(len) - len;
+      __syncwarp();
+      if (len > 0) tbl[__popc(full & below)] = reinterpret_cast<unsigned long long>(sbci) - 4ull * (unsigned)excl;
+      __syncwarp();
+      const int32_t begins = len > 0 ? excl : INT_MAX;
+      for (int32_t base = b_first; base < total; base += kAhead * b_step) {
+        int32_t j[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+          const int32_t b = base + u * b_step;
+          const int ahead = __popc(__ballot_sync(kFull, begins < b)) - 1;  // entries begun before the batch, less one
+          const unsigned heads = __reduce_or_sync(kFull, bit_or_none(begins - b));
+          const uint32_t q = min((uint32_t)(b + lane), (uint32_t)total - 1u);
+          j[u] = __ldg(reinterpret_cast<const int32_t*>(tbl[min(ahead + __popc(heads & upto), 31)] + 4ull * q));
         }
-        for (; q < be; q++) fs(__ldg(sbci + q));
-      }
-      unsigned longm = __ballot_sync(kFull, lng);
-      while (longm) {
-        const int src = __ffs(longm) - 1;
-        longm &= longm - 1;
-        const int32_t lb = __shfl_sync(kFull, bs, src), le = __shfl_sync(kFull, be, src);
-        const int32_t* lci = shfl_ptr(sbci, src);
-        const int32_t step = 32 * wparts;
-        int32_t q = lb + lane + 32 * wpart;
-        for (; q + 3 * step < le; q += 4 * step) {
-          const int32_t j0 = __ldg(lci + q), j1 = __ldg(lci + q + step);
-          const int32_t j2 = __ldg(lci + q + 2 * step), j3 = __ldg(lci + q + 3 * step);
-          fs(j0);
-          fs(j1);
-          fs(j2);
-          fs(j3);
-        }
-        for (; q < le; q += step) fs(__ldg(lci + q));
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+          if (base + u * b_step + lane < total) fs(j[u]);
       }
     }
   }
@@ -698,25 +682,199 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
   if (lane == 0 && mine) atomicAdd(products, mine);
 }
 
+// Products of every row for all of its C tiles at once, where no stage map
+// is in use (coarse grids): a warp takes a row of A's tile row ti, reads its
+// entries once, and for each tile column j adds up the lengths of the B_kj
+// rows they name; lane j holds the row's products in C tile (ti, j).  Taking
+// each C tile's row by itself (k_classify) reads the entries once per tile
+// column (438 instructions a row item): R-MAT s16 on 8x8 tiles 283 -> 235 us,
+// s18 on 16x16 1.88 -> 1.33 ms, R-MAT of 30,011 rows on 5x5 112 -> 48 us.  The
+// items of several rows go to the lists together, one atomic per list.
+// A row of more than kClassifyLong entries is taken by the whole block after
+// its other rows, its chunks dealt to the warps (a hub row is hundreds of
+// chunks of dependent loads); neighbouring rows, which hubs are, go to
+// different blocks.
+constexpr int kClassifyKeep = 8;    // rows whose items a warp keeps before it appends them
+constexpr int kClassifyCols = 8;    // tile columns whose loads are in flight
+constexpr int kClassifyLong = 512;
+constexpr int kClassifyDefer = 64;  // long rows a block can put off
+__global__ void __launch_bounds__(256) k_classify_rows(
+    SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
+    int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
+    int heavy_min_cols, int light_ub) {
+  __shared__ int32_t kept_all[8][3][kClassifyKeep * 32];
+  __shared__ unsigned long long sums[32];
+  __shared__ uint32_t deferred[kClassifyDefer];
+  __shared__ int n_deferred;
+  const int wid = threadIdx.x >> 5;
+  int32_t(*kept)[kClassifyKeep * 32] = kept_all[wid];
+  int32_t* const lists[3] = {light_list, heavy_list, vheavy_list};
+  const int lane = lane_id();
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t n_rows = (uint32_t)(g.gm * g.tm), tm = (uint32_t)g.tm;
+  const int gk = (int)g.gk, gn = (int)g.gn;
+  const uint32_t warp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * 8;
+  unsigned long long mine = 0;
+  int n_kept[3] = {0, 0, 0};
+  int rows = 0;
+  auto append = [&]() {
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (n_kept[c] == 0) continue;
+      int pos = 0;
+      if (lane == 0) pos = atomicAdd(&counters[c == 2 ? 3 : c], n_kept[c]);
+      pos = __shfl_sync(kFull, pos, 0);
+      for (int q = lane; q < n_kept[c]; q += 32) lists[c][pos + q] = kept[c][q];
+      n_kept[c] = 0;
+    }
+    rows = 0;
+    __syncwarp();
+  };
+  // lane's products in tile column j0 + lane: keep the row item in its class
+  auto keep = [&](uint32_t ti, uint32_t r, int j, int64_t tot) {
+    mine += (unsigned long long)tot;
+    int cls = -1;
+    if (tot > 0) {
+      const int64_t w = min(g.n - (int64_t)j * g.tn, g.tn);
+      cls = tot <= light_ub && w < heavy_min_cols ? 0 : (tot <= kVeryHeavyUb ? 1 : 2);
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const unsigned m = __ballot_sync(kFull, cls == c);
+      if (cls == c) kept[c][n_kept[c] + __popc(m & below)] = (int32_t)((ti * (uint32_t)gn + (uint32_t)j) * tm + r);
+      n_kept[c] += __popc(m);
+    }
+    if (++rows == kClassifyKeep) append();
+  };
+  // the products of row (ti, r), its chunks part, part + parts, ...; long rows
+  // (of all parts) are left out with -1 where `put_off`
+  auto count = [&](uint32_t ti, uint32_t r, int j0, int j1, int part, int parts, bool put_off) -> int64_t {
+    int64_t tot = 0;
+    for (int g0 = 0; g0 < gk; g0 += 32) {
+      // one lane per A tile: its segment of the row
+      int32_t alen = 0;
+      const int32_t* acol = nullptr;
+      if (g0 + lane < gk) {
+        const bclx_csr_t At = A.tile(ti, g0 + lane);
+        const int32_t as = __ldg(At.row_ptr + r);
+        alen = __ldg(At.row_ptr + r + 1) - as;
+        acol = At.col_ind + as;
+      }
+      const int32_t atot = __reduce_add_sync(kFull, alen);
+      if (put_off && g0 == 0 && atot > kClassifyLong) return -1;
+      if (atot == 0) continue;
+      const int32_t aincl = warp_inclusive_scan(alen);
+      const int32_t aexcl = aincl - alen;
+      for (int32_t e0 = 32 * part; e0 < atot; e0 += 32 * parts) {
+        const int32_t e = e0 + lane;
+        const int sl = warp_search(aincl, e);
+        const int32_t off = e - __shfl_sync(kFull, aexcl, sl);
+        const int32_t* sacol = shfl_ptr(acol, sl);
+        const int32_t kc = e < atot ? __ldg(sacol + off) : -1;
+        for (int j = j0; j < j1; j += kClassifyCols) {
+          uint32_t len[kClassifyCols];
+#pragma unroll
+          for (int q = 0; q < kClassifyCols; q++) {
+            len[q] = 0;
+            if (kc >= 0 && j + q < j1) {
+              const int32_t* brp = B.tile(g0 + sl, j + q).row_ptr;
+              len[q] = (uint32_t)(__ldg(brp + kc + 1) - __ldg(brp + kc));
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kClassifyCols; q++) {
+            const uint32_t sum = __reduce_add_sync(kFull, len[q]);
+            if (lane == j + q - j0) tot += sum;
+          }
+        }
+      }
+    }
+    return tot;
+  };
+  for (int j0 = 0; j0 < gn; j0 += 32) {  // (tile columns 32 at a time, one per lane)
+    const int j1 = min(gn, j0 + 32);
+    if (threadIdx.x == 0) n_deferred = 0;
+    if (threadIdx.x < 32) sums[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint32_t it = warp; it < n_rows; it += nwarps) {
+      const uint32_t ti = it / tm, r = it - ti * tm;
+      if ((int64_t)r >= A.rows_of(ti)) continue;
+      int64_t tot = count(ti, r, j0, j1, 0, 1, true);
+      if (tot < 0) {
+        int at = 0;
+        if (lane == 0) at = atomicAdd(&n_deferred, 1);
+        at = __shfl_sync(kFull, at, 0);
+        if (at < kClassifyDefer) {
+          if (lane == 0) deferred[at] = it;
+          continue;
+        }
+        tot = count(ti, r, j0, j1, 0, 1, false);
+      }
+      keep(ti, r, j0 + lane, tot);
+    }
+    __syncthreads();
+    const int n = min(n_deferred, kClassifyDefer);
+    for (int d = 0; d < n; d++) {
+      const uint32_t ti = deferred[d] / tm, r = deferred[d] - ti * tm;
+      const int64_t part = count(ti, r, j0, j1, wid, 8, false);
+      if (part) atomicAdd(&sums[lane], (unsigned long long)part);
+      __syncthreads();
+      if (wid == 0) {
+        keep(ti, r, j0 + lane, (int64_t)sums[lane]);
+        sums[lane] = 0;
+      }
+      __syncthreads();
+    }
+    append();
+  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) mine += __shfl_xor_sync(kFull, mine, d);
+  if (lane == 0 && mine) atomicAdd(products, mine);
+}
+
 // B-row table: for every row of every B tile (k, j), the position of the
 // first entry in each fine column block: tab[((k*gn + j)*tk + r)*(nfb+1) + b]
 // = first entry with column >= b*kFineCols (b = nfb: the row end).
-// One thread per B row (rows of a tile are short on average).
-__global__ void k_btable(SpGridView B, Geom g, int32_t* __restrict__ tab) {
+// One thread per B row (rows of a tile are short on average; a long one is
+// searched), its line in shared memory, and the block's lines written out
+// together: stored one by one they were as many L2 writes (R-MAT s16 on 8x8
+// tiles, 69 MB: 413 -> 210 us beside the symbolic pass; s18 on 16x16, 1.09 GB:
+// 3.0 -> 1.0 ms).
+constexpr int kBtableRows = 128;  // rows (threads) of a block
+__global__ void __launch_bounds__(kBtableRows) k_btable(SpGridView B, Geom g, int32_t* __restrict__ tab) {
+  __shared__ int32_t line[kBtableRows * (kMaxCols / kFineCols + 1)];
   const int64_t nrows = g.gk * g.gn * g.tk;
-  for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < nrows; x += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t kt = x / g.tk, r = x - kt * g.tk;
-    const int64_t k = kt / g.gn, j = kt - k * g.gn;
-    const bclx_csr_t Bt = B.tile(k, j);
-    if (r >= Bt.m) continue;  // the tile's own row count (sub-grids may reorder B's tiles)
-    int32_t* trow = tab + x * (g.nfb + 1);
-    const int32_t b0 = __ldg(Bt.row_ptr + r), b1 = __ldg(Bt.row_ptr + r + 1);
-    int b = 0;
-    for (int32_t q = b0; q < b1; q++) {
-      const int blk = __ldg(Bt.col_ind + q) / kFineCols;
-      while (b <= blk) trow[b++] = q;
+  const int nfb = (int)g.nfb, width = nfb + 1;
+  for (int64_t x0 = (int64_t)blockIdx.x * kBtableRows; x0 < nrows; x0 += (int64_t)gridDim.x * kBtableRows) {
+    const int64_t x = x0 + threadIdx.x;
+    int32_t* mine = line + threadIdx.x * width;
+    int32_t b0 = 0, b1 = 0;
+    const int32_t* ci = nullptr;
+    if (x < nrows) {
+      const int64_t kt = x / g.tk, r = x - kt * g.tk;
+      const bclx_csr_t Bt = B.tile(kt / g.gn, kt % g.gn);
+      if (r < Bt.m) {  // the tile's own row count (sub-grids may reorder B's tiles)
+        b0 = __ldg(Bt.row_ptr + r);
+        b1 = __ldg(Bt.row_ptr + r + 1);
+        ci = Bt.col_ind;
+      }
     }
-    while (b <= g.nfb) trow[b++] = b1;
+    int b = 0;
+    if (b1 - b0 <= 2 * nfb) {
+      for (int32_t q = b0; q < b1; q++) {
+        const int blk = __ldg(ci + q) / kFineCols;
+        while (b <= blk) mine[b++] = q;
+      }
+    } else {
+      int32_t q = b0;
+      for (; b < nfb; b++) mine[b] = q = lower_bound_i32(ci, q, b1, b * kFineCols);
+    }
+    while (b <= nfb) mine[b++] = b1;
+    __syncthreads();
+    const int n = (int)min((int64_t)kBtableRows, nrows - x0) * width;
+    for (int i = threadIdx.x; i < n; i += kBtableRows) tab[x0 * width + i] = line[i];
+    __syncthreads();
   }
 }
 
@@ -734,14 +892,19 @@ __global__ void k_btable(SpGridView B, Geom g, int32_t* __restrict__ tab) {
 // One warp per row for the light and ordinary heavy rows (heavy first),
 // rows taken from a device counter (each warp grabs its next row while it
 // walks the current one) ...
-// Four blocks per SM: 64 registers without spills (R-MAT s16: 5.50-5.52 ms
-// per product against 5.52-5.54 with 48 registers and spills, 5.66 with 40).
+// Bound by the latency of the dependent loads and by issue.  Short segments
+// walked by their own lane, 32 products cost some 40 instructions; packed, 20:
+// R-MAT s16 938 -> 787 us (beside the B-row table and the very heavy rows), s18
+// 8.1 -> 6.4 ms, R-MAT of 30,011 rows 350 -> 218 us; the 27-point stencil, 143
+// products a row item, 7.3 -> 7.9 ms.  Four blocks per SM: 64 registers (with
+// fewer the walk spills).
 __global__ void __launch_bounds__(kWarpsSym * 32, 4)
     k_symbolic(SpGridView A, SpGridView B, Geom g, const int32_t* __restrict__ light_list,
                const int32_t* __restrict__ heavy_list, int n_light, int n_heavy, int n_vheavy,
                int32_t* __restrict__ row_count, uint32_t* __restrict__ heavy_bitmaps, int64_t hbm_words,
                int16_t* __restrict__ heavy_span, unsigned long long* __restrict__ queue, int grab) {
   __shared__ __align__(16) uint32_t bm_all[kWarpsSym][kMaxWords];
+  __shared__ unsigned long long tbl_all[kWarpsSym][32];
   uint32_t* bm = bm_all[threadIdx.x >> 5];
   const int lane = lane_id();
   const unsigned long long n_items = (unsigned long long)((int64_t)n_light + n_heavy - n_vheavy);
@@ -760,7 +923,8 @@ __global__ void __launch_bounds__(kWarpsSym * 32, 4)
     const int words = block_words(x.w);
     for (int w = lane * 4; w < words; w += 128) *reinterpret_cast<uint4*>(bm + w) = make_uint4(0u, 0u, 0u, 0u);
     __syncwarp();
-    walk_columns(A, B, g, x, 0, 1, [&](int32_t j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
+    walk_columns(A, B, g, x, 0, 1, tbl_all[threadIdx.x >> 5],
+                 [&](int32_t j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
     __syncwarp();
     int cnt = 0, b0 = INT_MAX, b1 = 0;  // fine blocks with outputs: [b0, b1)
     for (int w = lane * 4; w < words; w += 128) {
@@ -798,6 +962,7 @@ __global__ void __launch_bounds__(kWarpsSym * 32)
                      int32_t* __restrict__ row_count, uint32_t* __restrict__ heavy_bitmaps, int64_t hbm_words,
                      int16_t* __restrict__ heavy_span) {
   __shared__ uint32_t bm[kMaxWords];
+  __shared__ unsigned long long tbl_all[kWarpsSym][32];
   __shared__ int red[kWarpsSym];
   __shared__ int first_word, last_word;
   const int wid = threadIdx.x >> 5;
@@ -811,7 +976,8 @@ __global__ void __launch_bounds__(kWarpsSym * 32)
       last_word = -1;
     }
     __syncthreads();
-    walk_columns(A, B, g, x, wid, kWarpsSym, [&](int32_t j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
+    walk_columns(A, B, g, x, wid, kWarpsSym, tbl_all[wid],
+                 [&](int32_t j) { atomicOr(&bm[j >> 5], 1u << (j & 31)); });
     __syncthreads();
     int cnt = 0, w0 = INT_MAX, w1 = -1;
     uint32_t* out = heavy_bitmaps + h * hbm_words;
@@ -865,11 +1031,12 @@ __global__ void k_tile_ptrs(Geom g, const int64_t* __restrict__ row_offset, int3
 }
 
 // Heavy rows are cut at fine-block boundaries into items of <= vcap outputs
-// (greedy left to right; leading empty blocks are skipped).  One warp per
-// heavy row (blocks of 256 threads): lanes count the fine blocks' outputs
-// from the row's bitmap, lane 0 cuts.  The first n_half rows' items hold half
-// as many outputs (see half_rows).  FILL = false counts the items,
-// FILL = true writes them.
+// (greedy left to right; leading empty blocks are skipped).  The first n_half
+// rows' items hold half as many outputs (see half_rows).  FILL = false counts
+// the items, FILL = true writes them.  Blocks of 256 threads, per_warp rows
+// (at most 32) per warp (with a warp per row and lane 0 cutting block by block the two launches took
+// 134 us at R-MAT s16, 1.9 ms at s18 and 3.1 ms on the 27-point stencil; now
+// 104 us, 1.2 and 0.21 ms).
 struct HeavyItem {
   int32_t h;       // heavy slot
   int16_t fb_lo;   // first fine block
@@ -882,86 +1049,81 @@ template <bool FILL>
 __global__ void __launch_bounds__(256)
     k_cut_heavy(Geom g, const int32_t* __restrict__ heavy_list, int n_heavy,
                 const uint32_t* __restrict__ heavy_bitmaps, int64_t hbm_words, int32_t* __restrict__ n_items,
-                const int64_t* __restrict__ first, HeavyItem* __restrict__ items, int vcap_most, int n_half,
+                const int64_t* __restrict__ first, HeavyItem* __restrict__ items, int vcap_most, int n_half, int per_warp,
                 const int32_t* __restrict__ row_count = nullptr, const int16_t* __restrict__ span = nullptr) {
-  __shared__ int32_t cnt_all[8][kMaxCols / kFineCols];
-  int32_t* cnt = cnt_all[threadIdx.x >> 5];
   const int lane = lane_id();
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  constexpr int kWordsPerBlock = kFineCols / 32;
-  for (int64_t h = warp; h < n_heavy; h += nwarps) {
-    const int64_t ri = heavy_list[h];
-    const RowInfo x = decode_row(g, ri);
-    const int nfb = (x.w + kFineCols - 1) / kFineCols;
-    const int vcap = h < n_half ? vcap_most / 2 : vcap_most;
-    if (span && row_count) {
-      // counted by the symbolic pass: a row whose outputs fit one item needs
-      // no look at its bitmap; the item spans its first to its last block
-      // with outputs
-      const int tot = __ldg(row_count + ri);
-      if (tot <= vcap) {
-        if (lane == 0) {
+  for (int64_t h0 = warp * per_warp; h0 < n_heavy; h0 += nwarps * per_warp) {
+    // counted by the symbolic pass: a row whose outputs fit one item needs no
+    // look at its bitmap, and each lane takes one; the item spans its first to
+    // its last block with outputs
+    int64_t my_ri = 0;
+    bool several = lane < per_warp && h0 + lane < n_heavy;
+    if (several) {
+      const int64_t h = h0 + lane;
+      my_ri = heavy_list[h];
+      if (span) {
+        const int tot = __ldg(row_count + my_ri);
+        if (tot <= (h < n_half ? vcap_most / 2 : vcap_most)) {
+          several = false;
           if (FILL && tot > 0)
             items[first[h]] = HeavyItem{(int32_t)h, __ldg(span + 2 * h), __ldg(span + 2 * h + 1), 0, tot};
           if (!FILL) n_items[h] = tot > 0 ? 1 : 0;
         }
-        continue;
       }
     }
-    const uint32_t* bm = heavy_bitmaps + h * hbm_words;
-    const int words = (x.w + 31) >> 5;
-    int tot = 0, first_nz = INT_MAX, last_nz = -1;
-    const int sp0 = span ? span[2 * h] : 0, sp1 = span ? span[2 * h + 1] : nfb;  // blocks that are stored
-    for (int b = lane; b < nfb; b += 32) {
-      int c = 0;
+    // the others by the warp, one after another: lanes count the fine blocks'
+    // outputs (at most 64) from the bitmap; an item ends before the first
+    // block that would exceed its bound, found by a ballot over the prefix sums
+    for (unsigned todo = __ballot_sync(kFull, several); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const int64_t h = h0 + src;
+      const RowInfo x = decode_row(g, __shfl_sync(kFull, my_ri, src));
+      const int nfb = (x.w + kFineCols - 1) / kFineCols;
+      const int vcap = h < n_half ? vcap_most / 2 : vcap_most;
+      const uint32_t* bm = heavy_bitmaps + h * hbm_words;
+      const int words = (x.w + 31) >> 5;
+      const int sp0 = span ? span[2 * h] : 0, sp1 = span ? span[2 * h + 1] : nfb;  // blocks that are stored
+      auto count = [&](int b) {
+        int c = 0;
+        if (b >= sp0 && b < sp1)
 #pragma unroll
-      for (int q = 0; q < kWordsPerBlock; q++) {
-        const int w = b * kWordsPerBlock + q;
-        if (w < words && b >= sp0 && b < sp1) c += __popc(__ldg(bm + w));
-      }
-      cnt[b] = c;
-      tot += c;
-      if (c > 0) {
-        first_nz = min(first_nz, b);
-        last_nz = max(last_nz, b);
-      }
-    }
-    tot = warp_sum(tot);
-    first_nz = __reduce_min_sync(kFull, first_nz);
-    last_nz = __reduce_max_sync(kFull, last_nz);
-    __syncwarp();
-    if (tot <= vcap) {
-      // one item, from the first to the last block with outputs: what the
-      // block-by-block cut below gives for such a row
-      if (lane == 0) {
-        if (FILL && tot > 0)
-          items[first[h]] = HeavyItem{(int32_t)h, (int16_t)first_nz, (int16_t)(last_nz + 1), 0, tot};
-        if (!FILL) n_items[h] = tot > 0 ? 1 : 0;
-      }
-    } else if (lane == 0) {
-      int nit = 0, cur = 0, start = 0, rel = 0, last = -1;
-      int64_t out = FILL ? first[h] : 0;
-      for (int b = 0; b < nfb; b++) {
-        const int c = cnt[b];
-        if (c > 0) last = b;
-        if (cur > 0 && cur + c > vcap) {
-          if (FILL) items[out++] = HeavyItem{(int32_t)h, (int16_t)start, (int16_t)b, rel, cur};
+          for (int q = 0; q < kBlockWords; q++) {
+            const int w = b * kBlockWords + q;
+            if (w < words) c += __popc(__ldg(bm + w));
+          }
+        return c;
+      };
+      const int c0 = lane < nfb ? count(lane) : 0, c1 = lane + 32 < nfb ? count(lane + 32) : 0;
+      const int lower = __reduce_add_sync(kFull, c0), tot = lower + __reduce_add_sync(kFull, c1);
+      const int p0 = warp_inclusive_scan(c0), p1 = lower + warp_inclusive_scan(c1);
+      const unsigned nz0 = __ballot_sync(kFull, c0 > 0), nz1 = __ballot_sync(kFull, c1 > 0);
+      int nit = 0;
+      if (tot > 0) {
+        const int last = nz1 ? 63 - __clz(nz1) : 31 - __clz(nz0);
+        int start = nz0 ? __ffs(nz0) - 1 : 31 + __ffs(nz1), base = 0;
+        int64_t out = FILL ? first[h] : 0;
+        for (;;) {
+          const unsigned m0 = __ballot_sync(kFull, lane >= start && p0 - base > vcap);
+          const unsigned m1 = __ballot_sync(kFull, lane + 32 >= start && p1 - base > vcap);
           nit++;
-          rel += cur;
-          cur = 0;
+          if (!(m0 | m1)) {
+            if (FILL && lane == 0)
+              items[out] = HeavyItem{(int32_t)h, (int16_t)start, (int16_t)(last + 1), base, tot - base};
+            break;
+          }
+          const int b = m0 ? __ffs(m0) - 1 : 31 + __ffs(m1);
+          const int before = __shfl_sync(kFull, b < 32 ? p0 - c0 : p1 - c1, b & 31);  // outputs before block b
+          if (FILL && lane == 0)
+            items[out] = HeavyItem{(int32_t)h, (int16_t)start, (int16_t)b, base, before - base};
+          out++;
           start = b;
+          base = before;
         }
-        if (cur == 0 && c == 0) start = b + 1;
-        cur += c;
       }
-      if (cur > 0) {  // the last item ends after the row's last block with outputs
-        if (FILL) items[out++] = HeavyItem{(int32_t)h, (int16_t)start, (int16_t)(last + 1), rel, cur};
-        nit++;
-      }
-      if (!FILL) n_items[h] = nit;
+      if (!FILL && lane == 0) n_items[h] = nit;
     }
-    __syncwarp();
   }
 }
 
@@ -1078,7 +1240,8 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
           atomicOr(&S.bm[xx >> 5], 1u << (xx & 31));
         });
       } else if (s0 == 0) {
-        walk_columns(A, B, g, x, 0, 1, [&](int32_t j) { atomicOr(&S.bm[j >> 5], 1u << (j & 31)); });
+        walk_columns(A, B, g, x, 0, 1, reinterpret_cast<unsigned long long*>(S.walk.seg),
+                     [&](int32_t j) { atomicOr(&S.bm[j >> 5], 1u << (j & 31)); });
       } else {
         for (int q = lane; q < cnt; q += 32) {
           const int j = out_col[off + q];
@@ -1488,7 +1651,11 @@ struct bclx_spgemm_plan_s {
   int32_t* smap_own = nullptr;    // stage map (Geom::smap / scount) owned by this plan
   int32_t* scount_own = nullptr;
   int32_t* rot_own = nullptr;     // sub-grid tile maps (Geom::rot_i, then rot_j) owned by this plan
-  unsigned long long* queue = nullptr;  // work-queue heads, one per stage launch
+  unsigned long long* queue = nullptr;  // work-queue heads, one per stage launch and planning pass
+  // scratch blocks that hold several of the arrays above (symbolic_impl):
+  // block1 counters .. row_offset, block2 the heavy rows' arrays
+  void* block1 = nullptr;
+  void* block2 = nullptr;
   // numeric tuning (bclx_spgemm_plan_tune)
   int grab = 1, blocks_per_sm = 4, long_seg = kLongSegDefault;
   int light_ub_max = kLightUb;         // light-row class bound (products), set at symbolic time
@@ -1559,6 +1726,20 @@ struct bclx_spgemm_plan_s {
     ub = light_ub = item_count = item_cap = row_failed = block_ub = failed_list = temp_col = redo_col = nullptr;
     light_slot = item_pos = item_off = redo_off = nullptr;
     temp_val = redo_val = nullptr;
+    if (block1) {
+      counters = row_count = light_list = heavy_list = vheavy_list = heavy_tmp = nullptr;
+      products_dev = queue = nullptr;
+      row_offset = nullptr;
+    }
+    if (block2) {
+      heavy_bitmaps = nullptr;
+      heavy_span = nullptr;
+      heavy_nitems = nullptr;
+      heavy_first = nullptr;
+    }
+    scratch_free(ctx, block1);
+    scratch_free(ctx, block2);
+    block1 = block2 = nullptr;
     void* ps[] = {queue, light_list, heavy_list, vheavy_list, heavy_tmp, counters, products_dev, row_count, row_offset, heavy_bitmaps,
                   heavy_nitems, heavy_first, heavy_items, tab, id_rp, id_ci, id_v, id_desc, acc_tile_offset,
                   smap_own, scount_own, rot_own, heavy_span};
@@ -1640,11 +1821,11 @@ static int launch_symbolic(Context* ctx, const SpGridView& A, const SpGridView& 
   }
   const int64_t rows = P->n_light + P->n_heavy - P->n_vheavy;
   if (rows > 0) {
-    // queue head 0 (each numeric launch clears its head before use)
-    BCLX_CK(cudaMemsetAsync(P->queue, 0, sizeof(unsigned long long), ctx->stream));
+    unsigned long long* queue = P->queue + kSymbolicSlot;
+    if (!P->block1) BCLX_CK(cudaMemsetAsync(queue, 0, sizeof(unsigned long long), ctx->stream));  // (block1 starts at 0)
     k_symbolic<<<grid_for(ctx, rows, kWarpsSym, 8), kWarpsSym * 32, 0, ctx->stream>>>(
         A, B, P->g, P->light_list, P->heavy_list, (int)P->n_light, (int)P->n_heavy, (int)P->n_vheavy,
-        P->row_count, P->heavy_bitmaps, P->hbm_words, P->heavy_span, P->queue, queue_grab(ctx, rows, kWarpsSym, 8, 8));
+        P->row_count, P->heavy_bitmaps, P->hbm_words, P->heavy_span, queue, queue_grab(ctx, rows, kWarpsSym, 8, 8));
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -1663,7 +1844,7 @@ static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView&
     configured.fetch_or(bit);
   }
   const int64_t n_total = P->n_light + P->n_heavy_items;
-  unsigned long long* q = P->queue + (s0 % kQueueSlots);
+  unsigned long long* q = P->queue + s0;  // (at most 254 stages)
   BCLX_CK(cudaMemsetAsync(q, 0, sizeof(unsigned long long), ctx->stream));
   const int bps = P->blocks_per_sm < 1 ? 1 : (P->blocks_per_sm > 4 ? 4 : P->blocks_per_sm);
   kern<<<grid_for(ctx, n_total, kWarpsNum, bps), kWarpsNum * 32, smem, ctx->stream>>>(
@@ -1777,7 +1958,7 @@ static int build_btable(Context* ctx, const SpGridView& B, const Geom& g, bclx_s
     BCLX_CK(cudaStreamWaitEvent(side, ctx->fork_ev, 0));
     st = side;
   }
-  k_btable<<<grid_for(ctx, nbrows / 32 + 1, 8, 16), 256, 0, st>>>(B, g, P->tab);
+  k_btable<<<grid_for(ctx, nbrows, kBtableRows, 6), kBtableRows, 0, st>>>(B, g, P->tab);
   note_launch();
   BCLX_CK_LAUNCH();
   return BCLX_OK;
@@ -1793,43 +1974,70 @@ static int half_rows(const Context* ctx, const bclx_spgemm_plan_s* P) {
   return P->n_vheavy <= ctx->num_sms ? (int)P->n_vheavy : 0;
 }
 
+// Pieces of one scratch block, each on 256 bytes: take() with base null adds up
+// the size, with the block's address hands the pieces out in the same order.
+struct Pieces {
+  unsigned char* base = nullptr;
+  size_t used = 0;
+  template <typename T>
+  void take(T** p, size_t count) {
+    if (base) *p = reinterpret_cast<T*>(base + used);
+    used += (sizeof(T) * (count > 0 ? count : 1) + 255) & ~size_t(255);
+  }
+};
+template <typename F>
+static int scratch_pieces(Context* ctx, void** block, F&& layout) {
+  Pieces p;
+  layout(p);
+  BCLX_TRY(scratch_alloc(ctx, block, p.used));
+  p = Pieces{reinterpret_cast<unsigned char*>(*block), 0};
+  layout(p);
+  return BCLX_OK;
+}
+
 // Classification, symbolic, row offsets and the heavy-row cut.
 static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B, Geom g, int dtype,
                          int32_t* tile_row_ptr, int64_t* tile_offset, bclx_spgemm_plan_s* P) {
   BCLX_TRY(build_stage_map(ctx, A, B, P, g));
   P->g = g;
-  // The B-row table depends on B alone: it is built on the side stream from
-  // the start, beside classification and the symbolic pass.
-  BCLX_TRY(ensure_side_stream(ctx));
-  BCLX_TRY(build_btable(ctx, B, g, P, ctx->side));
   P->dtype = dtype;
   const int64_t nri = g.n_row_items;
   P->hbm_words = padded_words(g.tn);
-  BCLX_TRY(scratch_alloc_n(ctx, &P->light_list, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_list, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->vheavy_list, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_tmp, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->counters, 4));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->products_dev, 1));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->row_count, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->row_offset, nri + 1));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->queue, kQueueSlots));
-  BCLX_CK(cudaMemsetAsync(P->counters, 0, 4 * sizeof(int32_t), ctx->stream));
-  BCLX_CK(cudaMemsetAsync(P->products_dev, 0, sizeof(unsigned long long), ctx->stream));
-  BCLX_CK(cudaMemsetAsync(P->row_count, 0, sizeof(int32_t) * (nri > 0 ? nri : 1), ctx->stream));
+  // (what starts at zero comes first: one memset; an allocation is some 2 us of
+  // the host and a memset 1.5 us of the GPU, which small products are made of)
+  int64_t* sums = nullptr;
+  BCLX_TRY(scratch_pieces(ctx, &P->block1, [&](Pieces& p) {
+    p.take(&P->counters, 4);
+    p.take(&P->products_dev, 1);
+    p.take(&P->queue, kQueueSlots);
+    p.take(&P->row_count, nri);
+    p.take(&P->light_list, nri);
+    p.take(&P->heavy_list, nri);
+    p.take(&P->vheavy_list, nri);
+    p.take(&P->heavy_tmp, nri);
+    p.take(&P->row_offset, nri + 1);
+    p.take(&sums, exclusive_scan_sums_len(nri));
+  }));
+  BCLX_CK(cudaMemsetAsync(P->block1, 0, reinterpret_cast<char*>(P->row_count + nri) - reinterpret_cast<char*>(P->block1),
+                          ctx->stream));
   // rows of tiles wider than 8192 columns take the heavy path unless the
   // context allows light rows there (BCLX_TUNE_WIDE_LIGHT)
   const int heavy_min_cols = tuning(ctx, BCLX_TUNE_WIDE_LIGHT) ? INT_MAX : 8192 + 1;
   P->light_ub_max = (int)tuning(ctx, BCLX_TUNE_LIGHT_UB);
   P->vcap = (int)tuning(ctx, BCLX_TUNE_ITEM_OUTPUTS);
   int32_t* live = nullptr;  // C tiles with stages (when the stage map says which)
-  if (nri > 0) {
-    BCLX_CK(cudaMemsetAsync(P->queue + 1, 0, sizeof(unsigned long long), ctx->stream));
+  if (nri > 0 && !g.scount) {
+    k_classify_rows<<<grid_for(ctx, g.gm * g.tm, 8, 8), 256, 0, ctx->stream>>>(
+        A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,
+        P->light_ub_max);
+    note_launch();
+    BCLX_CK_LAUNCH();
+  } else if (nri > 0) {
     const int64_t nt = g.gm * g.gn;
     BCLX_TRY(build_live_tiles(ctx, g, &live));
     k_classify<false><<<grid_for(ctx, nri, 8, 16), 256, 0, ctx->stream>>>(
         A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols, P->light_ub_max,
-        nullptr, nullptr, P->queue + 1, queue_grab(ctx, nri, 8, 16, 32, 8), live, live ? live + nt : nullptr);
+        nullptr, nullptr, P->queue + kClassifySlot, queue_grab(ctx, nri, 8, 16, 32, 8), live, live ? live + nt : nullptr);
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -1842,41 +2050,57 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   P->n_vheavy = cnts[3];
   P->n_heavy = cnts[1] + cnts[3];
   P->products = ctx->pinned[2];
-  // heavy slots: the very heavy rows first, then the others
-  if (P->n_vheavy > 0)
-    BCLX_CK(cudaMemcpyAsync(P->heavy_list, P->vheavy_list, sizeof(int32_t) * P->n_vheavy, cudaMemcpyDeviceToDevice,
-                            ctx->stream));
-  if (cnts[1] > 0)
-    BCLX_CK(cudaMemcpyAsync(P->heavy_list + P->n_vheavy, P->heavy_tmp, sizeof(int32_t) * cnts[1],
-                            cudaMemcpyDeviceToDevice, ctx->stream));
-
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_bitmaps, (size_t)P->n_heavy * P->hbm_words));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_span, 2 * (size_t)P->n_heavy));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_nitems, P->n_heavy));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_first, P->n_heavy + 1));
+  int64_t* sums_h = nullptr;
+  if (P->n_heavy > 0) {
+    // The B-row table depends on B alone and only heavy items read it: it is
+    // built on the side stream, beside the symbolic pass.
+    BCLX_TRY(ensure_side_stream(ctx));
+    BCLX_TRY(build_btable(ctx, B, g, P, ctx->side));
+    // heavy slots: the very heavy rows first, then the others
+    if (P->n_vheavy > 0)
+      BCLX_CK(cudaMemcpyAsync(P->heavy_list, P->vheavy_list, sizeof(int32_t) * P->n_vheavy, cudaMemcpyDeviceToDevice,
+                              ctx->stream));
+    if (cnts[1] > 0)
+      BCLX_CK(cudaMemcpyAsync(P->heavy_list + P->n_vheavy, P->heavy_tmp, sizeof(int32_t) * cnts[1],
+                              cudaMemcpyDeviceToDevice, ctx->stream));
+    BCLX_TRY(scratch_pieces(ctx, &P->block2, [&](Pieces& p) {
+      p.take(&P->heavy_bitmaps, (size_t)P->n_heavy * P->hbm_words);
+      p.take(&P->heavy_span, 2 * (size_t)P->n_heavy);
+      p.take(&P->heavy_nitems, P->n_heavy);
+      p.take(&P->heavy_first, P->n_heavy + 1);
+      p.take(&sums_h, exclusive_scan_sums_len(P->n_heavy));
+    }));
+  }
   BCLX_TRY(launch_symbolic(ctx, A, B, P, true));
-  // the side stream (B-row table, very heavy rows) joins before the scan
-  BCLX_CK(cudaEventRecord(ctx->join_ev, ctx->side));
-  BCLX_CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
-  BCLX_TRY(exclusive_scan_i32(ctx, P->row_count, P->row_offset, nri));
+  if (P->n_heavy > 0) {
+    // the side stream (B-row table, very heavy rows) joins before the scan
+    BCLX_CK(cudaEventRecord(ctx->join_ev, ctx->side));
+    BCLX_CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
+  }
+  BCLX_TRY(exclusive_scan_i32_buf(ctx, P->row_count, P->row_offset, nri, sums));
   const int64_t ntiles = g.gm * g.gn;
   k_tile_ptrs<<<grid_for(ctx, ntiles * (g.tm + 1) / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
       g, P->row_offset, tile_row_ptr, tile_offset, P->counters + 2);
   note_launch();
   BCLX_CK_LAUNCH();
+  // rows per warp: as many as leave every resident warp some
+  const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(32, P->n_heavy / ((int64_t)ctx->num_sms * 64)));
+  const unsigned cut_blocks = grid_for(ctx, ceil_div(P->n_heavy, (int64_t)per_warp), 8, 8);
   if (P->n_heavy > 0) {
-    const unsigned blocks = grid_for(ctx, P->n_heavy, 8, 8);
-    k_cut_heavy<false><<<blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
-                                                        P->hbm_words, P->heavy_nitems, nullptr, nullptr, P->vcap,
-                                                        half_rows(ctx, P), P->row_count, P->heavy_span);
+    k_cut_heavy<false><<<cut_blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
+                                                            P->hbm_words, P->heavy_nitems, nullptr, nullptr, P->vcap,
+                                                            half_rows(ctx, P), per_warp, P->row_count, P->heavy_span);
     note_launch();
     BCLX_CK_LAUNCH();
+    BCLX_TRY(exclusive_scan_i32_buf(ctx, P->heavy_nitems, P->heavy_first, P->n_heavy, sums_h));
+    BCLX_TRY(read_back(
+        ctx, {{P->row_offset + nri, 8, 0}, {P->counters + 2, 4, 2}, {P->heavy_first + P->n_heavy, 8, 1}}));
+  } else {
+    BCLX_TRY(read_back(ctx, {{P->row_offset + nri, 8, 0}, {P->counters + 2, 4, 2}}));
   }
-  BCLX_TRY(exclusive_scan_i32(ctx, P->heavy_nitems, P->heavy_first, P->n_heavy));
-  BCLX_TRY(read_back(ctx, {{P->row_offset + nri, 8, 0}, {P->heavy_first + P->n_heavy, 8, 1}, {P->counters + 2, 4, 2}}));
   BCLX_CK(cudaStreamSynchronize(ctx->stream));
   P->nnz = ctx->pinned[0];
-  P->n_heavy_items = ctx->pinned[1];
+  P->n_heavy_items = P->n_heavy > 0 ? ctx->pinned[1] : 0;
   int32_t overflow;
   std::memcpy(&overflow, ctx->pinned + 2, sizeof(overflow));
   if (overflow) {
@@ -1885,16 +2109,11 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   }
   if (P->n_heavy > 0) {
     BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_items, P->n_heavy_items));
-    const unsigned blocks = grid_for(ctx, P->n_heavy, 8, 8);
-    k_cut_heavy<true><<<blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
-                                                       P->hbm_words, nullptr, P->heavy_first, P->heavy_items, P->vcap,
-                                                       half_rows(ctx, P), P->row_count, P->heavy_span);
+    k_cut_heavy<true><<<cut_blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
+                                                           P->hbm_words, nullptr, P->heavy_first, P->heavy_items, P->vcap,
+                                                           half_rows(ctx, P), per_warp, P->row_count, P->heavy_span);
     note_launch();
     BCLX_CK_LAUNCH();
-  }
-  if (P->n_heavy == 0 && P->tab) {  // no heavy item reads the table
-    scratch_free(ctx, P->tab);
-    P->tab = nullptr;
   }
   return BCLX_OK;
 }
@@ -2305,7 +2524,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
   BCLX_CK_LAUNCH();
   if (P.n_heavy > 0) {
     k_cut_heavy<false><<<grid_for(ctx, P.n_heavy, 8, 8), 256, 0, ctx->stream>>>(
-        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, P.heavy_nitems, nullptr, nullptr, P.vcap, 0);
+        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, P.heavy_nitems, nullptr, nullptr, P.vcap, 0, 1);
     note_launch();
     BCLX_CK_LAUNCH();
   }
@@ -2340,11 +2559,11 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
     if (probe.ok) ar = probe;
     else P.tab = nullptr;
     k_cut_heavy<true><<<grid_for(ctx, P.n_heavy, 8, 8), 256, 0, ctx->stream>>>(
-        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, nullptr, P.heavy_first, P.heavy_items, P.vcap, 0);
+        g, P.heavy_list, (int)P.n_heavy, P.heavy_bitmaps, P.hbm_words, nullptr, P.heavy_first, P.heavy_items, P.vcap, 0, 1);
     note_launch();
     BCLX_CK_LAUNCH();
     if (P.tab && g.tk > 0) {
-      k_btable<<<grid_for(ctx, g.tk / 32 + 1, 8, 16), 256, 0, ctx->stream>>>(B, g, P.tab);
+      k_btable<<<grid_for(ctx, g.tk, kBtableRows, 6), kBtableRows, 0, ctx->stream>>>(B, g, P.tab);
       note_launch();
       BCLX_CK_LAUNCH();
     }
@@ -2594,7 +2813,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->row_offset = P->redo_off;  // borrowed
     const unsigned rb = grid_for(ctx, nf, 8, 8);
     k_cut_heavy<false><<<rb, 256, 0, ctx->stream>>>(g, R->heavy_list, nf, R->heavy_bitmaps, R->hbm_words,
-                                                    R->heavy_nitems, nullptr, nullptr, R->vcap, 0);
+                                                    R->heavy_nitems, nullptr, nullptr, R->vcap, 0, 1);
     note_launch();
     BCLX_CK_LAUNCH();
     BCLX_TRY(exclusive_scan_i32(ctx, R->heavy_nitems, R->heavy_first, nf));
@@ -2605,7 +2824,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->n_heavy_items = rt[0];
     BCLX_TRY(scratch_alloc_n(ctx, &R->heavy_items, R->n_heavy_items));
     k_cut_heavy<true><<<rb, 256, 0, ctx->stream>>>(g, R->heavy_list, nf, R->heavy_bitmaps, R->hbm_words, nullptr,
-                                                   R->heavy_first, R->heavy_items, R->vcap, 0);
+                                                   R->heavy_first, R->heavy_items, R->vcap, 0, 1);
     note_launch();
     BCLX_CK_LAUNCH();
     R->tab = P->tab;  // borrowed
