@@ -1657,7 +1657,7 @@ struct bclx_spgemm_plan_s {
   void* block1 = nullptr;
   void* block2 = nullptr;
   // numeric tuning (bclx_spgemm_plan_tune)
-  int grab = 1, blocks_per_sm = 4, long_seg = kLongSegDefault;
+  int grab = 0, blocks_per_sm = 4, long_seg = kLongSegDefault;  // (grab 0: see numeric_grab)
   int light_ub_max = kLightUb;         // light-row class bound (products), set at symbolic time
   int vcap = kVcap;                    // outputs per heavy item (512 or 1024), set at symbolic time
   // CUDA graph of the staged numeric pass (bclx_spgemm_numeric_staged)
@@ -1832,6 +1832,16 @@ static int launch_symbolic(Context* ctx, const SpGridView& A, const SpGridView& 
   return BCLX_OK;
 }
 
+// Items a warp of the numeric pass takes from the queue at a time: one where
+// there are very heavy rows (their items come first, and two of them in one
+// warp can be the launch's end: R-MAT s16 2.81 ms with 1, 3.10 with 2, 3.67 with
+// 4), otherwise about 32 grabs per resident warp and at most 8 (27-point
+// stencil, 10.4M items of 143 products: 24.4 ms with 1, 22.3 with 4, 21.9 with 8
+// and with 16: the counter is one address).
+static int numeric_grab(Context* ctx, const bclx_spgemm_plan_s* P, int64_t n_total) {
+  return P->n_vheavy > 0 ? 1 : queue_grab(ctx, n_total, kWarpsNum, 4, 8);
+}
+
 template <typename VT, int WORDS, bool LEARNED = false, int VCAP = kVcap>
 static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView& B, bclx_spgemm_plan_s* P,
                             int32_t* out_col, void* out_val, int s0, int s1) {
@@ -1850,7 +1860,7 @@ static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView&
   kern<<<grid_for(ctx, n_total, kWarpsNum, bps), kWarpsNum * 32, smem, ctx->stream>>>(
       A, B, P->g, P->light_list, P->heavy_list, (int)P->n_light, P->n_heavy_items, P->heavy_items, P->heavy_bitmaps,
       P->hbm_words, P->tab, P->row_count, P->row_offset, out_col, reinterpret_cast<VT*>(out_val), s0, s1, q,
-      P->grab < 1 ? 1 : P->grab, P->long_seg < 1 ? 1 : P->long_seg, LEARNED ? P->light_slot : nullptr,
+      P->grab > 0 ? P->grab : numeric_grab(ctx, P, n_total), P->long_seg < 1 ? 1 : P->long_seg, LEARNED ? P->light_slot : nullptr,
       LEARNED ? P->item_count : nullptr, LEARNED ? P->row_count : nullptr, LEARNED ? P->row_failed : nullptr,
       P->heavy_slot_base, LEARNED ? P->item_off : nullptr);
   note_launch();
