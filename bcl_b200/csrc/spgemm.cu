@@ -46,6 +46,7 @@
 #include <initializer_list>
 #include <mutex>
 #include <tuple>
+#include <utility>
 #include <type_traits>
 #include <vector>
 
@@ -59,6 +60,7 @@ constexpr int kMaxCols = kMaxWords * 32;
 constexpr int kWarpsSym = 8;
 constexpr int kWarpsNum = 8;
 constexpr int kNoStage = 0xff;
+constexpr int64_t kSplitMaxProducts = 40 << 20;  // largest product whose items are split by stage (SplitItems)
 // FP32 chunks whose B segments average fewer products are walked packed (see
 // walk_products).  Numeric pass with 1 (every chunk entry by entry), 6, 14, 28
 // and no bound: R-MAT s16 3.20, 2.92, 2.85, 2.88, 2.99 ms; R-MAT s18 34.0, 30.5,
@@ -66,6 +68,7 @@ constexpr int kNoStage = 0xff;
 constexpr int kLongSegDefault = 14;
 constexpr int kQueueSlots = 256;          // work-queue heads in a plan: one per stage launch (at most 254), and
 constexpr int kClassifySlot = 254, kSymbolicSlot = 255;  // the planning passes' (each used once)
+constexpr int64_t kMidHeavyUb = 8192;    // from here on where such rows are few (see symbolic_impl)
 constexpr int64_t kVeryHeavyUb = 32768;  // rows above this many products get a whole block in the symbolic pass
 
 constexpr int kBlockWords = kFineCols / 32;  // bitmap words of a fine block
@@ -536,9 +539,9 @@ __device__ __forceinline__ void walk_columns_ranged(const SpGridView& A, const S
 // to the host).
 
 struct ReadBack {
-  const void* src[4];
-  int32_t bytes[4];  // at most 8 each
-  int32_t slot[4];   // 8-byte destination slot
+  const void* src[5];
+  int32_t bytes[5];  // at most 8 each
+  int32_t slot[5];   // 8-byte destination slot
   int32_t n;
 };
 
@@ -549,12 +552,12 @@ __global__ void k_read_back(ReadBack r, int64_t* __restrict__ dst) {
       reinterpret_cast<volatile unsigned char*>(dst + r.slot[i])[t] = reinterpret_cast<const unsigned char*>(r.src[i])[t];
 }
 
-// Store up to four values (each at most 8 bytes) into ctx->pinned[slot] on
+// Store up to five values (each at most 8 bytes) into ctx->pinned[slot] on
 // the context's stream; the host reads them after synchronizing the stream.
 static int read_back(Context* ctx, std::initializer_list<std::tuple<const void*, int, int>> items) {
   ReadBack r{};
   for (const auto& it : items) {
-    if (r.n == 4 || std::get<1>(it) > 8) return BCLX_ERR_INVALID;
+    if (r.n == 5 || std::get<1>(it) > 8) return BCLX_ERR_INVALID;
     r.src[r.n] = std::get<0>(it);
     r.bytes[r.n] = std::get<1>(it);
     r.slot[r.n] = std::get<2>(it);
@@ -701,31 +704,31 @@ constexpr int kClassifyDefer = 64;  // long rows a block can put off
 __global__ void __launch_bounds__(256) k_classify_rows(
     SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
     int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
-    int heavy_min_cols, int light_ub) {
-  __shared__ int32_t kept_all[8][3][kClassifyKeep * 32];
+    int heavy_min_cols, int light_ub) {  // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list
+  __shared__ int32_t kept_all[8][4][kClassifyKeep * 32];
   __shared__ unsigned long long sums[32];
   __shared__ uint32_t deferred[kClassifyDefer];
   __shared__ int n_deferred;
   const int wid = threadIdx.x >> 5;
   int32_t(*kept)[kClassifyKeep * 32] = kept_all[wid];
-  int32_t* const lists[3] = {light_list, heavy_list, vheavy_list};
   const int lane = lane_id();
   const unsigned below = (1u << lane) - 1u;
   const uint32_t n_rows = (uint32_t)(g.gm * g.tm), tm = (uint32_t)g.tm;
   const int gk = (int)g.gk, gn = (int)g.gn;
   const uint32_t warp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * 8;
   unsigned long long mine = 0;
-  int n_kept[3] = {0, 0, 0};
+  int n_kept[4] = {0, 0, 0, 0};
   int rows = 0;
   auto append = [&]() {
     __syncwarp();
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
+    for (int c = 0; c < 4; c++) {  // light, heavy, very heavy, above kMidHeavyUb
       if (n_kept[c] == 0) continue;
       int pos = 0;
-      if (lane == 0) pos = atomicAdd(&counters[c == 2 ? 3 : c], n_kept[c]);
+      if (lane == 0) pos = atomicAdd(&counters[c < 2 ? c : c + 1], n_kept[c]);
       pos = __shfl_sync(kFull, pos, 0);
-      for (int q = lane; q < n_kept[c]; q += 32) lists[c][pos + q] = kept[c][q];
+      int32_t* const list = c == 0 ? light_list : (c == 1 ? heavy_list : vheavy_list);
+      for (int q = lane; q < n_kept[c]; q += 32) list[c == 3 ? g.n_row_items - 1 - (pos + q) : pos + q] = kept[c][q];
       n_kept[c] = 0;
     }
     rows = 0;
@@ -737,10 +740,10 @@ __global__ void __launch_bounds__(256) k_classify_rows(
     int cls = -1;
     if (tot > 0) {
       const int64_t w = min(g.n - (int64_t)j * g.tn, g.tn);
-      cls = tot <= light_ub && w < heavy_min_cols ? 0 : (tot <= kVeryHeavyUb ? 1 : 2);
+      cls = tot <= light_ub && w < heavy_min_cols ? 0 : (tot <= kMidHeavyUb ? 1 : (tot <= kVeryHeavyUb ? 3 : 2));
     }
 #pragma unroll
-    for (int c = 0; c < 3; c++) {
+    for (int c = 0; c < 4; c++) {
       const unsigned m = __ballot_sync(kFull, cls == c);
       if (cls == c) kept[c][n_kept[c] + __popc(m & below)] = (int32_t)((ti * (uint32_t)gn + (uint32_t)j) * tm + r);
       n_kept[c] += __popc(m);
@@ -1139,6 +1142,26 @@ struct WarpSmem {
   WalkTable<VT> walk;
 };
 
+// Items whose stages run as work items of their own, on warps of their own:
+// a column's stage partials are independent chains, added in stage order
+// afterwards.  Stage s of item i leaves its partials at val[(i*gk + s)*stride]
+// and a bit per column it reached in mask; the warp that finishes an item's
+// last stage (count[i], back to 0 for the next launch) adds them up.  For the
+// items of a few very heavy rows, where one item is the launch's end, and
+// only as many as give every resident warp one (item, stage) at most, of
+// products of at most kSplitMaxProducts (a larger one keeps the GPU busy for
+// longer than its longest item): graph x sparse features, 14.5M products,
+// 383 -> 204 us; R-MAT of 12,000 rows on 2x2 tiles, 34M, 336 -> 272; 50,000 rows x
+// features, 11.5M, 330 -> 281; R-MAT of 30,011 rows, 50M, 480 without and 504
+// with.
+struct SplitItems {
+  int n = 0;       // items [0, n)
+  int stride = 0;  // outputs per item, a multiple of 32
+  void* val = nullptr;
+  uint32_t* mask = nullptr;
+  int32_t* count = nullptr;
+};
+
 #ifndef BCLX_NUMERIC_MIN_BLOCKS
 #define BCLX_NUMERIC_MIN_BLOCKS 4
 #endif
@@ -1150,6 +1173,7 @@ struct WarpSmem {
 // sparse features 0.69 -> 0.39; the 27-point stencil on 128^3, whose rows are
 // one item each (walked by the B rows' own bounds instead of two binary
 // searches per A entry), 37.6 -> 24.8.
+// The first split.n items are taken stage by stage (SplitItems).
 // LEARNED: the learned product's single pass.  Heavy items come from the
 // predicted cut (their counts are unknown): each builds its bitmap from its
 // own products, and an item with more than kVcap outputs marks its row in
@@ -1158,7 +1182,7 @@ struct WarpSmem {
 // heavy_slot_base + item_off[idx], after all light slots; an item's slot
 // count, at most kVcap, comes from the prediction),
 // counts to item_count / row_count_w.
-template <typename VT, int WORDS, bool LEARNED, int VCAP>
+template <typename VT, int WORDS, bool LEARNED, int VCAP, bool SPLIT>
 __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     k_numeric(SpGridView A, SpGridView B, Geom g, const int32_t* __restrict__ light_list,
               const int32_t* __restrict__ heavy_list, int n_light, int64_t n_heavy_items,
@@ -1169,11 +1193,12 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
               unsigned long long* __restrict__ queue, int grab, int long_seg,
               const int64_t* __restrict__ light_slot, int32_t* __restrict__ item_count,
               int32_t* __restrict__ row_count_w, int32_t* __restrict__ row_failed, int64_t heavy_slot_base,
-              const int64_t* __restrict__ item_off) {
+              const int64_t* __restrict__ item_off, SplitItems split) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WarpSmem<VT, WORDS, VCAP>& S = reinterpret_cast<WarpSmem<VT, WORDS, VCAP>*>(smem_raw)[threadIdx.x >> 5];
   const int lane = lane_id();
-  const int64_t n_total = n_heavy_items + n_light;
+  const uint32_t n_sub = SPLIT ? (uint32_t)split.n * (uint32_t)g.gk : 0u;  // (item, stage) pairs come first
+  const int64_t n_total = n_heavy_items + n_light + (SPLIT ? (int64_t)n_sub - split.n : 0);
   // persistent warps: take `grab` consecutive items at a time from the queue
   uint32_t next = 0, stop = 0;
   for (;;) {
@@ -1185,7 +1210,20 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
       next = b;
       stop = min(b + (uint32_t)grab, (uint32_t)n_total);
     }
-    const uint32_t idx = next++;
+    uint32_t idx = next++;
+    const bool part_only = SPLIT && idx < n_sub;
+    if (SPLIT) {  // (such a launch covers every stage)
+      s0 = 0;
+      s1 = (int)g.gk;
+      if (part_only) {
+        const uint32_t item = idx / (uint32_t)g.gk;
+        s0 = (int)(idx - item * (uint32_t)g.gk);
+        s1 = s0 + 1;
+        idx = item;
+      } else {
+        idx = idx - n_sub + (uint32_t)split.n;
+      }
+    }
     // heavy items first (they are the larger ones)
     const bool heavy = idx < n_heavy_items;
     int64_t ri;
@@ -1317,7 +1355,7 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     // columns are put in order in shared memory (in the space of `part`) and
     // leave as whole lines: written one by one from the bitmap's words they
     // are as many separate L2 writes as outputs.
-    if (s0 == 0) {
+    if (s0 == 0 || part_only) {
       int32_t* const cols = reinterpret_cast<int32_t*>(S.part);
       for (int w = lane; w < words; w += 32) {
         uint32_t bits = S.bm[w];
@@ -1329,7 +1367,8 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
         }
       }
       __syncwarp();
-      for (int q = lane; q < cnt; q += 32) out_col[off + q] = cols[q];
+      if (s0 == 0)
+        for (int q = lane; q < cnt; q += 32) out_col[off + q] = cols[q];
       for (int q = lane * 4; q < cnt; q += 128) *reinterpret_cast<uint4*>(S.acc + q) = make_uint4(0u, 0u, 0u, 0u);
     } else {
       for (int q = lane; q < cnt; q += 32) S.acc[q] = out_val[off + q];
@@ -1386,6 +1425,37 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     walk_products<VT>(A, B, g, x, s0, s1, ranged, fb_lo, fb_hi, tab, long_seg, S.walk, update, update_direct);
 
     // 5. last fold and values out
+    if (part_only) {
+      const int gk = (int)g.gk;
+      const int64_t first = (int64_t)idx * gk * split.stride;  // stage 0's partials
+      VT* const val = reinterpret_cast<VT*>(split.val) + first;
+      uint32_t* const mask = split.mask + first / 32;
+      for (int q = lane; q - lane < cnt; q += 32) {
+        const bool on = q < cnt && (!kOrdered || S.tag[q] != kNoStage);
+        const unsigned m = __ballot_sync(kFull, on);
+        if (on) val[s0 * split.stride + q] = kOrdered ? S.part[q] : S.acc[q];
+        if (lane == 0) mask[(s0 * split.stride + q) / 32] = m;
+      }
+      __threadfence();
+      __syncwarp();
+      int done = 0;
+      if (lane == 0) done = atomicAdd(split.count + idx, 1);
+      done = __shfl_sync(kFull, done, 0);
+      if (done == gk - 1) {
+        __threadfence();
+        for (int q = lane; q < cnt; q += 32) {
+          VT v = VT(0);
+          for (int st = 0; st < gk; st++) {
+            const int64_t at = st * split.stride + q;
+            if ((__ldcg(mask + at / 32) >> (q & 31)) & 1u) v = vadd(v, __ldcg(val + at));
+          }
+          out_val[off + q] = v;
+        }
+        if (lane == 0) split.count[idx] = 0;
+      }
+      __syncwarp();
+      continue;
+    }
     for (int q = lane; q < cnt; q += 32) {
       VT v = S.acc[q];
       if (kOrdered && S.tag[q] != kNoStage) v = vadd(v, S.part[q]);
@@ -1656,6 +1726,8 @@ struct bclx_spgemm_plan_s {
   // block1 counters .. row_offset, block2 the heavy rows' arrays
   void* block1 = nullptr;
   void* block2 = nullptr;
+  SplitItems split;               // the very heavy rows' items, where there are few (split_block)
+  void* split_block = nullptr;
   // numeric tuning (bclx_spgemm_plan_tune)
   int grab = 0, blocks_per_sm = 4, long_seg = kLongSegDefault;  // (grab 0: see numeric_grab)
   int light_ub_max = kLightUb;         // light-row class bound (products), set at symbolic time
@@ -1739,7 +1811,9 @@ struct bclx_spgemm_plan_s {
     }
     scratch_free(ctx, block1);
     scratch_free(ctx, block2);
-    block1 = block2 = nullptr;
+    scratch_free(ctx, split_block);
+    block1 = block2 = split_block = nullptr;
+    split = SplitItems();
     void* ps[] = {queue, light_list, heavy_list, vheavy_list, heavy_tmp, counters, products_dev, row_count, row_offset, heavy_bitmaps,
                   heavy_nitems, heavy_first, heavy_items, tab, id_rp, id_ci, id_v, id_desc, acc_tile_offset,
                   smap_own, scount_own, rot_own, heavy_span};
@@ -1842,18 +1916,19 @@ static int numeric_grab(Context* ctx, const bclx_spgemm_plan_s* P, int64_t n_tot
   return P->n_vheavy > 0 ? 1 : queue_grab(ctx, n_total, kWarpsNum, 4, 8);
 }
 
-template <typename VT, int WORDS, bool LEARNED = false, int VCAP = kVcap>
+template <typename VT, int WORDS, bool LEARNED = false, int VCAP = kVcap, bool SPLIT = false>
 static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView& B, bclx_spgemm_plan_s* P,
                             int32_t* out_col, void* out_val, int s0, int s1) {
   constexpr size_t smem = sizeof(WarpSmem<VT, WORDS, VCAP>) * kWarpsNum;
-  auto kern = k_numeric<VT, WORDS, LEARNED, VCAP>;
+  auto kern = k_numeric<VT, WORDS, LEARNED, VCAP, SPLIT>;
   static std::atomic<unsigned long long> configured{0};  // one bit per device
   const unsigned long long bit = 1ull << (ctx->device & 63);
   if (!(configured.load() & bit)) {
     BCLX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured.fetch_or(bit);
   }
-  const int64_t n_total = P->n_light + P->n_heavy_items;
+  const SplitItems split = SPLIT ? P->split : SplitItems();
+  const int64_t n_total = P->n_light + P->n_heavy_items + split.n * (P->g.gk - 1);
   unsigned long long* q = P->queue + s0;  // (at most 254 stages)
   BCLX_CK(cudaMemsetAsync(q, 0, sizeof(unsigned long long), ctx->stream));
   const int bps = P->blocks_per_sm < 1 ? 1 : (P->blocks_per_sm > 4 ? 4 : P->blocks_per_sm);
@@ -1862,7 +1937,7 @@ static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView&
       P->hbm_words, P->tab, P->row_count, P->row_offset, out_col, reinterpret_cast<VT*>(out_val), s0, s1, q,
       P->grab > 0 ? P->grab : numeric_grab(ctx, P, n_total), P->long_seg < 1 ? 1 : P->long_seg, LEARNED ? P->light_slot : nullptr,
       LEARNED ? P->item_count : nullptr, LEARNED ? P->row_count : nullptr, LEARNED ? P->row_failed : nullptr,
-      P->heavy_slot_base, LEARNED ? P->item_off : nullptr);
+      P->heavy_slot_base, LEARNED ? P->item_off : nullptr, split);
   note_launch();
   BCLX_CK_LAUNCH();
   return BCLX_OK;
@@ -1871,11 +1946,16 @@ static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView&
 template <typename VT>
 static int launch_numeric(Context* ctx, const SpGridView& A, const SpGridView& B, bclx_spgemm_plan_s* P,
                           int32_t* out_col, void* out_val, int s0, int s1) {
+  const bool wide = P->g.tn > 8192;
   if (P->vcap == 1024) {
-    if (P->g.tn <= 8192) return launch_numeric_w<VT, 256, false, 1024>(ctx, A, B, P, out_col, out_val, s0, s1);
+    if (!wide) return launch_numeric_w<VT, 256, false, 1024>(ctx, A, B, P, out_col, out_val, s0, s1);
     return launch_numeric_w<VT, kMaxWords, false, 1024>(ctx, A, B, P, out_col, out_val, s0, s1);
   }
-  if (P->g.tn <= 8192) return launch_numeric_w<VT, 256>(ctx, A, B, P, out_col, out_val, s0, s1);
+  if (P->split.n > 0 && s0 == 0 && s1 == (int)P->g.gk) {
+    if (!wide) return launch_numeric_w<VT, 256, false, kVcap, true>(ctx, A, B, P, out_col, out_val, s0, s1);
+    return launch_numeric_w<VT, kMaxWords, false, kVcap, true>(ctx, A, B, P, out_col, out_val, s0, s1);
+  }
+  if (!wide) return launch_numeric_w<VT, 256>(ctx, A, B, P, out_col, out_val, s0, s1);
   return launch_numeric_w<VT, kMaxWords>(ctx, A, B, P, out_col, out_val, s0, s1);
 }
 
@@ -2017,7 +2097,7 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   // the host and a memset 1.5 us of the GPU, which small products are made of)
   int64_t* sums = nullptr;
   BCLX_TRY(scratch_pieces(ctx, &P->block1, [&](Pieces& p) {
-    p.take(&P->counters, 4);
+    p.take(&P->counters, 6);
     p.take(&P->products_dev, 1);
     p.take(&P->queue, kQueueSlots);
     p.take(&P->row_count, nri);
@@ -2051,14 +2131,19 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     note_launch();
     BCLX_CK_LAUNCH();
   }
-  BCLX_TRY(read_back(ctx, {{P->counters, 8, 0}, {P->counters + 2, 8, 1}, {P->products_dev, 8, 2}}));
+  BCLX_TRY(read_back(ctx, {{P->counters, 8, 0}, {P->counters + 2, 8, 1}, {P->products_dev, 8, 2}, {P->counters + 4, 4, 3}}));
   if (live) scratch_free(ctx, live);
   BCLX_CK(cudaStreamSynchronize(ctx->stream));
-  int32_t cnts[4];
+  int32_t cnts[4], n_mid;
   std::memcpy(cnts, ctx->pinned, sizeof(cnts));
+  std::memcpy(&n_mid, ctx->pinned + 3, sizeof(n_mid));
   P->n_light = cnts[0];
-  P->n_vheavy = cnts[3];
-  P->n_heavy = cnts[1] + cnts[3];
+  // the rows between kMidHeavyUb and kVeryHeavyUb products count as very heavy
+  // where all of these are no more than SMs: then they are what a small
+  // product waits for (numeric pass, graph of 10,000 x sparse features 125 -> 70
+  // us, of 3,000 147 -> 86, R-MAT of 5,000 rows squared 166 -> 121)
+  P->n_vheavy = cnts[3] + (cnts[3] + n_mid <= ctx->num_sms ? n_mid : 0);
+  P->n_heavy = cnts[1] + cnts[3] + n_mid;
   P->products = ctx->pinned[2];
   int64_t* sums_h = nullptr;
   if (P->n_heavy > 0) {
@@ -2067,12 +2152,14 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     BCLX_TRY(ensure_side_stream(ctx));
     BCLX_TRY(build_btable(ctx, B, g, P, ctx->side));
     // heavy slots: the very heavy rows first, then the others
-    if (P->n_vheavy > 0)
-      BCLX_CK(cudaMemcpyAsync(P->heavy_list, P->vheavy_list, sizeof(int32_t) * P->n_vheavy, cudaMemcpyDeviceToDevice,
-                              ctx->stream));
-    if (cnts[1] > 0)
-      BCLX_CK(cudaMemcpyAsync(P->heavy_list + P->n_vheavy, P->heavy_tmp, sizeof(int32_t) * cnts[1],
-                              cudaMemcpyDeviceToDevice, ctx->stream));
+    int32_t* to = P->heavy_list;
+    const std::pair<const int32_t*, int32_t> lists[] = {
+        {P->vheavy_list, cnts[3]}, {P->vheavy_list + (nri - n_mid), n_mid}, {P->heavy_tmp, cnts[1]}};
+    for (const auto& l : lists) {
+      if (l.second > 0)
+        BCLX_CK(cudaMemcpyAsync(to, l.first, sizeof(int32_t) * l.second, cudaMemcpyDeviceToDevice, ctx->stream));
+      to += l.second;
+    }
     BCLX_TRY(scratch_pieces(ctx, &P->block2, [&](Pieces& p) {
       p.take(&P->heavy_bitmaps, (size_t)P->n_heavy * P->hbm_words);
       p.take(&P->heavy_span, 2 * (size_t)P->n_heavy);
@@ -2103,8 +2190,11 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     note_launch();
     BCLX_CK_LAUNCH();
     BCLX_TRY(exclusive_scan_i32_buf(ctx, P->heavy_nitems, P->heavy_first, P->n_heavy, sums_h));
-    BCLX_TRY(read_back(
-        ctx, {{P->row_offset + nri, 8, 0}, {P->counters + 2, 4, 2}, {P->heavy_first + P->n_heavy, 8, 1}}));
+    BCLX_TRY(read_back(ctx, {{P->row_offset + nri, 8, 0},
+                             {P->counters + 2, 4, 2},
+                             {P->heavy_first + P->n_heavy, 8, 1},
+                             {P->heavy_first + half_rows(ctx, P), 8, 3},
+                             {P->heavy_first + std::min((int64_t)cnts[3], P->n_vheavy), 8, 4}}));
   } else {
     BCLX_TRY(read_back(ctx, {{P->row_offset + nri, 8, 0}, {P->counters + 2, 4, 2}}));
   }
@@ -2118,6 +2208,25 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     return BCLX_ERR_INDEX_OVERFLOW;
   }
   if (P->n_heavy > 0) {
+    // the items to split by stage: all half-size ones, or those of the rows
+    // above kVeryHeavyUb
+    const int64_t stride = P->vcap / 2, most = (int64_t)ctx->num_sms * 4 * kWarpsNum / g.gk;
+    int64_t n_split = 0;
+    if (half_rows(ctx, P) > 0 && g.gk > 1 && P->vcap == kVcap && P->products <= kSplitMaxProducts)
+      n_split = ctx->pinned[3] <= most ? ctx->pinned[3] : (ctx->pinned[4] <= most ? ctx->pinned[4] : 0);
+    // (without the scratch for it, at most 5 MB, they are left whole)
+    if (n_split > 0 && scratch_pieces(ctx, &P->split_block, [&](Pieces& p) {
+          p.take(&P->split.count, (size_t)n_split);
+          p.take(&P->split.mask, (size_t)(n_split * g.gk * stride / 32));
+          p.take(reinterpret_cast<float**>(&P->split.val), (size_t)(n_split * g.gk * stride));
+        }) == BCLX_OK) {
+      P->split.n = (int)n_split;
+      P->split.stride = (int)stride;
+      BCLX_CK(cudaMemsetAsync(P->split.count, 0, sizeof(int32_t) * n_split, ctx->stream));
+    } else if (n_split > 0) {
+      cudaGetLastError();
+      P->split = SplitItems();
+    }
     BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_items, P->n_heavy_items));
     k_cut_heavy<true><<<cut_blocks, 256, 0, ctx->stream>>>(g, P->heavy_list, (int)P->n_heavy, P->heavy_bitmaps,
                                                            P->hbm_words, nullptr, P->heavy_first, P->heavy_items, P->vcap,

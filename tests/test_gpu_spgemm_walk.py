@@ -103,3 +103,41 @@ def test_few_very_heavy_rows_cut_finer(n, tile, value_type):
     A, B = SPMatrix.from_csr(a, BlockCustom((16, 300))), SPMatrix.from_csr(b, BlockCustom((300, tile)))
     rp, ci, cv = O.gemm_tiled(a, b, 16, 300, tile, mode=value_type)
     assert_csr_identical(spgemm(A, B).get(), rp, ci, cv)
+
+
+@pytest.mark.parametrize("value_type", ["f32", "i32"])
+@pytest.mark.parametrize("n_mid,n_most,grid_k", [(3, 0, 4), (0, 2, 4), (60, 2, 5), (60, 2, 40), (200, 1, 3), (2, 1, 1)])
+def test_items_split_by_stage(n_mid, n_most, grid_k, value_type):
+    """Rows above 8192 products and above 32768, few or many of each, on one to
+    40 tiles along k (with and without a stage map): their items' stages run
+    apart and are added in order.  The numeric pass twice on one plan, the
+    second time with other values; signed zeros among them."""
+    from bcl_b200.containers import BlockCustom, SPMatrix, spgemm_numeric, spgemm_symbolic
+    import torch
+    rng = np.random.default_rng(n_mid * 10 + grid_k)
+    k, n, per = 800, 1500, 60
+
+    def vals(count):
+        if value_type == "i32":
+            return rng.integers(-2**31, 2**31, count).astype(np.int32)
+        v = rng.uniform(-1, 1, count).astype(np.float32)
+        v[rng.random(count) < 0.05] = -0.0
+        return v
+
+    lens = [2] * 30 + [200] * n_mid + [5] * 10 + [700] * n_most + [40] * 5
+    a = _csr(len(lens), k, [np.sort(rng.choice(k, c, replace=False)) for c in lens], vals)
+    b = _csr(k, n, [np.sort(rng.choice(n, per, replace=False)) for _ in range(k)], vals)
+    tk = -(-k // grid_k)
+    A, B = SPMatrix.from_csr(a, BlockCustom((len(lens), tk))), SPMatrix.from_csr(b, BlockCustom((tk, n)))
+    plan, out, trp, toff, nnz = spgemm_symbolic(A, B)
+    ci = torch.empty(nnz, dtype=torch.int32, device="cuda")
+    v = torch.empty(nnz, dtype=A.vals.dtype, device="cuda")
+    out.col_ind, out.vals = ci.data_ptr(), v.data_ptr()
+    for _ in range(2):
+        spgemm_numeric(plan, A, B, out)
+        C = SPMatrix(a.m, n, len(lens), n, a.vals.dtype, 0, trp, toff, ci, v)
+        rp, cols, cv = O.gemm_tiled(a, b, len(lens), tk, n, mode=value_type)
+        assert_csr_identical(C.get_host_gather() if value_type == "i32" else C.get(), rp, cols, cv)
+        a.vals[:] = vals(a.nnz)
+        A = SPMatrix.from_csr(a, BlockCustom((len(lens), tk)))
+    plan.close()
