@@ -67,7 +67,7 @@ constexpr int64_t kSplitMaxProducts = 40 << 20;  // largest product whose items 
 // 30.3, 30.4, 30.6; graph x sparse features 983, 492, 494, 502, 498 us.
 constexpr int kLongSegDefault = 14;
 constexpr int kQueueSlots = 256;          // work-queue heads in a plan: one per stage launch (at most 254), and
-constexpr int kClassifySlot = 254, kSymbolicSlot = 255;  // the planning passes' (each used once)
+constexpr int kSymbolicSlot = 255;        // the symbolic pass' (used once)
 constexpr int64_t kMidHeavyUb = 8192;    // from here on where such rows are few (see symbolic_impl)
 constexpr int64_t kVeryHeavyUb = 32768;  // rows above this many products get a whole block in the symbolic pass
 
@@ -685,8 +685,7 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
   if (lane == 0 && mine) atomicAdd(products, mine);
 }
 
-// Products of every row for all of its C tiles at once, where no stage map
-// is in use (coarse grids): a warp takes a row of A's tile row ti, reads its
+// Products of every row for all of its C tiles at once: a warp takes a row of A's tile row ti, reads its
 // entries once, and for each tile column j adds up the lengths of the B_kj
 // rows they name; lane j holds the row's products in C tile (ti, j).  Taking
 // each C tile's row by itself (k_classify) reads the entries once per tile
@@ -697,6 +696,15 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
 // its other rows, its chunks dealt to the warps (a hub row is hundreds of
 // chunks of dependent loads); neighbouring rows, which hubs are, go to
 // different blocks.
+// With a stage map (n_stages, the stages of all C tiles) it is for the maps that
+// are at least half full, where there are rows enough to keep every resident warp
+// busy (kClassifyMinRows), and k_classify_tiles for the others.  R-MAT s18 on 64x64
+// tiles 7.8 ms by rows, 14.6 by tiles, 12.8 with a warp for each row item; s17 on 32x32 1.61,
+// 2.27, 2.11; R-MAT of 5,000 rows on 40x40 340, 106, 173 us.
+__device__ __forceinline__ bool mostly_full(const Geom& g, const unsigned long long* n_stages) {
+  return 2 * __ldg(n_stages) >= (unsigned long long)(g.gm * g.gn * g.gk);
+}
+constexpr int kClassifyMinRows = 256;  // per SM, with a stage map
 constexpr int kClassifyKeep = 8;    // rows whose items a warp keeps before it appends them
 constexpr int kClassifyCols = 8;    // tile columns whose loads are in flight
 constexpr int kClassifyLong = 512;
@@ -704,11 +712,12 @@ constexpr int kClassifyDefer = 64;  // long rows a block can put off
 __global__ void __launch_bounds__(256) k_classify_rows(
     SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
     int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
-    int heavy_min_cols, int light_ub) {  // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list
+    int heavy_min_cols, int light_ub, const unsigned long long* __restrict__ n_stages) {  // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list
   __shared__ int32_t kept_all[8][4][kClassifyKeep * 32];
   __shared__ unsigned long long sums[32];
   __shared__ uint32_t deferred[kClassifyDefer];
   __shared__ int n_deferred;
+  if (n_stages && !mostly_full(g, n_stages)) return;
   const int wid = threadIdx.x >> 5;
   int32_t(*kept)[kClassifyKeep * 32] = kept_all[wid];
   const int lane = lane_id();
@@ -881,6 +890,111 @@ __global__ void __launch_bounds__(kBtableRows) k_btable(SpGridView B, Geom g, in
   }
 }
 
+// Products of every row of the C tiles that have stages (live[0..*n_live)),
+// for grids with a stage map: a warp takes 32 rows of one C tile, a lane each,
+// and goes through the tile's stages together; an A-row segment longer than
+// kClassifyLane is taken by all lanes.  A fine grid's rows have a few entries
+// per tile: a warp for each row item (k_classify) was bound by issue at some 440
+// instructions for it.  27-point stencil on 128^3, 10.4M row items of 1.8
+// stages: 4.70 -> 0.34 ms.
+constexpr int kClassifyLane = 16;
+__global__ void __launch_bounds__(256) k_classify_tiles(
+    SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
+    int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
+    int heavy_min_cols, int light_ub, const int32_t* __restrict__ live, const int32_t* __restrict__ n_live,
+    const unsigned long long* __restrict__ n_stages) {
+  __shared__ unsigned long long sums[8];
+  if (n_stages && mostly_full(g, n_stages)) return;  // k_classify_rows'
+  const int lane = lane_id();
+  const unsigned below = (1u << lane) - 1u;
+  const uint32_t per_tile = (uint32_t)((g.tm + 31) / 32);  // groups of 32 rows
+  const int64_t n_groups = (int64_t)__ldg(n_live) * per_tile;
+  unsigned long long mine = 0;
+  // (in order, for the lists keep near rows together, which the passes over them re-read in L2)
+  for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < n_groups; w += (int64_t)gridDim.x * 8) {
+    const int64_t t = __ldg(live + w / per_tile);
+    const int64_t ti = t / g.gn, tj = t - ti * g.gn;
+    const int64_t r = (w % per_tile) * 32 + lane;
+    const bool in = r < A.rows_of(ti);
+    const int rot = tile_rotation(g, ti, tj);
+    const int ns = stage_count(g, ti, tj);
+    int64_t tot = 0;
+    for (int g0 = 0; g0 < ns; g0 += 32) {
+      // one lane per stage: the tiles' pointers
+      const int32_t* my_arp = nullptr;
+      const int32_t* my_aci = nullptr;
+      const int32_t* my_brp = nullptr;
+      if (g0 + lane < ns) {
+        const int64_t k = stage_k(g, stage_at(g, ti, tj, g0 + lane), rot);
+        const bclx_csr_t At = A.tile(ti, k);
+        my_arp = At.row_ptr;
+        my_aci = At.col_ind;
+        my_brp = B.tile(k, tj).row_ptr;
+      }
+      const int n = min(32, ns - g0);
+      auto bounds = [&](int st, int32_t& b, int32_t& e) {
+        const int32_t* arp = shfl_ptr(my_arp, st);
+        b = in ? __ldg(arp + r) : 0;
+        e = in ? __ldg(arp + r + 1) : 0;
+      };
+      int32_t nb, ne;
+      bounds(0, nb, ne);
+      for (int st = 0; st < n; st++) {
+        const int32_t as = nb, len = ne - nb;
+        if (st + 1 < n) bounds(st + 1, nb, ne);  // the next stage's, in flight
+        const int32_t* aci = shfl_ptr(my_aci, st);
+        const int32_t* brp = shfl_ptr(my_brp, st);
+        const bool longer = len > kClassifyLane;
+        const int few = longer ? 0 : len;
+        const int most = __reduce_max_sync(kFull, few);
+        int32_t sum = 0;  // (at most kClassifyLane B rows; a B tile row has fewer than 2^16 columns)
+        for (int q = 0; q < most; q += 4) {
+          int32_t kc[4];
+#pragma unroll
+          for (int u = 0; u < 4; u++) kc[u] = q + u < few ? __ldg(aci + as + q + u) : -1;
+#pragma unroll
+          for (int u = 0; u < 4; u++)
+            if (kc[u] >= 0) sum += __ldg(brp + kc[u] + 1) - __ldg(brp + kc[u]);
+        }
+        tot += sum;
+        for (unsigned m = __ballot_sync(kFull, longer); m; m &= m - 1) {
+          const int src = __ffs(m) - 1;
+          const int32_t s0 = __shfl_sync(kFull, as, src), s1 = s0 + __shfl_sync(kFull, len, src);
+          int64_t part = 0;
+          for (int32_t q = s0 + lane; q < s1; q += 32) {
+            const int32_t kc = __ldg(aci + q);
+            part += __ldg(brp + kc + 1) - __ldg(brp + kc);
+          }
+          part = warp_sum(part);
+          if (lane == src) tot += part;
+        }
+      }
+    }
+    const int64_t wd = min(g.n - tj * g.tn, g.tn);
+    mine += (unsigned long long)tot;
+    int cls = -1;  // light, heavy, very heavy, above kMidHeavyUb
+    if (tot > 0) cls = tot <= light_ub && wd < heavy_min_cols ? 0 : (tot <= kMidHeavyUb ? 1 : (tot <= kVeryHeavyUb ? 3 : 2));
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      const unsigned m = __ballot_sync(kFull, cls == c);
+      if (m == 0) continue;
+      int pos = 0;
+      if (lane == 0) pos = atomicAdd(&counters[c < 2 ? c : c + 1], __popc(m));
+      pos = __shfl_sync(kFull, pos, 0) + __popc(m & below);
+      int32_t* const list = c == 0 ? light_list : (c == 1 ? heavy_list : vheavy_list);
+      if (cls == c) list[c == 3 ? g.n_row_items - 1 - pos : pos] = (int32_t)(t * g.tm + r);
+    }
+  }
+  const unsigned long long s = warp_sum(mine);
+  if (lane == 0) sums[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long all = 0;
+    for (int q = 0; q < 8; q++) all += sums[q];
+    if (all) atomicAdd(products, all);
+  }
+}
+
 // ---- symbolic ----------------------------------------------------------------------
 
 // Symbolic pass.  Heavy rows are numbered 0..n_heavy-1 (the very heavy ones
@@ -1015,6 +1129,89 @@ __global__ void __launch_bounds__(kWarpsSym * 32)
     }
     __syncthreads();
   }
+}
+
+// Row offsets, tile_row_ptr and tile_offset by tile, for grids with a stage map
+// of at least as many tiles as SMs: a block per tile adds up its rows
+// (k_tile_sums), the sums are scanned into tile_offset, and a block per tile
+// scans its rows and writes both arrays (k_tile_rows).  Tiles without stages
+// are not read, and their row offsets, which nothing reads, not written: the
+// scan over all row items and k_tile_ptrs go through 24 bytes of every row item
+// where this goes through 4.  27-point stencil on 128^3, 268M row items, 634 of
+// 16,384 tiles with stages: 3.07 -> 0.48 ms.
+__global__ void __launch_bounds__(256) k_tile_sums(Geom g, const int32_t* __restrict__ row_count,
+                                                   int64_t* __restrict__ tile_sum) {
+  __shared__ int64_t sums[8];
+  const int64_t ntiles = g.gm * g.gn;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    int64_t v = 0;
+    if (g.scount[t] > 0)
+      for (int64_t r = threadIdx.x; r < g.tm; r += 256) v += __ldg(row_count + t * g.tm + r);
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int q = 1; q < 8; q++) v += sums[q];
+      tile_sum[t] = v;
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) k_tile_rows(Geom g, const int32_t* __restrict__ row_count,
+                                                   const int64_t* __restrict__ tile_offset,
+                                                   int64_t* __restrict__ row_offset, int32_t* __restrict__ tile_row_ptr,
+                                                   int32_t* __restrict__ overflow) {
+  __shared__ int64_t before[8];
+  __shared__ int64_t carry;
+  const int lane = lane_id(), wid = threadIdx.x >> 5;
+  const int64_t ntiles = g.gm * g.gn;
+  for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    int32_t* const ptr = tile_row_ptr + t * (g.tm + 1);
+    if (g.scount[t] <= 0) {
+      for (int64_t r = threadIdx.x; r <= g.tm; r += 256) ptr[r] = 0;
+      continue;
+    }
+    const int64_t start = tile_offset[t];
+    if (threadIdx.x == 0) {
+      ptr[0] = 0;
+      if (tile_offset[t + 1] - start > INT32_MAX) *overflow = 1;
+    }
+    int64_t base = 0;  // outputs of the rows before the chunk
+    for (int64_t r0 = 0; r0 < g.tm; r0 += 1024) {
+      // four rows per thread, r0 + 4 * thread ..
+      const int64_t r = r0 + 4 * threadIdx.x;
+      int32_t c[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) c[q] = r + q < g.tm ? __ldg(row_count + t * g.tm + r + q) : 0;
+      const int64_t mine = (int64_t)c[0] + c[1] + c[2] + c[3];
+      const int64_t incl = warp_inclusive_scan(mine);
+      if (lane == 31) before[wid] = incl;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        int64_t run = base;
+        for (int q = 0; q < 8; q++) {
+          const int64_t v = before[q];
+          before[q] = run;
+          run += v;
+        }
+        carry = run;
+      }
+      __syncthreads();
+      int64_t at = before[wid] + incl - mine;
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        if (r + q < g.tm) {
+          row_offset[t * g.tm + r + q] = start + at;
+          at += c[q];
+          ptr[r + q + 1] = (int32_t)at;
+        }
+      }
+      base = carry;
+      __syncthreads();
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) row_offset[g.n_row_items] = tile_offset[ntiles];
 }
 
 // tile_row_ptr / tile_offset from the row offsets (rows are tile-major).
@@ -1978,17 +2175,23 @@ __global__ void k_stage_map(SpGridView A, SpGridView B, Geom g, int32_t* __restr
 }
 
 // C tiles with at least one stage (scount[t] > 0) into live[], their number
-// to *n_live (one atomic per warp; the order is immaterial).
+// to *n_live (one atomic per warp; the order is immaterial), the stages of all
+// to *n_stages.
 __global__ void k_live_tiles(const int32_t* __restrict__ scount, int64_t nt, int32_t* __restrict__ live,
-                             int32_t* __restrict__ n_live) {
+                             int32_t* __restrict__ n_live, unsigned long long* __restrict__ n_stages) {
   const int lane = lane_id();
   const int64_t end = (nt + 31) & ~int64_t(31);  // whole warps run every iteration
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < end; t += (int64_t)gridDim.x * blockDim.x) {
-    const bool on = t < nt && scount[t] > 0;
+    const int c = t < nt ? scount[t] : 0;
+    const bool on = c > 0;
     const unsigned m = __ballot_sync(kFull, on);
     if (m == 0) continue;
+    const int sum = __reduce_add_sync(kFull, c);
     int base = 0;
-    if (lane == 0) base = atomicAdd(n_live, __popc(m));
+    if (lane == 0) {
+      base = atomicAdd(n_live, __popc(m));
+      atomicAdd(n_stages, (unsigned long long)sum);
+    }
     base = __shfl_sync(kFull, base, 0);
     if (on) live[base + __popc(m & ((1u << lane) - 1u))] = (int32_t)t;
   }
@@ -2011,15 +2214,18 @@ static int build_stage_map(Context* ctx, const SpGridView& A, const SpGridView& 
 }
 
 // With a stage map: the C tiles that have stages, into a new scratch array
-// (their number in its last slot, written by the device); *live stays null
-// without a map (every tile is walked).
+// (their number in slot gm*gn and their stages, 64 bits, in slot live_stages_at,
+// written by the device); *live stays null without a map (every tile is walked).
+static int64_t live_stages_at(int64_t nt) { return (nt + 2) & ~int64_t(1); }
 static int build_live_tiles(Context* ctx, const Geom& g, int32_t** live) {
   *live = nullptr;
   if (!g.scount) return BCLX_OK;
   const int64_t nt = g.gm * g.gn;
-  BCLX_TRY(scratch_alloc_n(ctx, live, (size_t)nt + 1));
-  BCLX_CK(cudaMemsetAsync(*live + nt, 0, sizeof(int32_t), ctx->stream));
-  k_live_tiles<<<grid_for(ctx, nt / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(g.scount, nt, *live, *live + nt);
+  const int64_t at = live_stages_at(nt);
+  BCLX_TRY(scratch_alloc_n(ctx, live, (size_t)at + 2));
+  BCLX_CK(cudaMemsetAsync(*live + nt, 0, sizeof(int32_t) * (at + 2 - nt), ctx->stream));
+  k_live_tiles<<<grid_for(ctx, nt / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
+      g.scount, nt, *live, *live + nt, reinterpret_cast<unsigned long long*>(*live + at));
   note_launch();
   BCLX_CK_LAUNCH();
   return BCLX_OK;
@@ -2116,19 +2322,21 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   P->light_ub_max = (int)tuning(ctx, BCLX_TUNE_LIGHT_UB);
   P->vcap = (int)tuning(ctx, BCLX_TUNE_ITEM_OUTPUTS);
   int32_t* live = nullptr;  // C tiles with stages (when the stage map says which)
-  if (nri > 0 && !g.scount) {
-    k_classify_rows<<<grid_for(ctx, g.gm * g.tm, 8, 8), 256, 0, ctx->stream>>>(
-        A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,
-        P->light_ub_max);
-    note_launch();
-    BCLX_CK_LAUNCH();
-  } else if (nri > 0) {
-    const int64_t nt = g.gm * g.gn;
+  if (nri > 0) {
     BCLX_TRY(build_live_tiles(ctx, g, &live));
-    k_classify<false><<<grid_for(ctx, nri, 8, 16), 256, 0, ctx->stream>>>(
-        A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols, P->light_ub_max,
-        nullptr, nullptr, P->queue + kClassifySlot, queue_grab(ctx, nri, 8, 16, 32, 8), live, live ? live + nt : nullptr);
-    note_launch();
+    const int64_t nt = g.gm * g.gn;
+    // (few rows: see k_classify_rows)
+    const bool rows = !live || g.gm * g.tm >= (int64_t)ctx->num_sms * kClassifyMinRows;
+    const auto* n_stages = live ? reinterpret_cast<const unsigned long long*>(live + live_stages_at(nt)) : nullptr;
+    if (rows)
+      k_classify_rows<<<grid_for(ctx, g.gm * g.tm, 8, 8), 256, 0, ctx->stream>>>(
+          A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,
+          P->light_ub_max, n_stages);
+    if (live)
+      k_classify_tiles<<<grid_for(ctx, nri / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
+          A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,
+          P->light_ub_max, live, live + nt, rows ? n_stages : nullptr);
+    note_launch((rows ? 1 : 0) + (live ? 1 : 0));
     BCLX_CK_LAUNCH();
   }
   BCLX_TRY(read_back(ctx, {{P->counters, 8, 0}, {P->counters + 2, 8, 1}, {P->products_dev, 8, 2}, {P->counters + 4, 4, 3}}));
@@ -2174,12 +2382,23 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     BCLX_CK(cudaEventRecord(ctx->join_ev, ctx->side));
     BCLX_CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
   }
-  BCLX_TRY(exclusive_scan_i32_buf(ctx, P->row_count, P->row_offset, nri, sums));
   const int64_t ntiles = g.gm * g.gn;
-  k_tile_ptrs<<<grid_for(ctx, ntiles * (g.tm + 1) / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
-      g, P->row_offset, tile_row_ptr, tile_offset, P->counters + 2);
-  note_launch();
-  BCLX_CK_LAUNCH();
+  if (g.scount && ntiles >= ctx->num_sms) {
+    int64_t* const tile_sum = P->row_offset;  // (its entries are written later)
+    const unsigned blocks = (unsigned)std::min<int64_t>(ntiles, (int64_t)ctx->num_sms * 8);
+    k_tile_sums<<<blocks, 256, 0, ctx->stream>>>(g, P->row_count, tile_sum);
+    BCLX_TRY(exclusive_scan_i64(ctx, tile_sum, tile_offset, ntiles));
+    k_tile_rows<<<blocks, 256, 0, ctx->stream>>>(g, P->row_count, tile_offset, P->row_offset, tile_row_ptr,
+                                                 P->counters + 2);
+    note_launch(2);
+    BCLX_CK_LAUNCH();
+  } else {
+    BCLX_TRY(exclusive_scan_i32_buf(ctx, P->row_count, P->row_offset, nri, sums));
+    k_tile_ptrs<<<grid_for(ctx, ntiles * (g.tm + 1) / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
+        g, P->row_offset, tile_row_ptr, tile_offset, P->counters + 2);
+    note_launch();
+    BCLX_CK_LAUNCH();
+  }
   // rows per warp: as many as leave every resident warp some
   const int per_warp = (int)std::max<int64_t>(1, std::min<int64_t>(32, P->n_heavy / ((int64_t)ctx->num_sms * 64)));
   const unsigned cut_blocks = grid_for(ctx, ceil_div(P->n_heavy, (int64_t)per_warp), 8, 8);

@@ -61,3 +61,47 @@ def test_against_oracle(name, value_type):
         assert st["heavy_items"] > st["heavy_rows"] > 0
     rp, ci, cv = O.gemm_tiled(a, b, *tiles, mode=value_type)
     assert_csr_identical(C.get(), rp, ci, cv)
+
+
+def band(n, width):
+    rows = [np.arange(max(0, i - width), min(n, i + width + 1)) for i in range(n)]
+    return [r.size for r in rows], np.concatenate(rows).astype(np.int32)
+
+
+@pytest.mark.parametrize("value_type", ["f32", "i32"])
+@pytest.mark.parametrize("name", ["band", "band_one_row_tiles", "full_few_rows", "full_many_rows", "few_tiles", "empty"])
+def test_fine_grids(name, value_type):
+    """Grids of 17 stages and more, which have a stage map: few of the C tiles
+    with stages and all of them, with few rows and many, tile heights off 32
+    and of 1, A-row segments of 16, 17 and more entries in a tile, fewer C
+    tiles than SMs, no stages at all."""
+    from bcl_b200.containers import BlockCustom, SPMatrix, spgemm
+    rng = np.random.default_rng(len(name))
+    if name.startswith("band"):
+        n, width, tile = (2000, 12, 33) if name == "band" else (150, 20, 1)
+        mats = []
+        for _ in range(2):
+            lens, ci = band(n, width)
+            m = random_csr(lens, n, rng, value_type)
+            m.col_ind[:] = ci
+            mats.append(m)
+        a, b, tiles = mats[0], mats[1], (tile, tile, tile)
+    elif name == "full_few_rows":
+        a = random_csr([5, 0, 380, 40] * 100, 400, rng, value_type)
+        b, tiles = random_csr([30] * 400, 400, rng, value_type), (20, 20, 20)
+    elif name == "full_many_rows":
+        a = random_csr([8] * 39990, 136, rng, value_type)
+        b, tiles = random_csr([6] * 136, 100, rng, value_type), (2353, 8, 10)
+    elif name == "few_tiles":
+        a = random_csr([100, 900, 3] * 20, 1000, rng, value_type)
+        b, tiles = random_csr([20] * 1000, 300, rng, value_type), (60, 25, 300)
+    else:
+        a = random_csr([0] * 100, 100, rng, value_type)
+        b, tiles = random_csr([3] * 100, 100, rng, value_type), (5, 5, 5)
+    A, B = SPMatrix.from_csr(a, BlockCustom(tiles[:2])), SPMatrix.from_csr(b, BlockCustom(tiles[1:]))
+    C, plan = spgemm(A, B, keep_plan=True)
+    st = plan.stats()
+    plan.close()
+    assert st["products"] == gen.intermediate_products(a, b)
+    rp, ci, cv = O.gemm_tiled(a, b, *tiles, mode=value_type)
+    assert_csr_identical(C.get(), rp, ci, cv)
