@@ -88,27 +88,14 @@ struct Vec<__nv_bfloat16> {
 
 constexpr int kSpmmUnroll = 4;  // B-row loads in flight per lane (with 32 warps per SM)
 
-// Ask L2 for the 128-byte lines of [p, p + bytes) (no-op for null).
-__device__ __forceinline__ void l2_prefetch_slice(const void* p, int bytes) {
-  if (p == nullptr) return;
-  const char* q = reinterpret_cast<const char*>(p);
-  for (int o = 0; o < bytes; o += 128) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(q + o));
-}
-
 constexpr int kSpmmMaxRows = 4;  // rows of one C tile a warp walks together
-constexpr int kARing = 4;        // A-entry staging slots (chunks of 32 entries) per warp
-constexpr int kTabBufs = 3;      // entry-table buffers per warp: applied, next, being built
 
 // Per-warp shared memory of the walk:
-//  * entry tables: per chunk of 32 entries, (B-row address, A value, row) of
-//    each entry, read back with broadcast 16-byte loads;
-//  * A staging ring: the (column, value) pair of each entry, copied by
-//    cp.async kARing - 1 chunks ahead, with the entry's stage lane;
+//  * the entry table of a chunk of 32 entries: (B-row address, A value, row) of
+//    each, read back with broadcast 16-byte loads;
 //  * C staging: the C row slices the item updates (one 16-byte vector per
 //    lane and row), copied by cp.async while the A and B loads are in flight.
-__shared__ uint4 spmm_tables[kSpmmWarps * kTabBufs * 32];
-__shared__ uint2 spmm_aring[kSpmmWarps * kARing * 32];
-__shared__ uint8_t spmm_asrc[kSpmmWarps * kARing * 32];
+__shared__ uint4 spmm_tables[kSpmmWarps * 32];
 __shared__ uint4 spmm_cstage[kSpmmWarps * kSpmmMaxRows * 32];
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -179,16 +166,18 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 // One warp per (R consecutive rows of C tile (ti, tj) from r0, panel of 32
 // 16-byte vectors from column c0).  The A entries of the rows' stages are
 // flattened (row by row, each row's stages in rotated order) and taken in
-// chunks of 32, one entry per lane, through a software pipeline:
-//   * chunk c + kARing + 1: each lane finds its entry's stage and copies the
-//     entry's (column, value) into the warp's staging ring by cp.async;
-//   * chunk c + 2: each lane turns its staged entry into a table entry
-//     (B-row address, value, row) and asks L2 for that B-row slice;
-//   * chunk c: the warp reads the table UNROLL entries at a time, so that
-//     many B-row loads (raw 16-byte vectors) are in flight before their
-//     multiply-adds are applied in entry order.
-// No load result is waited for before it is used, so the A loads of later
-// chunks never stall the current one.  A row's chain starts from its C
+// chunks of 32, one entry per lane: each lane turns its entry into a table entry
+// (B-row address, value, row) and loads its entry of the next chunk; the warp
+// reads the table UNROLL entries at a time, so that many B-row loads (raw
+// 16-byte vectors) are in flight before their multiply-adds are applied in
+// entry order.  The loads in flight are what the registers of 32 warps per SM
+// hold, 10 MB over the GPU, which is enough for DRAM.  Asking L2 for the B-row
+// slices of the next two chunks as well put 155 MB in flight, more than L2: the
+// lines were evicted before their use.  Without it, and without the A entries'
+// staging through shared memory, uniform matrix of 1,000,000 rows x 256 BF16
+// 1.66 -> 1.31 ms, of 300,000 x 256 FP32 885 -> 703 us, stencil of 512,000 x 128 574
+// -> 496, R-MAT s21 x 256 FP32 (with k_spmm_long) 4.11 -> 3.52 ms.
+// A row's chain starts from its C
 // value, staged in shared memory by cp.async once the row is known to have
 // entries; rows without entries are not touched.  R > 1 needs R * gk <= 32
 // (one lane per (row, stage)); R == 1 takes the stages 32 at a time.
@@ -210,12 +199,8 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
   const bool own = col < W;
   const int bcol = own ? col : 0;  // lanes past the tile edge load column 0 (in bounds) and store nothing
   const int wib = threadIdx.x >> 5;
-  uint4* tb = spmm_tables + wib * (kTabBufs * 32);
-  uint2* ar = spmm_aring + wib * (kARing * 32);
-  uint8_t* asrc = spmm_asrc + wib * (kARing * 32);
+  uint4* tb = spmm_tables + wib * 32;
   uint4* cs = spmm_cstage + wib * (kSpmmMaxRows * 32);
-  // bytes of this warp's panel in one B row
-  const int pbytes = min(32 * VN, W - c0) * (int)sizeof(ST);
   const int gk = (int)A.gn;
   float acc[VN];
   int cur = -1;  // row whose chain is in acc
@@ -267,71 +252,51 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
         if (vec && own && hi > lo) cp_async16(cs + q * 32 + lane, crow0 + q * C.ld + col);
       }
     }
-    const int32_t nch = (atot + 31) >> 5;
-    // chunk x: each lane's entry x*32 + lane into ring slot x % kARing (one
-    // commit group per chunk, empty past the end)
-    auto issue_a = [&](int32_t x) {
-      if (x < nch) {
-        const int32_t e = x * 32 + lane;
-        int src = 0;
+    // each lane's entry of chunk e0 / 32, loaded while the chunk before is
+    // applied (past the end: none)
+    int32_t nkc = 0;
+    float nval = 0.f;
+    int nsrc = 0;
+    auto fetch = [&](int32_t e0) {
+      const int32_t e = e0 + lane;
+      int src = 0;
 #pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-          const int32_t t = __shfl_sync(kFull, aincl, src + step - 1);
-          if (t <= e) src += step;
-        }
-        src = min(src, 31);
-        const int32_t off = e - __shfl_sync(kFull, aexcl, src);
-        const int32_t* sacol = reinterpret_cast<const int32_t*>(
-            __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
-        const float* saval = reinterpret_cast<const float*>(
-            __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
-        const int slot = (x % kARing) * 32 + lane;
-        asrc[slot] = (uint8_t)src;
-        if (e < atot) {
-          cp_async4_nb(&ar[slot].x, sacol + off);
-          cp_async4_nb(&ar[slot].y, saval + off);
-        }
+      for (int step = 16; step >= 1; step >>= 1) {
+        const int32_t t = __shfl_sync(kFull, aincl, src + step - 1);
+        if (t <= e) src += step;
       }
-      cp_async_commit();
-    };
-    // chunk x (staged): table entries and L2 requests for the B-row slices.
-    // Entries past the end point at the last entry's B row with value 0 (an
-    // in-bounds load whose product is never applied).
-    auto build = [&](int32_t x) {
-      if (x >= nch) return;
-      const int slot = (x % kARing) * 32 + lane;
-      const int src = asrc[slot];
-      const ST* sbt = reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), src));
-      const int32_t e = x * 32 + lane;
-      float v = 0.f;
-      const ST* brow = sbt;
+      nsrc = src;
+      const int32_t off = e - __shfl_sync(kFull, aexcl, src);
+      const int32_t* sacol = reinterpret_cast<const int32_t*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
+      const float* saval = reinterpret_cast<const float*>(
+          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
       if (e < atot) {
-        const uint2 a = ar[slot];
-        v = __uint_as_float(a.y);
-        brow = sbt + (int64_t)(int32_t)a.x * B.ld;
+        nkc = __ldg(sacol + off);
+        nval = __ldg(saval + off);
       }
-      const ST* last = reinterpret_cast<const ST*>(
-          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(brow), (atot - 1) & 31));
-      if (e >= atot) brow = last;
-      const uint64_t pa = reinterpret_cast<uint64_t>(brow);
-      tb[(x % kTabBufs) * 32 + lane] =
-          make_uint4((uint32_t)pa, (uint32_t)(pa >> 32), __float_as_uint(v), GROUP ? (uint32_t)(src / gk) : 0u);
-      l2_prefetch_slice(vec && e < atot ? brow + c0 : nullptr, pbytes);
     };
-    // pipeline fill: chunks 0 .. kARing-1 staged, 0 and 1 built, kARing staged
-    for (int x = 0; x < kARing; x++) issue_a(x);
-    cp_async_wait_group<kARing - 2>();
-    build(0);
-    build(1);
-    issue_a(kARing);
-    __syncwarp();
+    fetch(0);
     if (!GROUP && cur < 0) enter(0);
-    for (int32_t c = 0; c < nch; c++) {
-      issue_a(c + kARing + 1);
-      cp_async_wait_group<kARing - 1>();
-      build(c + 2);
-      const int ne = min(32, atot - c * 32);
-      const uint4* t = tb + (c % kTabBufs) * 32;
+    for (int32_t e0 = 0; e0 < atot; e0 += 32) {
+      const int ne = min(32, atot - e0);
+      // the chunk's table.  Entries past the end point at the last entry's B
+      // row (an in-bounds load whose product is never applied).
+      const ST* brow = reinterpret_cast<const ST*>(
+                           __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), nsrc)) +
+                       (int64_t)nkc * B.ld;
+      const uint64_t pa = __shfl_sync(kFull, reinterpret_cast<unsigned long long>(brow), min(lane, ne - 1));
+      const int row = GROUP ? nsrc / gk : 0;
+      tb[lane] = make_uint4((uint32_t)pa, (uint32_t)(pa >> 32), __float_as_uint(nval), (uint32_t)row);
+      // entries that begin a row
+      unsigned heads = 0;
+      if (GROUP) {
+        const int before = __shfl_up_sync(kFull, row, 1);
+        heads = __ballot_sync(kFull, row != (lane == 0 ? cur : before));
+      }
+      __syncwarp();
+      if (e0 + 32 < atot) fetch(e0 + 32);
+      const uint4* t = tb;
       if (vec) {
         for (int u0 = 0; u0 < ne; u0 += UNROLL) {
           uint4 ent[UNROLL];
@@ -344,20 +309,23 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
             raw[u] = __ldg(reinterpret_cast<const uint4*>(rp + bcol));
           }
           auto apply = [&](int u) {
-            if (GROUP && (int)ent[u].w != cur) enter((int)ent[u].w);
             float b[VN];
             V::unpack_raw(raw[u], b);
             const float vs = __uint_as_float(ent[u].z);
 #pragma unroll
             for (int x = 0; x < VN; x++) acc[x] = __fmaf_rn(vs, b[x], acc[x]);
           };
-          if (u0 + UNROLL <= ne) {  // whole group: no test between the loads and their use
+          if (u0 + UNROLL <= ne && ((heads >> u0) & ((1u << UNROLL) - 1u)) == 0u) {
+            // a whole group of one row: no test between the loads and their use
 #pragma unroll
             for (int u = 0; u < UNROLL; u++) apply(u);
           } else {
 #pragma unroll
             for (int u = 0; u < UNROLL; u++)
-              if (u0 + u < ne) apply(u);
+              if (u0 + u < ne) {
+                if (GROUP && ((heads >> (u0 + u)) & 1u)) enter((int)ent[u].w);
+                apply(u);
+              }
           }
         }
       } else {
@@ -392,6 +360,12 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
   unsigned long long it = 0;
   if (lane == 0) it = atomicAdd(next_item, 1ULL);
   it = __shfl_sync(kFull, it, 0);
+  // item numbers and their parts: 32-bit divisions where they all fit (a 64-bit
+  // one is some 70 instructions)
+  const bool small = n_items <= UINT32_MAX;
+  auto divide = [small](int64_t a, int64_t b) { return small ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b; };
+  int64_t at = -1;  // the C tile `aligned` is for
+  bool aligned = false;
   while (it < (unsigned long long)n_items) {
     unsigned long long nx = 0;
     if (lane == 0) nx = atomicAdd(next_item, 1ULL);
@@ -399,20 +373,24 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     int64_t rg;
     int panel;
     if (panel_major) {  // all row groups of panel 0, then of panel 1, ...
-      const int64_t n_rg = n_items / npanels;
-      panel = (int)(item / n_rg);
+      const int64_t n_rg = divide(n_items, npanels);
+      panel = (int)divide(item, n_rg);
       rg = item - panel * n_rg;
     } else {  // the panels of a row group one after another
-      rg = item / npanels;
+      rg = divide(item, npanels);
       panel = (int)(item - rg * npanels);
     }
-    const int64_t t = rg / ngroups;
+    const int64_t t = divide(rg, ngroups);
     const int64_t r0 = (rg - t * ngroups) * R;
-    const int64_t ti = t / tjn, tj = t - ti * tjn;
+    const int64_t ti = divide(t, tjn), tj = t - ti * tjn;
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
-      const bool vec = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+      if (t != at) {
+        aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+        at = t;
+      }
+      const bool vec = aligned;
       // rows flagged long are k_spmm_long's (it takes the aligned ones)
       spmm_rows<ST, GROUP, SUB>(A, B, C, ti, tj, r0, R, c0, W, vec, vec ? long_flag : nullptr);
     }
@@ -428,19 +406,19 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
 // A row with thousands of entries is one chain of multiply-adds per output
 // element (the reference's order): it cannot be split, only fed faster.  Such
 // rows are found first (k_spmm_find_long), skipped by k_spmm and run by
-// k_spmm_long on the context's side stream at the same time, one warp per
+// k_spmm_long on the context's side stream at the same time, a pair of warps per
 // (row, C tile column, panel), with the B-row slices themselves copied into
 // shared memory by cp.async two chunks (64 entries) ahead: the loads in
 // flight cost no registers, and a chunk's multiply-adds read shared memory.
 // Rows of 8 times the long-row threshold or more are listed first, so that
 // the longest chains start first.
 
-constexpr int kLongWarps = 4;
+constexpr int kLongPairs = 4;   // pairs of warps per block
 constexpr int kLongBSlots = 3;  // chunks of B slices per warp: applied, in flight, being issued
 constexpr int kLongTSlots = 3;  // chunks of table entries per warp (with the B slices)
 constexpr int kLongASlots = 6;  // chunks of staged A entries per warp
-// A row is long from BCLX_TUNE_SPMM_LONG_ROW entries over all stages (512
-// for FP32, 1024 for BF16 by default).
+// A row is long from BCLX_TUNE_SPMM_LONG_ROW entries over all stages (512 by
+// default).
 constexpr int64_t kSpmmLongMinRows = 65536;  // smaller products do not use the long-row path
 
 struct LongSmem {
@@ -448,7 +426,14 @@ struct LongSmem {
   uint4 tab[kLongTSlots][32];    // [chunk slot][entry]: B-row address, A value
   uint2 a[kLongASlots][32];      // [chunk slot][entry]: staged A (column, value)
   uint8_t src[kLongASlots][32];  // the entry's stage lane
+  unsigned long long next;       // the pair's next item
 };
+
+// The two warps of a pair (a producer and a consumer) meet.
+__device__ __forceinline__ void pair_sync(int pair) {
+  __syncwarp();
+  asm volatile("bar.sync %0, 64;\n" ::"r"(pair + 1) : "memory");
+}
 
 // Thread per A row (ti, r): entries over all stages; rows with at least
 // long_row are flagged and listed: very long rows from list[0] up
@@ -476,31 +461,63 @@ __global__ void k_spmm_find_long(SpGridView A, int long_row, int very_long_row, 
 }
 
 // One long row r of C tile (ti, tj), panel from column c0 (16-byte aligned
-// access: the caller checked).  Pipeline at chunk c (32 entries, one per
-// lane when staged or built):
-//   * A of chunk c + 6 staged (cp.async, 8 bytes per lane);
-//   * chunk c + 2 built: each lane's entry -> table (B-row address, value),
-//     then every lane copies its 16 bytes of each of the chunk's 32 B rows
-//     into the chunk's B slot (cp.async);
-//   * chunk c applied: the multiply-adds in entry order from shared memory.
-// One commit group per chunk step holds A(c+6) and B(c+2); B(c) is in the
-// group two steps back.  The stages are at most 32 (one lane each).
+// access: the caller checked), by a pair of warps.  In step c (a chunk of 32
+// entries, one per lane when staged or built)
+//   * the consumer applies chunk c: the multiply-adds in entry order from
+//     shared memory;
+//   * the producer stages A of chunk c + 6 (cp.async, 8 bytes per lane),
+//     builds chunk c + 2 (each lane's entry -> table: B-row address, value),
+//     copies its B rows into the slot that chunk c - 1 left (cp.async, every
+//     lane 16 bytes of each row) and waits for chunk c + 1's;
+// and the two meet.  One commit group per step holds A(c+6) and B(c+2).  The
+// stages are at most 32 (one lane each).  The row's chain sets the time of
+// these products: one warp doing both parts took some 60 cycles per entry, on
+// an SM to itself as well. 
+// Now a pair takes the SM's share of L2 traffic: R-MAT of 1,000,000 rows x 256
+// BF16 1.56 -> 1.13 ms, of 300,000 x 128 FP32 551 -> 388 us, of 100,000 x 128 274 ->
+// 188, s21 x 256 BF16 2.19 -> 1.91 ms.
 template <typename ST, bool SUB>
-__device__ __forceinline__ void spmm_long_row(LongSmem& S, const SpGridView& A, const DGridView& B,
-                                              const DGridView& C, int64_t ti, int64_t tj, int64_t r, int c0, int W) {
+__device__ __forceinline__ void spmm_long_row(LongSmem& S, int pair, bool producer, const SpGridView& A,
+                                              const DGridView& B, const DGridView& C, int64_t ti, int64_t tj, int64_t r,
+                                              int c0, int W) {
   using V = Vec<ST>;
   constexpr int VN = V::N;
   const int lane = lane_id();
   ST* __restrict__ crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld;
   const int col = c0 + lane * VN;
   const bool own = col < W;
-  float acc[VN];
-  if (own) V::load_c(crow + col, acc);
   const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, lane, true);
   const int32_t aincl = warp_inclusive_scan(sl.alen);
   const int32_t atot = __shfl_sync(kFull, aincl, 31);
   const int32_t aexcl = aincl - sl.alen;
   const int32_t nch = (atot + 31) >> 5;
+  if (!producer) {
+    float acc[VN];
+    if (own) V::load_c(crow + col, acc);
+    pair_sync(pair);  // chunk 0 is there
+    for (int32_t c = 0; c < nch; c++) {
+      const int ne = min(32, atot - c * 32);
+      const int bslot = c % kLongBSlots, tslot = c % kLongTSlots;
+      auto apply = [&](int u) {
+        float b[VN];
+        V::unpack_raw(S.b[bslot][u][lane], b);
+        const float vs = __uint_as_float(S.tab[tslot][u].z);
+#pragma unroll
+        for (int x = 0; x < VN; x++) acc[x] = __fmaf_rn(vs, b[x], acc[x]);
+      };
+      if (own) {
+        if (ne == 32) {
+#pragma unroll 16
+          for (int u = 0; u < 32; u++) apply(u);
+        } else {
+          for (int u = 0; u < ne; u++) apply(u);
+        }
+      }
+      pair_sync(pair);
+    }
+    if (own) V::store(crow + col, acc);
+    return;
+  }
   auto issue_a = [&](int32_t x) {
     if (x >= nch) return;
     const int32_t e = x * 32 + lane;
@@ -573,53 +590,33 @@ __device__ __forceinline__ void spmm_long_row(LongSmem& S, const SpGridView& A, 
   issue_b(1);
   issue_a(5);
   cp_async_commit();
-  cp_async_wait_group<2>();
+  cp_async_wait_group<1>();  // B(0) and A(4) have landed
+  pair_sync(pair);
   for (int32_t c = 0; c < nch; c++) {
     issue_a(c + 6);
     build(c + 2);
     __syncwarp();
     issue_b(c + 2);
     cp_async_commit();
-    cp_async_wait_group<2>();  // B(c) and A(c + 4) have landed
-    const int ne = min(32, atot - c * 32);
-    const int bslot = c % kLongBSlots, tslot = c % kLongTSlots;
-    if (own) {
-      if (ne == 32) {
-#pragma unroll 8
-        for (int u = 0; u < 32; u++) {
-          float b[VN];
-          V::unpack_raw(S.b[bslot][u][lane], b);
-          const float vs = __uint_as_float(S.tab[tslot][u].z);
-#pragma unroll
-          for (int x = 0; x < VN; x++) acc[x] = __fmaf_rn(vs, b[x], acc[x]);
-        }
-      } else {
-        for (int u = 0; u < ne; u++) {
-          float b[VN];
-          V::unpack_raw(S.b[bslot][u][lane], b);
-          const float vs = __uint_as_float(S.tab[tslot][u].z);
-#pragma unroll
-          for (int x = 0; x < VN; x++) acc[x] = __fmaf_rn(vs, b[x], acc[x]);
-        }
-      }
-    }
-    __syncwarp();
+    cp_async_wait_group<1>();  // B(c + 1) and A(c + 5) have landed
+    pair_sync(pair);
   }
   cp_async_wait_all();
-  if (own) V::store(crow + col, acc);
 }
 
 // Items (listed row, C tile column, panel), a row's items consecutive, taken
 // from a device counter in list order.  Every block, once placed, lets a
 // programmatic dependent (k_spmm under the dependent-launch schedule) launch.
 template <typename ST, bool SUB>
-__global__ void __launch_bounds__(kLongWarps * 32)
+__global__ void __launch_bounds__(kLongPairs * 64)
     k_spmm_long(SpGridView A, DGridView B, DGridView C, int tjn, const int64_t* __restrict__ list,
                 const int32_t* __restrict__ count, int npanels, int row_align_ok,
                 unsigned long long* __restrict__ next_item) {
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   extern __shared__ __align__(16) unsigned char long_smem[];
-  LongSmem& S = reinterpret_cast<LongSmem*>(long_smem)[threadIdx.x >> 5];
+  const int pair = threadIdx.x >> 6;
+  const bool producer = (threadIdx.x >> 5) & 1;
+  LongSmem& S = reinterpret_cast<LongSmem*>(long_smem)[pair];
   constexpr int PW = 32 * Vec<ST>::N;
   const int lane = lane_id();
   const int64_t rows = A.gm * A.tm;
@@ -627,12 +624,13 @@ __global__ void __launch_bounds__(kLongWarps * 32)
   const int64_t nl = nv + count[1];
   const int64_t per_row = (int64_t)tjn * npanels;
   const unsigned long long n = (unsigned long long)(nl * per_row);
-  unsigned long long it = 0;
-  if (lane == 0) it = atomicAdd(next_item, 1ULL);
-  it = __shfl_sync(kFull, it, 0);
+  // the first items, dealt to the blocks in turn: neighbouring rows, which the
+  // longest are, go to different SMs
+  unsigned long long it = (unsigned long long)pair * gridDim.x + blockIdx.x;
+  const unsigned long long dealt = (unsigned long long)gridDim.x * kLongPairs;
   while (it < n) {
     unsigned long long nx = 0;
-    if (lane == 0) nx = atomicAdd(next_item, 1ULL);
+    if (producer && lane == 0) nx = dealt + atomicAdd(next_item, 1ULL);
     const int64_t li = (int64_t)it / per_row;
     const int64_t pt = (int64_t)it - li * per_row;
     const int panel = (int)(pt % npanels);
@@ -642,9 +640,13 @@ __global__ void __launch_bounds__(kLongWarps * 32)
     const int W = (int)C.cols_of(tj);
     if (panel * PW < W) {
       const bool vec = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
-      if (vec) spmm_long_row<ST, SUB>(S, A, B, C, ti, tj, r, panel * PW, W);  // otherwise k_spmm did it element-wise
+      // (otherwise k_spmm does it element-wise)
+      if (vec) spmm_long_row<ST, SUB>(S, pair, producer, A, B, C, ti, tj, r, panel * PW, W);
     }
-    it = __shfl_sync(kFull, nx, 0);
+    if (producer && lane == 0) S.next = nx;
+    pair_sync(pair);
+    it = *reinterpret_cast<volatile unsigned long long*>(&S.next);
+    pair_sync(pair);
   }
 }
 
@@ -1173,13 +1175,14 @@ __global__ void k_spmm_launch_delay(unsigned ns) {
 }
 
 // Blocks of k_spmm_long (one per SM: its shared memory fills the SM); the
-// other SMs run k_spmm.  By default a quarter of the SMs per column panel of
-// a long row, at most half (R-MAT s21 x 256: FP32, two panels, 74 blocks;
-// BF16, one panel, 37 blocks, measured 2.39 against 2.75 ms with 74);
-// BCLX_TUNE_SPMM_LONG_BLOCKS sets the count.
-static int spmm_long_blocks(const Context* ctx, int npanels) {
+// other SMs run k_spmm.  By default five twelfths of the SMs (61): with 49, 62
+// and 74, R-MAT s21 x 256 FP32 3.84, 3.52 and 3.69 ms, BF16 2.02, 1.91 and 1.93;
+// R-MAT of 1,000,000 rows x 256 FP32 2.03, 1.67 and 1.64, BF16 1.17, 1.13 and
+// 1.16; of 300,000 x 128 FP32 401, 388 and 386 us.  BCLX_TUNE_SPMM_LONG_BLOCKS
+// sets the count.
+static int spmm_long_blocks(const Context* ctx) {
   int b = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_BLOCKS);
-  if (b <= 0) b = std::min(ctx->num_sms / 2, ctx->num_sms / 4 * npanels);
+  if (b <= 0) b = ctx->num_sms * 5 / 12;
   return std::max(1, std::min(b, ctx->num_sms));
 }
 
@@ -1208,8 +1211,9 @@ static int spmm_rows_per_item(const Context* ctx, const DGridView& C, int64_t tj
 //  1: one stream; k_spmm launched as k_spmm_long's programmatic dependent
 //    (it launches once every long-row block has started, and finishes only
 //    after k_spmm_long).
-// Measured on R-MAT s21 x 256 (one B200): schedule 0 4.14 ms FP32 / 2.45 ms
-// BF16, schedule 1 4.63 / 3.45 ms.  Also measured, and slower: one-warp
+// Measured on R-MAT s21 x 256 (one B200): schedule 0 3.46 ms FP32 / 1.89 ms
+// BF16, schedule 1 3.63 / 1.90 ms.  Also measured, with one warp for both parts
+// of a long row (4.14 and 2.45 ms), and slower: one-warp
 // long-row blocks small enough to share every SM with four k_spmm blocks
 // (k_spmm capped at 56 registers, both kernels at the largest shared-memory
 // carveout): 5.08 / 3.91 ms, k_spmm alone losing 15 % to the smaller L1;
@@ -1229,10 +1233,10 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
   const int64_t arows = A.gm * A.tm;
   const bool long_path = align_ok && A.gn <= 32 && arows >= spmm_long_min_rows();
   // rows of at least long_row entries go to the long-row kernel: by default
-  // 512 for FP32 and 1024 for BF16 (R-MAT s21 x 256: FP32 4.00 against
-  // 4.21 ms with 1024; BF16 2.42 against 3.11 ms with 512)
+  // 512 (R-MAT s21 x 256: FP32 3.52 against 3.81 ms with 1024, BF16 1.91 against
+  // 2.05; of 300,000 rows x 256 BF16 425 against 528 us)
   int long_row = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_ROW);
-  if (long_row <= 0) long_row = sizeof(ST) == 4 ? 512 : 1024;
+  if (long_row <= 0) long_row = 512;
   const bool dependent = tuning(ctx, BCLX_TUNE_SPMM_SCHEDULE) == 1;
   // counters: [0] k_spmm items, [1] k_spmm_long items, [2] listed very long / other long rows (2 x int32)
   unsigned long long* ctr = nullptr;
@@ -1256,9 +1260,9 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
     note_launch();
     BCLX_CK_LAUNCH();
     if (!dependent) BCLX_CK(cudaEventRecord(ctx->fork2_ev, ctx->side));
-    const size_t lsmem = sizeof(LongSmem) * kLongWarps;
+    const size_t lsmem = sizeof(LongSmem) * kLongPairs;
     BCLX_CK(cudaFuncSetAttribute(k_spmm_long<ST, SUB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lsmem));
-    k_spmm_long<ST, SUB><<<(unsigned)spmm_long_blocks(ctx, npanels), kLongWarps * 32, lsmem, ls>>>(A, B, C, tjn, list, cnt, npanels,
+    k_spmm_long<ST, SUB><<<(unsigned)spmm_long_blocks(ctx), kLongPairs * 64, lsmem, ls>>>(A, B, C, tjn, list, cnt, npanels,
                                                                                     align_ok, ctr + 1);
     note_launch();
     BCLX_CK_LAUNCH();
