@@ -323,7 +323,7 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
 #pragma unroll
             for (int u = 0; u < UNROLL; u++)
               if (u0 + u < ne) {
-                if (GROUP && ((heads >> (u0 + u)) & 1u)) enter((int)ent[u].w);
+                if (GROUP && ((heads >> (u0 + u)) & 1u)) enter((int)t[u0 + u].w);
                 apply(u);
               }
           }
@@ -387,12 +387,13 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
       if (t != at) {
-        aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+        aligned = row_align_ok > 0 && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
         at = t;
       }
       const bool vec = aligned;
-      // rows flagged long are k_spmm_long's (it takes the aligned ones)
-      spmm_rows<ST, GROUP, SUB>(A, B, C, ti, tj, r0, R, c0, W, vec, vec ? long_flag : nullptr);
+      // rows flagged long are k_spmm_long's (it takes the aligned ones), or
+      // k_spmm_chain's (row_align_ok < 0: all of them)
+      spmm_rows<ST, GROUP, SUB>(A, B, C, ti, tj, r0, R, c0, W, vec, vec || row_align_ok < 0 ? long_flag : nullptr);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -683,6 +684,12 @@ constexpr int kNarrowUnroll = 4;          // entries per lane group whose loads 
 // a warp its longest row (R-MAT 50,000 x 8: 82 us with 16 steps, 83 with 32, 111
 // with 64; R-MAT 300,000 x 32 BF16: 284, 264, 289).
 constexpr int kNarrowLongSteps = 32;
+// In products of few rows (not listed, see launch_narrow_nv), where a warp has
+// an item or two and waits for its longest row, also a row of this many entries and
+// of four times its tile row's mean (rows that are all alike stay with their
+// warps): R-MAT 2,412 x 119 FP32 60 -> 39 us, 4,313 x 72 BF16 82 -> 42, 20,000 x 47
+// FP32 106 -> 80, 40,000 x 90 152 -> 123.
+constexpr int kNarrowFewLong = 128;
 // Widest row of an aligned tile that k_spmm_narrow takes: two 128-byte lines
 // (one warp then walks two rows).  At 256 bytes: R-MAT 300,000 x 64 FP32 0.32
 // ms against 0.51 with k_spmm, uniform 100,000 x 128 BF16 93 us against 108.
@@ -1111,11 +1118,13 @@ __global__ void __launch_bounds__(kChainWarps * 32, 2)
 
 // Short rows of tile columns [tj0, tj0 + tjn).  With `met` the long rows go to
 // that list (met_count their number), otherwise they are left to k_spmm_chain.
+// A row is long from long_most entries, or from long_least and four times the
+// mean of its tile row.
 template <typename ST, int U, int NV, bool SUB>
 __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
     k_spmm_narrow(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int L, int npanels, int64_t n_items,
-                  int64_t ngroups, int long_row, int64_t* __restrict__ met, int32_t* __restrict__ met_count,
-                  unsigned long long* __restrict__ next_item) {
+                  int64_t ngroups, int long_most, int long_least, int64_t* __restrict__ met,
+                  int32_t* __restrict__ met_count, unsigned long long* __restrict__ next_item) {
   constexpr int PW = 32 * NV * Unit<ST, U>::N;  // columns of a panel
   const int lane = lane_id();
   unsigned long long it = 0;
@@ -1123,6 +1132,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
   it = __shfl_sync(kFull, it, 0);
   int64_t at = -1, ti = 0, tj = 0;  // the C tile of the last item
   bool on = false;
+  int long_row = long_most;
   while ((int64_t)it < n_items) {
     unsigned long long nx = 0;
     if (lane == 0) nx = atomicAdd(next_item, 1ULL);
@@ -1135,6 +1145,10 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
       ti = t / tjn;
       tj = tj0 + (t - ti * tjn);
       on = tile_on<ST, U>(B, C, ti, tj, (int)C.cols_of(tj));
+      if (long_least < long_most) {  // (at most 32 tiles along k)
+        const float nnz = warp_sum(lane < A.gn ? (float)A.tile(ti, lane).nnz : 0.f);
+        long_row = min(long_most, max(long_least, (int)min(4.f * nnz / (float)C.rows_of(ti), 1e9f)));
+      }
     }
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
@@ -1348,8 +1362,10 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   const bool chains = A.gn <= 32;  // one lane per stage
   const bool listed = chains && arows >= spmm_long_min_rows();
   int long_row = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_ROW);
-  if (long_row <= 0) long_row = kNarrowLongSteps * L;
+  const bool few = chains && !listed && long_row <= 0;
+  if (long_row <= 0) long_row = std::min(kNarrowLongSteps * L, listed && L == 32 && tj0 == 0 ? 512 : INT_MAX);
   if (!chains) long_row = INT_MAX;
+  const int long_least = few ? std::min(kNarrowFewLong, long_row) : long_row;
   // counters: [0] row groups taken, [1] long rows taken, [2] listed very long / other long rows (2 x int32)
   unsigned long long* ctr = nullptr;
   uint8_t* flag = nullptr;
@@ -1368,7 +1384,25 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   auto narrow = [&]() {
     const int64_t blocks = std::min(ceil_div(n_items, kNarrowWarps), (int64_t)ctx->num_sms * 4);
     return launch_after(ctx, listed, (unsigned)blocks, kNarrowWarps * 32, 0, k_spmm_narrow<ST, U, NV, SUB>, A, B, C,
-                        tj0, tjn, L, npanels, n_items, ngroups, long_row, listed ? nullptr : list, cnt, ctr);
+                        tj0, tjn, L, npanels, n_items, ngroups, long_row, long_least, listed ? nullptr : list, cnt, ctr);
+  };
+  // A lane group of 32 takes one row; k_spmm shares a warp's set-up among up to
+  // four, element by element, and a panel of its lanes is 512 bytes.  So it takes the
+  // short rows where the long ones are listed: uniform 186,581 x 150 FP32, 5
+  // entries a row, 438 -> 270 us; stencil of 262,144 x 185 BF16 1041 -> 799 (R-MAT of 273,612 x
+  // 118 FP32 570 -> 769, of 300,000 x 201 1184 -> 1361, of 1,432,750 x 87 2467 -> 2391,
+  // of 100,000 x 90 BF16 229 -> 217, with rows long from 512 entries).
+  auto wide = [&]() {
+    const int wp = (int)ceil_div(width, 32 * Vec<ST>::N);
+    const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
+    const int64_t groups = ceil_div(C.tm, (int64_t)R), items = C.gm * tjn * groups * wp;
+    const int64_t blocks = std::min(ceil_div(items, kSpmmWarps), (int64_t)ctx->num_sms * 4);
+    const uint8_t* skip = flag;
+    if (R > 1)
+      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, true, SUB>, A, B, C, tjn, items, wp, R,
+                          groups, -1, 0, skip, ctr);
+    return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, false, SUB>, A, B, C, tjn, items, wp, 1,
+                        groups, -1, 0, skip, ctr);
   };
   if (!listed) BCLX_TRY(narrow());
   if (chains) {
@@ -1380,7 +1414,7 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
                           (int)ceil_div(width * (int64_t)sizeof(ST), 4 * kChainPanelWords), stride, each, !listed, list,
                           cnt, ctr + 1));
   }
-  if (listed) BCLX_TRY(narrow());
+  if (listed) BCLX_TRY(L == 32 && tj0 == 0 ? wide() : narrow());
   scratch_free(ctx, flag);
   scratch_free(ctx, list);
   scratch_free(ctx, ctr);

@@ -101,3 +101,21 @@ def test_tile_bases_and_leading_dimensions(matrix, dtype, shift, ld):
         assert np.array_equal(as_u16(got), O.spmm_tiled_bf16(a, as_u16(b), as_u16(c0), *tiles))
     rows(C, a.m)[:, :n] = rows(before, a.m)[:, :n]
     assert torch.equal(C, before)
+
+
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+@pytest.mark.parametrize("n,tiles", [(119, (700, 800, 119)), (13, (2048, 64, 13)), (56, (300, 2048, 56)), (40, (2048, 2048, 16))])
+def test_few_rows(matrix, n, tiles, dtype):
+    """Few rows, the knob left at its default: rows of 128 entries and of four
+    times their tile row's mean go to the chains (and of two and three tile
+    columns, the last one narrower)."""
+    check(matrix, n, tiles, dtype, seed=n)
+
+
+@pytest.mark.parametrize("dtype,n", [("f32", 65), ("f32", 119), ("f32", 150), ("f32", 201), ("bf16", 99), ("bf16", 185), ("bf16", 258), ("bf16", 270)])
+@pytest.mark.parametrize("tiles", [(700, 800), (2048, 64)])
+def test_wide_unaligned_listed(monkeypatch, matrix, dtype, n, tiles):
+    """Rows off 16 bytes of more units than a lane group holds, long rows
+    listed: the others go to the wide kernel, several to a warp and one."""
+    monkeypatch.setenv("BCLX_SPMM_LONG_MIN_ROWS", "0")
+    check(matrix, n, (*tiles, n), dtype, seed=n)
