@@ -19,16 +19,17 @@
 // Numeric, per item (one warp): the item's column bitmap (rebuilt from the
 // products for light rows, loaded for heavy items) is turned into per-word
 // prefix counts, so that column j's output position is
-// rank(j) = prefix[j/32] + popc(lower bits of its word); sorted columns are
-// written directly.  Then the products are walked in the reference's order
+// rank(j) = prefix[j/32] + popc(lower bits of its word); the columns, sorted by
+// their bits, leave through shared memory.  Then the products are walked in the reference's order
 // and values are accumulated in shared memory at rank(j).
 //
 // Order.  The product stream of a row is: stages k = (k_ + i + j) mod G for
 // k_ = 0..G-1; inside a stage the A-row entries in stored order; inside an
 // entry the B-row entries in stored order.  It is walked 32 products at a
-// time, packed across A entries and stages.  Lanes holding the same column
-// are grouped with __match_any_sync and the lowest lane applies the group's
-// updates in lane order; batches are separated by __syncwarp.  Every column
+// time, those of one A entry or packed across A entries and stages
+// (walk_products).  Packed, lanes holding the same column are found with
+// __match_any_sync and take turns in lane order; batches are separated by
+// __syncwarp.  Every column
 // keeps a running stage partial (`part`, started at 0 and advanced with a
 // fused multiply-add per product) and the sum of its finished stage partials
 // (`acc`, started at 0); when a product of a later stage arrives the partial
