@@ -1,4 +1,4 @@
-"""Narrow and unaligned dense tiles (k_spmm_staged): widths around one and two
+"""Narrow and unaligned dense tiles (k_spmm_narrow, k_spmm_chain): widths around one and two
 words per lane and around the bound to the wide kernel, rows on 16, 4 and 2
 bytes, tile bases off 16 bytes, one to 40 tiles along k, long rows listed or
 not, rows without entries.  The order of the multiply-adds is the oracle's, so
