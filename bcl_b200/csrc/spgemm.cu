@@ -43,6 +43,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cstring>
 #include <initializer_list>
 #include <mutex>
@@ -67,6 +68,7 @@ constexpr int64_t kSplitMaxProducts = 40 << 20;  // largest product whose items 
 // and no bound: R-MAT s16 3.20, 2.92, 2.85, 2.88, 2.99 ms; R-MAT s18 34.0, 30.5,
 // 30.3, 30.4, 30.6; graph x sparse features 983, 492, 494, 502, 498 us.
 constexpr int kLongSegDefault = 14;
+constexpr int kOnlyPacked = INT_MAX;      // every chunk, and no two products of a batch known to differ in column
 constexpr int kQueueSlots = 256;          // work-queue heads in a plan: one per stage launch (at most 254), and
 constexpr int kSymbolicSlot = 255;        // the symbolic pass' (used once)
 constexpr int64_t kMidHeavyUb = 8192;    // from here on where such rows are few (see symbolic_impl)
@@ -225,17 +227,19 @@ struct WalkTable {
 // 32 at a time (a chunk), one per lane, each finding its B segment; the
 // non-empty ones go to `tbl`, compacted.  The chunk's products are walked
 // in one of two ways:
-//  * entry by entry, 32 products of one segment at a time: the columns of one
-//    B row are distinct, so the lanes never touch the same column, and each
+//  * entry by entry, 32 products of one segment at a time: where the columns of
+//    one B row are distinct the lanes never touch the same column, and each
 //    calls fd(on, j, a, b, stage) for its own product;
 //  * packed 32 products per batch whatever entries they belong to: every lane
 //    calls f(on, j, a, b, stage, one) once per batch (warp-uniform); `on`
 //    lanes form a prefix of the warp and lane order is product order; `one`:
-//    the batch is 32 products of one entry.
+//    the batch is 32 products of one entry, of distinct columns.
 // Either way a __syncwarp follows and the next loads are issued before f or
 // fd runs.  A batch costs about four steps (finding each product's entry and
 // ordering equal columns: some 170 instructions against 40), so a chunk is
-// packed where its segments average fewer than long_seg products.
+// packed where its segments average fewer than long_seg products.  With
+// kOnlyPacked every chunk is: a B row then may name a column twice
+// (look_for_repeats), and no batch counts as `one`.
 //
 // Packed, the table's addresses are moved back by the entry's first product,
 // so that product q is at seg + q whatever its entry.  Which entry a lane's
@@ -334,6 +338,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
         const int32_t begins = len > 0 ? excl : INT_MAX;  // this entry's first product
         int ahead = -1;                                   // entries begun before the batch, less one
         const uint32_t end = (uint32_t)total - 1u;
+        const int32_t one_end = long_seg != kOnlyPacked ? total : 0;
         unsigned heads;
         auto fetch = [&](int32_t base) {
           heads = __reduce_or_sync(kFull, bit_or_none(begins - base));
@@ -351,7 +356,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
           const int32_t j = nj;
           const VT a = na, b = nb;
           const int st = (int)(nls & 255u);
-          const bool one = (heads & ~1u) == 0u && base + 32 <= total;  // no entry begins after the first product
+          const bool one = (heads & ~1u) == 0u && base + 32 <= one_end;  // no entry begins after the first product
           if (base + 32 < total) fetch(base + 32);
           f(base + lane < total, j, a, b, st, one);
         }
@@ -572,6 +577,49 @@ static int read_back(Context* ctx, std::initializer_list<std::tuple<const void*,
 
 // ---- planning --------------------------------------------------------------------
 
+// Does a row of a B tile name a column twice (or descend)?  Then *repeats is
+// set, and the numeric pass does not take a row's products for products of
+// distinct columns.  A part of the classification kernels, by blocks of 256: of
+// kRepeatRows rows the block counts the entries whose column is not above the
+// one before, and takes away the rows that begin with such an entry; what is
+// left are repeats.  (By the rows' ends alone, so that a hub row is no
+// thread's own walk.  After the classification: before it, blocks with more to
+// look through appended their rows later, and the lists' order, which the numeric
+// pass re-reads B in, cost the 27-point stencil on 128^3 22.1 -> 22.4 ms.)
+constexpr int kRepeatRows = 2048;
+__device__ __forceinline__ void look_for_repeats(const SpGridView& B, const Geom& g, int32_t* __restrict__ repeats) {
+  __shared__ int found;
+  const int64_t nt = g.gk * g.gn;
+  int64_t t = blockIdx.x;
+  for (int64_t r0 = 0; r0 < g.tk; r0 += kRepeatRows) {  // (these rows of every tile, then the next)
+    for (; t < nt; t += gridDim.x) {
+      const bclx_csr_t Bt = B.tile(0, t);
+      const int64_t r1 = min(r0 + kRepeatRows, Bt.m);  // (the tile's own row count)
+      if (r0 >= r1 || (g.scount && Bt.nnz <= 0)) continue;  // (the stage map leaves such tiles out as well)
+      if (threadIdx.x == 0) found = 0;
+      __syncthreads();
+      const int32_t first = __ldg(Bt.row_ptr + r0), end = __ldg(Bt.row_ptr + r1);
+      int mine = 0;
+      const int n = end - first;
+#pragma unroll 8
+      for (int p = 1 + threadIdx.x; p < n; p += 256)
+        mine += __ldg(Bt.col_ind + first + p) <= __ldg(Bt.col_ind + first + p - 1);
+#pragma unroll 4
+      for (int64_t r = r0 + 1 + threadIdx.x; r < r1; r += 256) {
+        const int32_t s = __ldg(Bt.row_ptr + r);
+        if (s < __ldg(Bt.row_ptr + r + 1) && s > first && s < end)
+          mine -= __ldg(Bt.col_ind + s) <= __ldg(Bt.col_ind + s - 1);
+      }
+      mine = __reduce_add_sync(kFull, mine);
+      if (lane_id() == 0 && mine != 0) atomicAdd(&found, mine);
+      __syncthreads();
+      if (threadIdx.x == 0 && found != 0) *repeats = 1;
+      __syncthreads();
+    }
+    t -= nt;
+  }
+}
+
 // Per row: intermediate products; light/heavy classification into two lists.
 // One warp per row: one lane per stage reads the A-row segment, then the
 // flattened entries are read 32 at a time.
@@ -581,6 +629,7 @@ static int read_back(Context* ctx, std::initializer_list<std::tuple<const void*,
 // and the row's product count (capped at 2^31-1) to ub_out[ri].
 // `live` (or null: every C tile): the n_live[0] C tiles with at least one
 // stage; only their rows are walked (the others have no products).
+// counters [5]: look_for_repeats.
 template <bool FEATURES>
 __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list,
                            int32_t* __restrict__ heavy_list, int32_t* __restrict__ vheavy_list,
@@ -684,6 +733,7 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
     base = __shfl_sync(kFull, nx, 0);
   }
   if (lane == 0 && mine) atomicAdd(products, mine);
+  look_for_repeats(B, g, counters + 5);
 }
 
 // Products of every row for all of its C tiles at once: a warp takes a row of A's tile row ti, reads its
@@ -713,7 +763,8 @@ constexpr int kClassifyDefer = 64;  // long rows a block can put off
 __global__ void __launch_bounds__(256) k_classify_rows(
     SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
     int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
-    int heavy_min_cols, int light_ub, const unsigned long long* __restrict__ n_stages) {  // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list
+    int heavy_min_cols, int light_ub, const unsigned long long* __restrict__ n_stages) {
+  // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list; [5]: look_for_repeats
   __shared__ int32_t kept_all[8][4][kClassifyKeep * 32];
   __shared__ unsigned long long sums[32];
   __shared__ uint32_t deferred[kClassifyDefer];
@@ -844,6 +895,7 @@ __global__ void __launch_bounds__(256) k_classify_rows(
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mine += __shfl_xor_sync(kFull, mine, d);
   if (lane == 0 && mine) atomicAdd(products, mine);
+  look_for_repeats(B, g, counters + 5);
 }
 
 // B-row table: for every row of every B tile (k, j), the position of the
@@ -994,6 +1046,7 @@ __global__ void __launch_bounds__(256) k_classify_tiles(
     for (int q = 0; q < 8; q++) all += sums[q];
     if (all) atomicAdd(products, all);
   }
+  look_for_repeats(B, g, counters + 5);
 }
 
 // ---- symbolic ----------------------------------------------------------------------
@@ -1906,7 +1959,9 @@ struct bclx_spgemm_plan_s {
   int32_t* heavy_list = nullptr;   // very heavy rows first, then the other heavy rows
   int32_t* vheavy_list = nullptr;
   int32_t* heavy_tmp = nullptr;
-  int32_t* counters = nullptr;  // [0] light rows, [1] heavy rows (total after planning), [2] overflow, [3] very heavy
+  // [0] light rows, [1] heavy rows, [2] overflow, [3] very heavy, [4] above kMidHeavyUb, [5] look_for_repeats
+  int32_t* counters = nullptr;
+  bool repeats = false;  // a B row names a column twice (walk_products)
   unsigned long long* products_dev = nullptr;
   int32_t* row_count = nullptr;
   int64_t* row_offset = nullptr;
@@ -2133,7 +2188,8 @@ static int launch_numeric_w(Context* ctx, const SpGridView& A, const SpGridView&
   kern<<<grid_for(ctx, n_total, kWarpsNum, bps), kWarpsNum * 32, smem, ctx->stream>>>(
       A, B, P->g, P->light_list, P->heavy_list, (int)P->n_light, P->n_heavy_items, P->heavy_items, P->heavy_bitmaps,
       P->hbm_words, P->tab, P->row_count, P->row_offset, out_col, reinterpret_cast<VT*>(out_val), s0, s1, q,
-      P->grab > 0 ? P->grab : numeric_grab(ctx, P, n_total), P->long_seg < 1 ? 1 : P->long_seg, LEARNED ? P->light_slot : nullptr,
+      P->grab > 0 ? P->grab : numeric_grab(ctx, P, n_total),
+      P->repeats ? kOnlyPacked : std::max(1, std::min(P->long_seg, kOnlyPacked - 1)), LEARNED ? P->light_slot : nullptr,
       LEARNED ? P->item_count : nullptr, LEARNED ? P->row_count : nullptr, LEARNED ? P->row_failed : nullptr,
       P->heavy_slot_base, LEARNED ? P->item_off : nullptr, split);
   note_launch();
@@ -2340,12 +2396,14 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     note_launch((rows ? 1 : 0) + (live ? 1 : 0));
     BCLX_CK_LAUNCH();
   }
-  BCLX_TRY(read_back(ctx, {{P->counters, 8, 0}, {P->counters + 2, 8, 1}, {P->products_dev, 8, 2}, {P->counters + 4, 4, 3}}));
+  BCLX_TRY(read_back(ctx, {{P->counters, 8, 0}, {P->counters + 2, 8, 1}, {P->products_dev, 8, 2}, {P->counters + 4, 8, 3}}));
   if (live) scratch_free(ctx, live);
   BCLX_CK(cudaStreamSynchronize(ctx->stream));
-  int32_t cnts[4], n_mid;
+  int32_t cnts[4], more[2];
   std::memcpy(cnts, ctx->pinned, sizeof(cnts));
-  std::memcpy(&n_mid, ctx->pinned + 3, sizeof(n_mid));
+  std::memcpy(more, ctx->pinned + 3, sizeof(more));
+  const int32_t n_mid = more[0];
+  P->repeats = more[1] != 0;
   P->n_light = cnts[0];
   // the rows between kMidHeavyUb and kVeryHeavyUb products count as very heavy
   // where all of these are no more than SMs: then they are what a small
@@ -2821,7 +2879,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
   P.heavy_list = ar.take<int32_t>(nri);
   P.vheavy_list = ar.take<int32_t>(nri);
   P.heavy_tmp = ar.take<int32_t>(nri);
-  P.counters = ar.take<int32_t>(4);
+  P.counters = ar.take<int32_t>(6);
   P.products_dev = ar.take<unsigned long long>(1);
   P.row_count = ar.take<int32_t>(nri);
   P.row_offset = ar.take<int64_t>(nri + 1);
@@ -2829,7 +2887,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
   int64_t* sums = ar.take<int64_t>(exclusive_scan_sums_len(nri));
   P.queue = ar.take<unsigned long long>(kQueueSlots);
   if (!ar.ok) return noalloc_exhausted();
-  BCLX_CK(cudaMemsetAsync(P.counters, 0, 4 * sizeof(int32_t), ctx->stream));
+  BCLX_CK(cudaMemsetAsync(P.counters, 0, 6 * sizeof(int32_t), ctx->stream));
   BCLX_CK(cudaMemsetAsync(P.products_dev, 0, sizeof(unsigned long long), ctx->stream));
   BCLX_CK(cudaMemsetAsync(P.row_count, 0, sizeof(int32_t) * nri, ctx->stream));
   BCLX_CK(cudaMemsetAsync(P.queue + 1, 0, sizeof(unsigned long long), ctx->stream));
@@ -2838,9 +2896,10 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
       P.queue + 1, queue_grab(ctx, nri, 8, 16, 32, 8));
   note_launch();
   BCLX_CK_LAUNCH();
-  int32_t cnts[4];
+  int32_t cnts[6];
   BCLX_CK(cudaMemcpyAsync(cnts, P.counters, sizeof(cnts), cudaMemcpyDeviceToHost, ctx->stream));
   BCLX_CK(cudaStreamSynchronize(ctx->stream));
+  P.repeats = cnts[5] != 0;
   P.n_light = cnts[0];
   P.n_vheavy = cnts[3];
   P.n_heavy = cnts[1] + cnts[3];
@@ -2986,7 +3045,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
   BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_list, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->vheavy_list, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->heavy_tmp, nri));
-  BCLX_TRY(scratch_alloc_n(ctx, &P->counters, 4));
+  BCLX_TRY(scratch_alloc_n(ctx, &P->counters, 6));
   BCLX_TRY(scratch_alloc_n(ctx, &P->products_dev, 1));
   BCLX_TRY(scratch_alloc_n(ctx, &P->row_count, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->row_offset, nri + 1));
@@ -2994,7 +3053,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
   BCLX_TRY(scratch_alloc_n(ctx, &P->feat, (size_t)nri * 5));
   BCLX_TRY(scratch_alloc_n(ctx, &P->ub, nri));
   BCLX_TRY(scratch_alloc_n(ctx, &P->pred, nri));
-  BCLX_CK(cudaMemsetAsync(P->counters, 0, 4 * sizeof(int32_t), ctx->stream));
+  BCLX_CK(cudaMemsetAsync(P->counters, 0, 6 * sizeof(int32_t), ctx->stream));
   BCLX_CK(cudaMemsetAsync(P->products_dev, 0, sizeof(unsigned long long), ctx->stream));
   BCLX_CK(cudaMemsetAsync(P->row_count, 0, sizeof(int32_t) * (nri > 0 ? nri : 1), ctx->stream));
   int32_t* live = nullptr;  // C tiles with stages (rows of the others have no products)
@@ -3010,7 +3069,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     BCLX_CK_LAUNCH();
     if (live) scratch_free(ctx, live);
   }
-  int32_t cnts[4];
+  int32_t cnts[6];
   int64_t prod = 0;
   BCLX_CK(cudaMemcpyAsync(cnts, P->counters, sizeof(cnts), cudaMemcpyDeviceToHost, ctx->stream));
   BCLX_CK(cudaMemcpyAsync(&prod, P->products_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
@@ -3019,6 +3078,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
   P->n_vheavy = 0;  // the learned cut treats every heavy row alike
   P->n_heavy = cnts[1] + cnts[3];
   P->products = prod;
+  P->repeats = cnts[5] != 0;
   if (cnts[3] > 0)
     BCLX_CK(cudaMemcpyAsync(P->heavy_list, P->vheavy_list, sizeof(int32_t) * cnts[3], cudaMemcpyDeviceToDevice,
                             ctx->stream));
@@ -3135,6 +3195,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->grab = P->grab;
     R->blocks_per_sm = P->blocks_per_sm;
     R->long_seg = P->long_seg;
+    R->repeats = P->repeats;
     R->heavy_list = P->failed_list;  // borrowed
     R->light_list = P->light_list;   // borrowed (unused: no light rows)
     R->n_light = 0;
@@ -3292,10 +3353,10 @@ int bclx_spgemm_row_features(bclx_context_t c, const bclx_spgrid_t* a, const bcl
   int32_t* cnt = nullptr;
   unsigned long long* prod = nullptr;
   BCLX_TRY(scratch_alloc_n(ctx, &lists, 3 * (size_t)nri));
-  int rc = scratch_alloc_n(ctx, &cnt, 4);
+  int rc = scratch_alloc_n(ctx, &cnt, 6);
   if (rc == BCLX_OK) rc = scratch_alloc_n(ctx, &prod, 2);  // products, row counter
   if (rc == BCLX_OK) {
-    cudaMemsetAsync(cnt, 0, 4 * sizeof(int32_t), ctx->stream);
+    cudaMemsetAsync(cnt, 0, 6 * sizeof(int32_t), ctx->stream);
     cudaMemsetAsync(prod, 0, 2 * sizeof(unsigned long long), ctx->stream);
     k_classify<true><<<grid_for(ctx, nri, 8, 16), 256, 0, ctx->stream>>>(
         make_view(*a), make_view(*b), g, lists, lists + nri, lists + 2 * nri, cnt, prod, 8192 + 1, kLightUb, X, ub, prod + 1,

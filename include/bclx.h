@@ -81,7 +81,8 @@ typedef enum {
 typedef struct {
   int64_t m, n, nnz;
   int32_t* row_ptr; /* [m+1] */
-  int32_t* col_ind; /* [nnz], tile-local columns, sorted per row */
+  int32_t* col_ind; /* [nnz], tile-local columns, sorted per row (a row of a sparse product's B, or of a
+                       part to accumulate, may repeat a column: its values count one after another) */
   void* vals;       /* [nnz] of dtype */
   int32_t dtype;
   int32_t pad_;
