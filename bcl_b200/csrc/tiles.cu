@@ -404,13 +404,13 @@ int bclx_csr_to_tiles(bclx_context_t c, const bclx_csr_t* a, bclx_spgrid_out_t* 
 
 int bclx_spgrid_describe(bclx_context_t c, const bclx_spgrid_out_t* g, bclx_csr_t* desc) {
   Context* ctx = reinterpret_cast<Context*>(c);
-  if (!ctx || !g || !g->tile_row_ptr || !g->tile_offset || g->tile_m <= 0 || g->tile_n <= 0 ||
-      g->grid_m != ceil_div(g->m, g->tile_m) || g->grid_n != ceil_div(g->n, g->tile_n))
+  if (!ctx || !g || g->tile_m <= 0 || g->tile_n <= 0 || g->grid_m != ceil_div(g->m, g->tile_m) ||
+      g->grid_n != ceil_div(g->n, g->tile_n))
     return BCLX_ERR_INVALID;
   if (g->dtype != BCLX_F32 && g->dtype != BCLX_I32) return BCLX_ERR_DTYPE;
   const int64_t nt = g->grid_m * g->grid_n;
-  if (nt <= 0) return BCLX_OK;
-  if (!desc) return BCLX_ERR_INVALID;
+  if (nt <= 0) return BCLX_OK;  // (no rows or no columns: arrays of no tiles, which may be null)
+  if (!g->tile_row_ptr || !g->tile_offset || !desc) return BCLX_ERR_INVALID;
   BCLX_CK(cudaSetDevice(ctx->device));
   k_describe<<<blocks_for(ctx, nt, 256), 256, 0, ctx->stream>>>(*g, desc);
   note_launch();

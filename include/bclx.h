@@ -329,9 +329,11 @@ BCLX_API int bclx_spgemm_tile_noalloc(const bclx_csr_t* a, const bclx_csr_t* b, 
  * Rows whose columns are not ascending or out of range: BCLX_ERR_INVALID,
  * nothing written to col_ind/vals.  Synchronizes the context's stream. */
 BCLX_API int bclx_csr_to_tiles(bclx_context_t ctx, const bclx_csr_t* a, bclx_spgrid_out_t* out);
-/* The descriptor array of a packed grid: desc[t] = tile t of `g` (all four
- * arrays set), for a bclx_spgrid_t over it.  `desc`: device array of
- * grid_m*grid_n.  No counterpart in the reference (its tiles are objects). */
+/* The descriptor array of a packed grid: desc[t] = tile t of `g`, for a
+ * bclx_spgrid_t over it.  tile_row_ptr, tile_offset (device arrays) and `desc`
+ * (device array of grid_m*grid_n) must be set unless the grid has no tiles;
+ * col_ind and vals are only pointed at.  No counterpart in the reference (its
+ * tiles are objects). */
 BCLX_API int bclx_spgrid_describe(bclx_context_t ctx, const bclx_spgrid_out_t* g, bclx_csr_t* desc);
 /* Gather every tile of `g` into one CSR matrix: row_ptr [m+1], col_ind and
  * vals [nnz] (nnz = sum of tile nnz), global columns, each row's tiles in
