@@ -293,10 +293,11 @@ class SPMatrix:
         td = self.tile_row_ptr.device
         if td.type == "cuda":
             self.desc = torch.empty((ntiles, 7), dtype=torch.int64, device=td)
+            # the kernel reads int64 offsets on the tiles' device, one after another
+            toff = self.tile_offset.to(device=td, dtype=torch.int64).contiguous()
             g = SpGridOut(self.m, self.n, self.tm, self.tn, self.gm, self.gn, self.tile_row_ptr.data_ptr(),
-                          self.tile_offset.data_ptr(), self.col_ind.data_ptr(), self.vals.data_ptr(),
-                          _NP_TO_DT[self.dtype], 0)
-            call("bclx_spgrid_describe", context(self.device).use_current_stream(), ctypes.byref(g),
+                          toff.data_ptr(), self.col_ind.data_ptr(), self.vals.data_ptr(), _NP_TO_DT[self.dtype], 0)
+            call("bclx_spgrid_describe", context(td.index).use_current_stream(), ctypes.byref(g),
                  ctypes.c_void_p(self.desc.data_ptr()))
             self._offsets_host = None
             return
