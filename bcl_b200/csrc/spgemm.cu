@@ -821,9 +821,11 @@ __global__ void __launch_bounds__(256) k_classify_rows(
       const int32_t* acol = nullptr;
       if (g0 + lane < gk) {
         const bclx_csr_t At = A.tile(ti, g0 + lane);
-        const int32_t as = __ldg(At.row_ptr + r);
-        alen = __ldg(At.row_ptr + r + 1) - as;
-        acol = At.col_ind + as;
+        if (!n_stages || At.nnz > 0) {  // (with a stage map, tiles without entries may have no arrays)
+          const int32_t as = __ldg(At.row_ptr + r);
+          alen = __ldg(At.row_ptr + r + 1) - as;
+          acol = At.col_ind + as;
+        }
       }
       const int32_t atot = __reduce_add_sync(kFull, alen);
       if (put_off && g0 == 0 && atot > kClassifyLong) return -1;
@@ -843,7 +845,7 @@ __global__ void __launch_bounds__(256) k_classify_rows(
             len[q] = 0;
             if (kc >= 0 && j + q < j1) {
               const int32_t* brp = B.tile(g0 + sl, j + q).row_ptr;
-              len[q] = (uint32_t)(__ldg(brp + kc + 1) - __ldg(brp + kc));
+              if (brp) len[q] = (uint32_t)(__ldg(brp + kc + 1) - __ldg(brp + kc));
             }
           }
 #pragma unroll

@@ -105,3 +105,25 @@ def test_fine_grids(name, value_type):
     assert st["products"] == gen.intermediate_products(a, b)
     rp, ci, cv = O.gemm_tiled(a, b, *tiles, mode=value_type)
     assert_csr_identical(C.get(), rp, ci, cv)
+
+
+@pytest.mark.parametrize("n,grid", [(40003, 17), (3000, 20)])
+def test_empty_tiles_of_a_without_arrays(n, grid):
+    """Grids with a stage map do not read A's tiles that have no entries: their
+    descriptors may hold no arrays (rows classified at once, and by tiles)."""
+    import torch
+    from bcl_b200.containers import BlockCustom, SPMatrix, spgemm
+    t = -(-n // grid)
+    a = gen.erdos_renyi(n, 12, seed=5)
+    rows = np.repeat(np.arange(n), np.diff(a.row_ptr))
+    keep = (rows // t * 3 + a.col_ind // t) % 4 != 0  # every fourth tile empty
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows[keep], minlength=n))]).astype(np.int32)
+    a = gen.CSR(n, n, rp, a.col_ind[keep], a.vals[keep])
+    A, B = SPMatrix.from_csr(a, BlockCustom((t, t))), SPMatrix.from_csr(gen.erdos_renyi(n, 9, seed=6), BlockCustom((t, t)))
+    want = spgemm(A, B)
+    empty = A.desc[:, 2] == 0
+    assert int(empty.sum()) > grid
+    A.desc[empty, 3:6] = 0
+    got = spgemm(A, B)
+    for f in ("tile_row_ptr", "tile_offset", "col_ind", "vals"):
+        assert torch.equal(getattr(got, f), getattr(want, f)), f
