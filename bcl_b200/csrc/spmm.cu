@@ -185,7 +185,13 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 // test for inside the unrolled loop).  `skip` (or null): rows flagged there
 // are left to another kernel.  `vec`: every B and C row slice of this tile
 // pair is 16-byte aligned; otherwise element-wise access.
-template <typename ST, bool GROUP, bool SUB, int UNROLL = kSpmmUnroll>
+// There a lane's columns are every 32nd, so that the warp's loads of an entry are
+// of neighbouring words, and EU entries' loads are in flight: with a lane's
+// columns side by side and each entry's loads waited for (EU = 0), uniform
+// 186,581 x 150 FP32 270 us, now 201, stencil of 262,144 x 185 BF16 799, now 587,
+// R-MAT of 273,612 x 118 FP32 765, now 524; tiles whose bases lie off 16 bytes,
+// uniform 300,000 x 256 FP32 1834, now 927.
+template <typename ST, bool GROUP, bool SUB, int EU, int UNROLL = kSpmmUnroll>
 __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
                                           int64_t tj, int64_t r0, int R, int c0, int W, bool vec,
                                           const uint8_t* __restrict__ skip) {
@@ -195,7 +201,8 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
   const int lane = lane_id();
   const int64_t nrows = min((int64_t)R, C.rows_of(ti) - r0);
   ST* __restrict__ crow0 = reinterpret_cast<ST*>(C.tile(ti, tj)) + r0 * C.ld;
-  const int col = c0 + lane * VN;
+  constexpr int S = EU > 0 ? 32 : 1;  // distance of an element-wise lane's columns
+  const int col = c0 + (vec || EU == 0 ? lane * VN : lane);
   const bool own = col < W;
   const int bcol = own ? col : 0;  // lanes past the tile edge load column 0 (in bounds) and store nothing
   const int wib = threadIdx.x >> 5;
@@ -213,7 +220,7 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
     } else {
 #pragma unroll
       for (int x = 0; x < VN; x++)
-        if (col + x < W) p[col + x] = V::from_f(acc[x]);
+        if (col + S * x < W) p[col + S * x] = V::from_f(acc[x]);
     }
   };
   auto enter = [&](int q) {
@@ -226,7 +233,7 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
     } else {
       const ST* p = crow0 + q * C.ld;
 #pragma unroll
-      for (int x = 0; x < VN; x++) acc[x] = (col + x < W) ? V::to_f(p[col + x]) : 0.f;
+      for (int x = 0; x < VN; x++) acc[x] = (col + S * x < W) ? V::to_f(p[col + S * x]) : 0.f;
     }
   };
   for (int64_t g0 = 0; g0 < gk; g0 += 32) {
@@ -329,14 +336,37 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
           }
         }
       } else {
-        for (int u = 0; u < ne; u++) {
-          const uint4 en = t[u];
-          if (GROUP && (int)en.w != cur) enter((int)en.w);
-          const ST* rp = reinterpret_cast<const ST*>((uint64_t)en.x | ((uint64_t)en.y << 32));
-          const float vs = __uint_as_float(en.z);
+        if constexpr (EU == 0) {
+          for (int u = 0; u < ne; u++) {
+            const uint4 en = t[u];
+            if (GROUP && (int)en.w != cur) enter((int)en.w);
+            const ST* rp = reinterpret_cast<const ST*>((uint64_t)en.x | ((uint64_t)en.y << 32));
+            const float vs = __uint_as_float(en.z);
 #pragma unroll
-          for (int x = 0; x < VN; x++)
-            if (col + x < W) acc[x] = __fmaf_rn(vs, V::to_f(rp[col + x]), acc[x]);
+            for (int x = 0; x < VN; x++)
+              if (col + x < W) acc[x] = __fmaf_rn(vs, V::to_f(rp[col + x]), acc[x]);
+          }
+        }
+        for (int u0 = 0; EU > 0 && u0 < ne; u0 += EU) {
+          ST raw[EU > 0 ? EU : 1][VN];
+          float vs[EU > 0 ? EU : 1];
+#pragma unroll
+          for (int u = 0; u < EU; u++) {
+            const uint4 en = t[(u0 + u) & 31];
+            const ST* rp = reinterpret_cast<const ST*>((uint64_t)en.x | ((uint64_t)en.y << 32));
+            vs[u] = __uint_as_float(en.z);
+#pragma unroll
+            for (int x = 0; x < VN; x++)
+              if (col + S * x < W) raw[u][x] = rp[col + S * x];
+          }
+#pragma unroll
+          for (int u = 0; u < EU; u++)
+            if (u0 + u < ne) {
+              if (GROUP && ((heads >> (u0 + u)) & 1u)) enter((int)t[u0 + u].w);
+#pragma unroll
+              for (int x = 0; x < VN; x++)
+                if (col + S * x < W) acc[x] = __fmaf_rn(vs[u], V::to_f(raw[u][x]), acc[x]);
+            }
         }
       }
       __syncwarp();
@@ -350,7 +380,11 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
 // flight while the current item runs), so warps that draw short rows take
 // more of them: the cost of a (row group, panel) item varies by orders of
 // magnitude on power-law matrices.
-template <typename ST, bool GROUP, bool SUB>
+// ELEM: every tile element by element (rows off 16 bytes).  Otherwise the tiles
+// whose bases lie off 16 bytes are, with as many loads in flight as cost the
+// vector walk no registers (with 16, R-MAT s21 x 256 FP32 3.94 -> 4.26 ms; in BF16
+// a second copy of the walk costs it as much: 2.10 -> 2.22 ms).
+template <typename ST, bool GROUP, bool SUB, bool ELEM>
 __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     k_spmm(SpGridView A, DGridView B, DGridView C, int tjn, int64_t n_items, int npanels, int R, int64_t ngroups,
            int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag,
@@ -386,14 +420,20 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
-      if (t != at) {
-        aligned = row_align_ok > 0 && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+      if (!ELEM && t != at) {
+        aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
         at = t;
       }
-      const bool vec = aligned;
       // rows flagged long are k_spmm_long's (it takes the aligned ones), or
-      // k_spmm_chain's (row_align_ok < 0: all of them)
-      spmm_rows<ST, GROUP, SUB>(A, B, C, ti, tj, r0, R, c0, W, vec, vec || row_align_ok < 0 ? long_flag : nullptr);
+      // k_spmm_chain's (ELEM: all of them)
+      if (ELEM)
+        spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag);
+      else if (sizeof(ST) == 2)
+        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, aligned, aligned ? long_flag : nullptr);
+      else if (aligned)
+        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag);
+      else
+        spmm_rows<ST, GROUP, SUB, 2>(A, B, C, ti, tj, r0, R, c0, W, false, nullptr);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1302,10 +1342,10 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
   const uint8_t* lflag = flag;
   const int pmajor = (int)tuning(ctx, BCLX_TUNE_SPMM_PANEL_MAJOR);
   if (R > 1)
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB, false>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
                                ctr));
   else
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB, false>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
                                ctr));
   note_launch();
   BCLX_CK_LAUNCH();
@@ -1388,10 +1428,11 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   };
   // A lane group of 32 takes one row; k_spmm shares a warp's set-up among up to
   // four, element by element, and a panel of its lanes is 512 bytes.  So it takes the
-  // short rows where the long ones are listed: uniform 186,581 x 150 FP32, 5
-  // entries a row, 438 -> 270 us; stencil of 262,144 x 185 BF16 1041 -> 799 (R-MAT of 273,612 x
-  // 118 FP32 570 -> 769, of 300,000 x 201 1184 -> 1361, of 1,432,750 x 87 2467 -> 2391,
-  // of 100,000 x 90 BF16 229 -> 217, with rows long from 512 entries).
+  // short rows where the long ones are listed: k_spmm_narrow against k_spmm,
+  // uniform 186,581 x 150 FP32, 5 entries a row, 438 and 201 us; stencil of
+  // 262,144 x 185 BF16 1041 and 587; R-MAT FP32 of 273,612 x 118 570 and 524, of
+  // 300,000 x 201 1184 and 1001, of 1,432,750 x 87 2467 and 2360 (with rows long
+  // from 512 entries).
   auto wide = [&]() {
     const int wp = (int)ceil_div(width, 32 * Vec<ST>::N);
     const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
@@ -1399,10 +1440,10 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
     const int64_t blocks = std::min(ceil_div(items, kSpmmWarps), (int64_t)ctx->num_sms * 4);
     const uint8_t* skip = flag;
     if (R > 1)
-      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, true, SUB>, A, B, C, tjn, items, wp, R,
-                          groups, -1, 0, skip, ctr);
-    return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, false, SUB>, A, B, C, tjn, items, wp, 1,
-                        groups, -1, 0, skip, ctr);
+      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, true, SUB, true>, A, B, C, tjn, items,
+                          wp, R, groups, 0, 0, skip, ctr);
+    return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, false, SUB, true>, A, B, C, tjn, items,
+                        wp, 1, groups, 0, 0, skip, ctr);
   };
   if (!listed) BCLX_TRY(narrow());
   if (chains) {
