@@ -380,6 +380,8 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
 // flight while the current item runs), so warps that draw short rows take
 // more of them: the cost of a (row group, panel) item varies by orders of
 // magnitude on power-law matrices.
+// all_long: every row flagged long is k_spmm_chain's; otherwise k_spmm_long
+// takes them on aligned tiles.
 // ELEM: every tile element by element (rows off 16 bytes).  Otherwise the tiles
 // whose bases lie off 16 bytes are, with as many loads in flight as cost the
 // vector walk no registers (with 16, R-MAT s21 x 256 FP32 3.94 -> 4.26 ms; in BF16
@@ -387,7 +389,7 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
 template <typename ST, bool GROUP, bool SUB, bool ELEM>
 __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     k_spmm(SpGridView A, DGridView B, DGridView C, int tjn, int64_t n_items, int npanels, int R, int64_t ngroups,
-           int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag,
+           int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag, bool all_long,
            unsigned long long* __restrict__ next_item) {
   constexpr int PW = 32 * Vec<ST>::N;
   const int lane = lane_id();
@@ -424,16 +426,14 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
         aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
         at = t;
       }
-      // rows flagged long are k_spmm_long's (it takes the aligned ones), or
-      // k_spmm_chain's (ELEM: all of them)
       if (ELEM)
         spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag);
       else if (sizeof(ST) == 2)
-        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, aligned, aligned ? long_flag : nullptr);
+        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, aligned, aligned || all_long ? long_flag : nullptr);
       else if (aligned)
         spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag);
       else
-        spmm_rows<ST, GROUP, SUB, 2>(A, B, C, ti, tj, r0, R, c0, W, false, nullptr);
+        spmm_rows<ST, GROUP, SUB, 2>(A, B, C, ti, tj, r0, R, c0, W, false, all_long ? long_flag : nullptr);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1343,10 +1343,10 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
   const int pmajor = (int)tuning(ctx, BCLX_TUNE_SPMM_PANEL_MAJOR);
   if (R > 1)
     BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB, false>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
-                               ctr));
+                               false, ctr));
   else
     BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB, false>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
-                               ctr));
+                               false, ctr));
   note_launch();
   BCLX_CK_LAUNCH();
   if (long_path) {
@@ -1385,7 +1385,7 @@ static int launch_after(Context* ctx, bool early, unsigned grid, unsigned thread
 // columns each (the last may have fewer), rows on U bytes.
 template <typename ST, int U, int NV, bool SUB>
 static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& B, const DGridView& C, int tj0,
-                            int tjn, int64_t width, int L) {
+                            int tjn, int64_t width, int L, bool wide_rows) {
   constexpr int PW = 32 * NV * Unit<ST, U>::N;
   const int npanels = (int)ceil_div(width, PW);
   const int64_t ngroups = ceil_div(C.tm, (int64_t)(32 / L));
@@ -1403,7 +1403,7 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   const bool listed = chains && arows >= spmm_long_min_rows();
   int long_row = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_ROW);
   const bool few = chains && !listed && long_row <= 0;
-  if (long_row <= 0) long_row = std::min(kNarrowLongSteps * L, listed && L == 32 && tj0 == 0 ? 512 : INT_MAX);
+  if (long_row <= 0) long_row = std::min(kNarrowLongSteps * L, listed && wide_rows ? 512 : INT_MAX);
   if (!chains) long_row = INT_MAX;
   const int long_least = few ? std::min(kNarrowFewLong, long_row) : long_row;
   // counters: [0] row groups taken, [1] long rows taken, [2] listed very long / other long rows (2 x int32)
@@ -1427,23 +1427,28 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
                         tj0, tjn, L, npanels, n_items, ngroups, long_row, long_least, listed ? nullptr : list, cnt, ctr);
   };
   // A lane group of 32 takes one row; k_spmm shares a warp's set-up among up to
-  // four, element by element, and a panel of its lanes is 512 bytes.  So it takes the
+  // four, and a panel of its lanes is 512 bytes.  So it takes the
   // short rows where the long ones are listed: k_spmm_narrow against k_spmm,
   // uniform 186,581 x 150 FP32, 5 entries a row, 438 and 201 us; stencil of
   // 262,144 x 185 BF16 1041 and 587; R-MAT FP32 of 273,612 x 118 570 and 524, of
   // 300,000 x 201 1184 and 1001, of 1,432,750 x 87 2467 and 2360 (with rows long
-  // from 512 entries).
+  // from 512 entries).  With 17 tiles along k and more every row takes 32 lanes,
+  // and k_spmm has the lighter set-up for one as well (by 16-byte vectors where the
+  // rows lie on 16 bytes): R-MAT of 400,000 on 20 x 20 tiles, x 16 FP32 488 and 410 us
+  // (k_spmm with its own long rows, as launch_wide runs it: 640), x 64 572 and
+  // 495 (650), x 64 BF16 649 and 479 (798), x 17 FP32 577 and 447, x 47 597 and 556.
   auto wide = [&]() {
     const int wp = (int)ceil_div(width, 32 * Vec<ST>::N);
     const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
     const int64_t groups = ceil_div(C.tm, (int64_t)R), items = C.gm * tjn * groups * wp;
     const int64_t blocks = std::min(ceil_div(items, kSpmmWarps), (int64_t)ctx->num_sms * 4);
     const uint8_t* skip = flag;
-    if (R > 1)
-      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, true, SUB, true>, A, B, C, tjn, items,
-                          wp, R, groups, 0, 0, skip, ctr);
-    return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, k_spmm<ST, false, SUB, true>, A, B, C, tjn, items,
-                        wp, 1, groups, 0, 0, skip, ctr);
+    auto go = [&](auto kern) {
+      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, kern, A, B, C, tjn, items, wp, R, groups, 1, 0,
+                          skip, true, ctr);
+    };
+    if constexpr (U == 16) return R > 1 ? go(k_spmm<ST, true, SUB, false>) : go(k_spmm<ST, false, SUB, false>);
+    else return R > 1 ? go(k_spmm<ST, true, SUB, true>) : go(k_spmm<ST, false, SUB, true>);
   };
   if (!listed) BCLX_TRY(narrow());
   if (chains) {
@@ -1455,7 +1460,7 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
                           (int)ceil_div(width * (int64_t)sizeof(ST), 4 * kChainPanelWords), stride, each, !listed, list,
                           cnt, ctr + 1));
   }
-  if (listed) BCLX_TRY(L == 32 && tj0 == 0 ? wide() : narrow());
+  if (listed) BCLX_TRY(wide_rows ? wide() : narrow());
   scratch_free(ctx, flag);
   scratch_free(ctx, list);
   scratch_free(ctx, ctr);
@@ -1473,11 +1478,14 @@ static int launch_narrow_u(Context* ctx, const SpGridView& A, const DGridView& B
   int L = 8;
   while (L < 32 && (L * per < units || L < A.gn)) L *= 2;
   const int64_t nv = ceil_div(std::min<int64_t>(units, 32 * per), L);
+  // rows that take all 32 lanes, for their width or for the stages' sake (k_spmm
+  // starts at tile column 0): see `wide` in launch_narrow_nv
+  const bool wide_rows = L == 32 && tj0 == 0;
   if constexpr (U != 16) {
-    if (nv > 2) return launch_narrow_nv<ST, U, 4, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
-    if (nv > 1) return launch_narrow_nv<ST, U, 2, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
+    if (nv > 2) return launch_narrow_nv<ST, U, 4, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L, wide_rows);
+    if (nv > 1) return launch_narrow_nv<ST, U, 2, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L, wide_rows);
   }
-  return launch_narrow_nv<ST, U, 1, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L);
+  return launch_narrow_nv<ST, U, 1, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L, wide_rows);
 }
 
 template <typename ST, bool SUB>
