@@ -737,7 +737,12 @@ constexpr int64_t kNarrowMaxBytes = 256;
 constexpr int kChainWarps = 8;            // one applies, the others copy
 constexpr int kChainPanelWords = 32;      // words of a long row that a block takes at once: one per consumer lane
 constexpr int kChainBuffers = 3;
-constexpr int kChainBytes = 92 * 1024;    // shared memory for their slices and values (two blocks per SM)
+constexpr int kChainEach = 32;            // entries of a batch per copying warp: one per lane
+// Shared memory for slices of `stride` words and their values.
+constexpr size_t chain_bytes(int stride) {
+  return 4 * (size_t)(kChainBuffers * (kChainWarps - 1) * kChainEach * (stride + 1) + kChainPanelWords);
+}
+static_assert(chain_bytes(kChainPanelWords) <= 92 * 1024, "two blocks per SM");
 
 // First lane whose inclusive prefix exceeds e (32 when none does).
 __device__ __forceinline__ int warp_search_lanes(int32_t incl, int32_t e) {
@@ -904,15 +909,18 @@ __device__ __forceinline__ unsigned narrow_rows(const SpGridView& A, const DGrid
 // Rows [r0, r1) of C tile (ti, tj), columns [c0, c1), one column per lane and
 // one entry at a time: tiles whose base is off the launch's unit (the host
 // sees their leading dimensions and widths, not the device array of bases).
+// Rows of long_row entries or more are left out; their mask is returned.
 template <typename ST, bool SUB>
-__device__ __forceinline__ void elem_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
-                                          int64_t tj, int64_t r0, int64_t r1, int c0, int c1, int long_row) {
+__device__ __forceinline__ unsigned elem_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
+                                              int64_t tj, int64_t r0, int64_t r1, int c0, int c1, int long_row) {
+  unsigned left = 0u;
   for (int64_t r = r0; r < r1; r++) {
     int64_t total = 0;
     for (int64_t k = 0; k < A.gn; k++) {
       const int32_t* rp = A.tile(ti, k).row_ptr + r;
       total += __ldg(rp + 1) - __ldg(rp);
     }
+    if (total >= long_row) left |= 1u << (r - r0);
     if (total == 0 || total >= long_row) continue;
     ST* crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld;
     for (int c = c0 + lane_id(); c < c1; c += 32) {
@@ -925,6 +933,7 @@ __device__ __forceinline__ void elem_rows(const SpGridView& A, const DGridView& 
       crow[c] = Vec<ST>::from_f(acc);
     }
   }
+  return left;
 }
 
 // The chains of n entries in a buffer: this lane's word of each slice at `sw`
@@ -980,21 +989,21 @@ __device__ __forceinline__ void chain_apply(const uint32_t* sw, const float* sv,
 
 // One long row r of C tile (ti, tj), columns [c0, c0 + W) (at most
 // kChainPanelWords words), by the whole block: warp 0 applies, the others
-// copy, `each` entries of a batch per producer warp.  While batch b is
+// copy, kChainEach entries of a batch per producer warp.  While batch b is
 // applied from its buffer, batches b + 1 and b + 2 are in flight.  One barrier
 // per batch: past it batch b has landed (each producer waited for its own
 // copies) and batch b - 1, whose buffer batch b + 2 overwrites, has been
 // applied.  At most 32 stages.  Buffers: slices of `stride` words, then the
 // values.
 template <typename ST, bool SUB>
-__device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int stride, int each, const SpGridView& A,
+__device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int stride, const SpGridView& A,
                                           const DGridView& B, const DGridView& C, int64_t ti, int64_t tj, int64_t r,
                                           int c0, int W, int unit) {
   constexpr int CN = 4 / (int)sizeof(ST);  // columns per word
   const int lane = lane_id();
   const int prod = (int)(threadIdx.x >> 5) - 1;  // producer number; -1: the consumer
   const int nw = (W * (int)sizeof(ST) + 3) >> 2;
-  const int batch = each * (kChainWarps - 1);
+  constexpr int each = kChainEach, batch = each * (kChainWarps - 1);
   ST* __restrict__ crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld + c0;
   const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, lane, true);
   const int32_t aincl = warp_inclusive_scan(sl.alen);
@@ -1107,24 +1116,24 @@ __device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int str
 }
 
 // Long rows of tile columns [tj0, tj0 + tjn), a block per (row, tile column,
-// panel).  `met`: list[0, count[0]) holds row * tjn + tile column of the rows
-// that k_spmm_narrow met (its programmatic dependent: it waits for it);
+// panel).  `met`: list[0, count[0]) holds the rows that k_spmm_narrow met (its
+// programmatic dependent: it waits for it);
 // otherwise the rows k_spmm_find_long listed, and k_spmm_narrow may start.
 template <typename ST, bool SUB>
 __global__ void __launch_bounds__(kChainWarps * 32, 2)
-    k_spmm_chain(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int npanels, int stride, int each, bool met,
+    k_spmm_chain(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int npanels, int stride, bool met,
                  const int64_t* __restrict__ list, const int32_t* __restrict__ count,
                  unsigned long long* __restrict__ next_item) {
   if (met) asm volatile("griddepcontrol.wait;\n" ::: "memory");
   else asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   extern __shared__ __align__(16) unsigned char chain_smem[];
-  __shared__ int64_t item[2], code[2];
+  __shared__ int64_t item[2], row[2];
   uint32_t* slices = reinterpret_cast<uint32_t*>(chain_smem);
-  float* vals = reinterpret_cast<float*>(slices + kChainBuffers * (kChainWarps - 1) * each * stride + kChainPanelWords);
+  float* vals = reinterpret_cast<float*>(slices + kChainBuffers * (kChainWarps - 1) * kChainEach * stride + kChainPanelWords);
   constexpr int PW = kChainPanelWords * 4 / (int)sizeof(ST);
   const int64_t rows = A.gm * A.tm;
   const int64_t nv = count[0], nl = nv + (met ? 0 : count[1]);
-  const int64_t per = (met ? 1 : tjn) * (int64_t)npanels;
+  const int64_t per = tjn * (int64_t)npanels;
   const int64_t n = nl * per;
   // thread 0 takes an item and reads its row ahead, while the block works on
   // the one before
@@ -1133,7 +1142,7 @@ __global__ void __launch_bounds__(kChainWarps * 32, 2)
     item[slot] = it < n ? it : -1;
     if (it < n) {
       const int64_t q = it / per;
-      code[slot] = q < nv ? list[q] : list[rows - 1 - (q - nv)];
+      row[slot] = q < nv ? list[q] : list[rows - 1 - (q - nv)];
     }
   };
   if (threadIdx.x == 0) take(0);
@@ -1141,23 +1150,24 @@ __global__ void __launch_bounds__(kChainWarps * 32, 2)
   for (int slot = 0;; slot ^= 1) {
     const int64_t it = item[slot];
     if (it < 0) break;
-    const int64_t x = met ? code[slot] / tjn : code[slot];  // the row, over all tile rows
-    const int pt = (int)(it % per);
-    const int64_t tj = tj0 + (met ? code[slot] - x * tjn : pt / npanels);
+    const int64_t x = row[slot];  // over all tile rows
+    const int64_t pt = it % per;
+    const int64_t tj = tj0 + pt / npanels;
     const int64_t ti = x / A.tm;
-    const int W = (int)C.cols_of(tj), c0 = pt % npanels * PW;
+    const int W = (int)C.cols_of(tj), c0 = (int)(pt % npanels) * PW;
     if (threadIdx.x == 0) take(slot ^ 1);
     if (c0 < W) {
       const int unit = tile_on<ST, 16>(B, C, ti, tj, W) ? 16 : (tile_on<ST, 4>(B, C, ti, tj, W) ? 4 : 2);
-      chain_row<ST, SUB>(slices, vals, stride, each, A, B, C, ti, tj, x - ti * A.tm, c0, min(PW, W - c0), unit);
+      chain_row<ST, SUB>(slices, vals, stride, A, B, C, ti, tj, x - ti * A.tm, c0, min(PW, W - c0), unit);
     } else {
       __syncthreads();  // (chain_row ends with a barrier)
     }
   }
 }
 
-// Short rows of tile columns [tj0, tj0 + tjn).  With `met` the long rows go to
-// that list (met_count their number), otherwise they are left to k_spmm_chain.
+// Short rows of tile columns [tj0, tj0 + tjn); the long rows are left to
+// k_spmm_chain.  With `met` the first tile column's items list them there
+// (met_count their number): which rows are long depends on A alone.
 // A row is long from long_most entries, or from long_least and four times the
 // mean of its tile row.
 template <typename ST, int U, int NV, bool SUB>
@@ -1194,15 +1204,11 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
       const int c1 = min(W, c0 + PW);
-      if (on) {
-        unsigned left = narrow_rows<ST, U, NV, SUB>(A, B, C, ti, tj, r0, L, c0, c1 - c0, long_row);
-        if (met && panel == 0 && lane == 0)
-          for (; left; left &= left - 1)
-            met[atomicAdd(met_count, 1)] = (ti * A.tm + r0 + __ffs(left) - 1) * tjn + (tj - tj0);
-      } else {
-        // (met: none is left to k_spmm_chain, whose list this kernel fills by rows on the unit)
-        elem_rows<ST, SUB>(A, B, C, ti, tj, r0, min(r0 + 32 / L, C.rows_of(ti)), c0, c1, met ? INT_MAX : long_row);
-      }
+      unsigned left;
+      if (on) left = narrow_rows<ST, U, NV, SUB>(A, B, C, ti, tj, r0, L, c0, c1 - c0, long_row);
+      else left = elem_rows<ST, SUB>(A, B, C, ti, tj, r0, min(r0 + 32 / L, C.rows_of(ti)), c0, c1, long_row);
+      if (met && tj == tj0 && panel == 0 && lane == 0)
+        for (; left; left &= left - 1) met[atomicAdd(met_count, 1)] = ti * A.tm + r0 + __ffs(left) - 1;
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1391,13 +1397,10 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   const int64_t ngroups = ceil_div(C.tm, (int64_t)(32 / L));
   const int64_t n_items = C.gm * tjn * ngroups * npanels;
   if (n_items == 0) return BCLX_OK;
-  // long rows: slices a power of two of words apart, batches of as many
-  // entries as three buffers hold, a whole number of eights per producer warp
+  // long rows: slices a power of two of words apart
   int stride = 4;
   while (stride < kChainPanelWords && stride * 4 < width * (int64_t)sizeof(ST)) stride *= 2;
-  const int fit = kChainBytes / (kChainBuffers * (kChainWarps - 1) * (stride + 1) * 4);
-  const int each = std::min(32, fit / 8 * 8);
-  const size_t smem = 4 * (size_t)(kChainBuffers * (kChainWarps - 1) * each * (stride + 1) + kChainPanelWords);
+  const size_t smem = chain_bytes(stride);
   const int64_t arows = A.gm * A.tm;
   const bool chains = A.gn <= 32;  // one lane per stage
   const bool listed = chains && arows >= spmm_long_min_rows();
@@ -1413,7 +1416,7 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   BCLX_TRY(scratch_alloc_n(ctx, &ctr, 3));
   BCLX_CK(cudaMemsetAsync(ctr, 0, 3 * sizeof(unsigned long long), ctx->stream));
   int32_t* cnt = reinterpret_cast<int32_t*>(ctr + 2);
-  if (chains) BCLX_TRY(scratch_alloc_n(ctx, &list, (size_t)arows * (listed ? 1 : tjn)));
+  if (chains) BCLX_TRY(scratch_alloc_n(ctx, &list, (size_t)arows));
   if (listed) {
     BCLX_TRY(scratch_alloc_n(ctx, &flag, (size_t)arows));
     k_spmm_find_long<<<(unsigned)std::min<int64_t>(ceil_div(arows, 256), (int64_t)ctx->num_sms * 16), 256, 0,
@@ -1457,7 +1460,7 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
     // one block per SM beside k_spmm_narrow, two where it has finished
     const int64_t blocks = std::min<int64_t>(arows * tjn, (int64_t)ctx->num_sms * (listed ? 1 : 2));
     BCLX_TRY(launch_after(ctx, !listed, (unsigned)blocks, kChainWarps * 32, smem, kern, A, B, C, tj0, tjn,
-                          (int)ceil_div(width * (int64_t)sizeof(ST), 4 * kChainPanelWords), stride, each, !listed, list,
+                          (int)ceil_div(width * (int64_t)sizeof(ST), 4 * kChainPanelWords), stride, !listed, list,
                           cnt, ctr + 1));
   }
   if (listed) BCLX_TRY(wide_rows ? wide() : narrow());

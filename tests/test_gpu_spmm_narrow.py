@@ -119,3 +119,29 @@ def test_wide_unaligned_listed(monkeypatch, matrix, dtype, n, tiles):
     listed: the others go to the wide kernel, several to a warp and one."""
     monkeypatch.setenv("BCLX_SPMM_LONG_MIN_ROWS", "0")
     check(matrix, n, (*tiles, n), dtype, seed=n)
+
+
+def test_scratch_does_not_grow_with_the_tile_columns():
+    """Few rows and many narrow tile columns: the long rows are listed once for all of
+    them (and run for each)."""
+    import torch
+    from bcl_b200 import gen
+    from bcl_b200.containers import BlockCustom, DMatrix, SPMatrix, context, gemm
+    m, k, n = 60000, 600, 512
+    rng = np.random.default_rng(0)
+    lens = np.where(np.arange(m) % 9000 == 17, 500, 1)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(k, x, replace=False)) for x in lens]).astype(np.int32)
+    a = gen.CSR(m, k, rp, ci, rng.integers(-4, 5, ci.size).astype(np.float32))
+    A = SPMatrix.from_csr(a, BlockCustom((m, k)))
+    b = torch.from_numpy(rng.integers(-4, 5, (k, n)).astype(np.float32)).cuda()
+    B, C = DMatrix.from_array(b, BlockCustom((k, 1))), DMatrix.zeros((m, n), BlockCustom((m, 1)))
+    dense = torch.sparse_csr_tensor(*(torch.from_numpy(x).cuda() for x in (a.row_ptr.astype(np.int64), a.col_ind.astype(np.int64), a.vals)), (m, k))
+    context().synchronize()
+    context().release_cached()
+    before = torch.cuda.mem_get_info()[0]
+    gemm(A, B, C)
+    torch.cuda.synchronize()
+    used = before - torch.cuda.mem_get_info()[0]
+    assert used <= 64 << 20, used
+    assert torch.equal(C.get_matrix(), (dense @ b))  # whole values: exact in any order
