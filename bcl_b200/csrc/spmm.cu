@@ -183,7 +183,8 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 // (one lane per (row, stage)); R == 1 takes the stages 32 at a time.
 // GROUP = false compiles the one-row walk alone (R == 1, no row changes to
 // test for inside the unrolled loop).  `skip` (or null): rows flagged there
-// are left to another kernel.  `vec`: every B and C row slice of this tile
+// are left to another kernel.  MET (at most 32 stages): so are rows of long_row
+// entries or more, and their mask is returned.  `vec`: every B and C row slice of this tile
 // pair is 16-byte aligned; otherwise element-wise access.
 // There a lane's columns are every 32nd, so that the warp's loads of an entry are
 // of neighbouring words, and EU entries' loads are in flight: with a lane's
@@ -191,10 +192,10 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 // 186,581 x 150 FP32 270 us, now 201, stencil of 262,144 x 185 BF16 799, now 587,
 // R-MAT of 273,612 x 118 FP32 765, now 524; tiles whose bases lie off 16 bytes,
 // uniform 300,000 x 256 FP32 1834, now 927.
-template <typename ST, bool GROUP, bool SUB, int EU, int UNROLL = kSpmmUnroll>
-__device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
-                                          int64_t tj, int64_t r0, int R, int c0, int W, bool vec,
-                                          const uint8_t* __restrict__ skip) {
+template <typename ST, bool GROUP, bool SUB, int EU, bool MET = false, int UNROLL = kSpmmUnroll>
+__device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
+                                              int64_t tj, int64_t r0, int R, int c0, int W, bool vec,
+                                              const uint8_t* __restrict__ skip, int long_row = INT_MAX) {
   if (!GROUP) R = 1;
   using V = Vec<ST>;
   constexpr int VN = V::N;
@@ -212,6 +213,7 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
   float acc[VN];
   int cur = -1;  // row whose chain is in acc
   bool staged = false;
+  unsigned left = 0u;
   auto flush = [&]() {
     if (cur < 0 || !own) return;
     ST* p = crow0 + cur * C.ld;
@@ -241,8 +243,18 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
     const int64_t kk = GROUP ? lane - ql * gk : g0 + lane;
     bool valid = ql < nrows;
     if (valid && skip) valid = skip[ti * C.tm + r0 + ql] == 0;
-    const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r0 + ql, kk, valid);
-    const int32_t aincl = warp_inclusive_scan(sl.alen);
+    StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r0 + ql, kk, valid);
+    int32_t aincl = warp_inclusive_scan(sl.alen);
+    if (MET) {
+      const int last = GROUP ? min(ql * gk + gk - 1, 31) : 31, first = GROUP ? min(ql * gk, 31) : 0;
+      const int32_t through = __shfl_sync(kFull, aincl, last), from = __shfl_sync(kFull, aincl - sl.alen, first);
+      const bool lng = valid && through - from >= long_row;
+      left = __reduce_or_sync(kFull, lng ? 1u << ql : 0u);
+      if (left) {
+        if (lng) sl.alen = 0;
+        aincl = warp_inclusive_scan(sl.alen);
+      }
+    }
     const int32_t atot = __shfl_sync(kFull, aincl, 31);
     if (atot == 0) continue;
     const int32_t aexcl = aincl - sl.alen;
@@ -373,6 +385,26 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
     }
   }
   flush();
+  return left;
+}
+
+// Rows that a kernel of short rows lists and leaves to k_spmm_chain: from `most`
+// entries, or from `least` and four times the mean of their tile row.  (Which
+// rows are long depends on A alone: the first tile column's items list them.)
+struct MetRows {
+  int64_t* list;   // or null: they are listed already
+  int32_t* count;
+  int most, least;
+};
+// The bound in tile row ti (at most 32 tiles along k where least < most).
+__device__ __forceinline__ int met_bound(const MetRows& met, const SpGridView& A, const DGridView& C, int64_t ti) {
+  if (met.least >= met.most) return met.most;
+  const float nnz = warp_sum(lane_id() < A.gn ? (float)A.tile(ti, lane_id()).nnz : 0.f);
+  return min(met.most, max(met.least, (int)min(4.f * nnz / (float)C.rows_of(ti), 1e9f)));
+}
+// Rows x0 + (bits of left), by one lane.
+__device__ __forceinline__ void list_met(const MetRows& met, int64_t x0, unsigned left) {
+  for (; left; left &= left - 1) met.list[atomicAdd(met.count, 1)] = x0 + __ffs(left) - 1;
 }
 
 // Tile columns [0, tjn) (k_spmm_narrow takes the others).  Warp items come
@@ -380,17 +412,19 @@ __device__ __forceinline__ void spmm_rows(const SpGridView& A, const DGridView& 
 // flight while the current item runs), so warps that draw short rows take
 // more of them: the cost of a (row group, panel) item varies by orders of
 // magnitude on power-law matrices.
+// MET: with at most 32 tiles along k, long rows are listed and left out.
 // all_long: every row flagged long is k_spmm_chain's; otherwise k_spmm_long
 // takes them on aligned tiles.
 // ELEM: every tile element by element (rows off 16 bytes).  Otherwise the tiles
 // whose bases lie off 16 bytes are, with as many loads in flight as cost the
 // vector walk no registers (with 16, R-MAT s21 x 256 FP32 3.94 -> 4.26 ms; in BF16
-// a second copy of the walk costs it as much: 2.10 -> 2.22 ms).
-template <typename ST, bool GROUP, bool SUB, bool ELEM>
+// a second copy of the walk costs it as much: 2.10 -> 2.22 ms; with MET, uniform
+// 60,000 x 16 FP32 on 20 x 20 tiles 90 -> 96 us).
+template <typename ST, bool GROUP, bool SUB, bool ELEM, bool MET = false>
 __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     k_spmm(SpGridView A, DGridView B, DGridView C, int tjn, int64_t n_items, int npanels, int R, int64_t ngroups,
            int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag, bool all_long,
-           unsigned long long* __restrict__ next_item) {
+           MetRows met, unsigned long long* __restrict__ next_item) {
   constexpr int PW = 32 * Vec<ST>::N;
   const int lane = lane_id();
   unsigned long long it = 0;
@@ -400,8 +434,9 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
   // one is some 70 instructions)
   const bool small = n_items <= UINT32_MAX;
   auto divide = [small](int64_t a, int64_t b) { return small ? (int64_t)((uint32_t)a / (uint32_t)b) : a / b; };
-  int64_t at = -1;  // the C tile `aligned` is for
+  int64_t at = -1;  // the C tile `aligned` and `bound` are for
   bool aligned = false;
+  int bound = INT_MAX;
   while (it < (unsigned long long)n_items) {
     unsigned long long nx = 0;
     if (lane == 0) nx = atomicAdd(next_item, 1ULL);
@@ -422,18 +457,23 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
     if (r0 < C.rows_of(ti) && c0 < W) {
-      if (!ELEM && t != at) {
-        aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+      if ((!ELEM || MET) && t != at) {
         at = t;
+        if (!ELEM) aligned = row_align_ok && (W % Vec<ST>::N) == 0 && tiles_aligned(B, C, ti, tj);
+        if (MET) bound = met_bound(met, A, C, ti);
       }
+      unsigned left;
       if (ELEM)
-        spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag);
-      else if (sizeof(ST) == 2)
-        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, aligned, aligned || all_long ? long_flag : nullptr);
+        left = spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N, MET>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag, bound);
+      else if (sizeof(ST) == 2 || MET)
+        left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, aligned,
+                                                 aligned || all_long ? long_flag : nullptr, bound);
       else if (aligned)
-        spmm_rows<ST, GROUP, SUB, 0>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag);
+        left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag, bound);
       else
-        spmm_rows<ST, GROUP, SUB, 2>(A, B, C, ti, tj, r0, R, c0, W, false, all_long ? long_flag : nullptr);
+        left = spmm_rows<ST, GROUP, SUB, 2, MET>(A, B, C, ti, tj, r0, R, c0, W, false, all_long ? long_flag : nullptr,
+                                                 bound);
+      if (MET && left && tj == 0 && panel == 0 && lane == 0) list_met(met, ti * A.tm + r0, left);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1166,15 +1206,11 @@ __global__ void __launch_bounds__(kChainWarps * 32, 2)
 }
 
 // Short rows of tile columns [tj0, tj0 + tjn); the long rows are left to
-// k_spmm_chain.  With `met` the first tile column's items list them there
-// (met_count their number): which rows are long depends on A alone.
-// A row is long from long_most entries, or from long_least and four times the
-// mean of its tile row.
+// k_spmm_chain, and listed for it (MetRows) unless they are listed already.
 template <typename ST, int U, int NV, bool SUB>
 __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
     k_spmm_narrow(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int L, int npanels, int64_t n_items,
-                  int64_t ngroups, int long_most, int long_least, int64_t* __restrict__ met,
-                  int32_t* __restrict__ met_count, unsigned long long* __restrict__ next_item) {
+                  int64_t ngroups, MetRows met, unsigned long long* __restrict__ next_item) {
   constexpr int PW = 32 * NV * Unit<ST, U>::N;  // columns of a panel
   const int lane = lane_id();
   unsigned long long it = 0;
@@ -1182,7 +1218,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
   it = __shfl_sync(kFull, it, 0);
   int64_t at = -1, ti = 0, tj = 0;  // the C tile of the last item
   bool on = false;
-  int long_row = long_most;
+  int long_row = met.most;
   while ((int64_t)it < n_items) {
     unsigned long long nx = 0;
     if (lane == 0) nx = atomicAdd(next_item, 1ULL);
@@ -1195,10 +1231,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
       ti = t / tjn;
       tj = tj0 + (t - ti * tjn);
       on = tile_on<ST, U>(B, C, ti, tj, (int)C.cols_of(tj));
-      if (long_least < long_most) {  // (at most 32 tiles along k)
-        const float nnz = warp_sum(lane < A.gn ? (float)A.tile(ti, lane).nnz : 0.f);
-        long_row = min(long_most, max(long_least, (int)min(4.f * nnz / (float)C.rows_of(ti), 1e9f)));
-      }
+      long_row = met_bound(met, A, C, ti);
     }
     const int W = (int)C.cols_of(tj);
     const int c0 = panel * PW;
@@ -1207,8 +1240,7 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
       unsigned left;
       if (on) left = narrow_rows<ST, U, NV, SUB>(A, B, C, ti, tj, r0, L, c0, c1 - c0, long_row);
       else left = elem_rows<ST, SUB>(A, B, C, ti, tj, r0, min(r0 + 32 / L, C.rows_of(ti)), c0, c1, long_row);
-      if (met && tj == tj0 && panel == 0 && lane == 0)
-        for (; left; left &= left - 1) met[atomicAdd(met_count, 1)] = ti * A.tm + r0 + __ffs(left) - 1;
+      if (met.list && left && tj == tj0 && panel == 0 && lane == 0) list_met(met, ti * A.tm + r0, left);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1349,10 +1381,10 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
   const int pmajor = (int)tuning(ctx, BCLX_TUNE_SPMM_PANEL_MAJOR);
   if (R > 1)
     BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB, false>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
-                               false, ctr));
+                               false, MetRows{}, ctr));
   else
     BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB, false>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
-                               false, ctr));
+                               false, MetRows{}, ctr));
   note_launch();
   BCLX_CK_LAUNCH();
   if (long_path) {
@@ -1409,16 +1441,17 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   if (long_row <= 0) long_row = std::min(kNarrowLongSteps * L, listed && wide_rows ? 512 : INT_MAX);
   if (!chains) long_row = INT_MAX;
   const int long_least = few ? std::min(kNarrowFewLong, long_row) : long_row;
-  // counters: [0] row groups taken, [1] long rows taken, [2] listed very long / other long rows (2 x int32)
+  // one scratch block: counters ([0] row groups taken, [1] long rows taken, [2] listed very long / other long rows,
+  // 2 x int32), the list of long rows, and their flags where they are listed first
   unsigned long long* ctr = nullptr;
-  uint8_t* flag = nullptr;
-  int64_t* list = nullptr;
-  BCLX_TRY(scratch_alloc_n(ctx, &ctr, 3));
+  BCLX_TRY(scratch_alloc(ctx, reinterpret_cast<void**>(&ctr),
+                         sizeof(int64_t) * (size_t)(3 + (chains ? arows : 0)) + (size_t)(listed ? arows : 0)));
   BCLX_CK(cudaMemsetAsync(ctr, 0, 3 * sizeof(unsigned long long), ctx->stream));
   int32_t* cnt = reinterpret_cast<int32_t*>(ctr + 2);
-  if (chains) BCLX_TRY(scratch_alloc_n(ctx, &list, (size_t)arows));
+  int64_t* list = chains ? reinterpret_cast<int64_t*>(ctr + 3) : nullptr;
+  uint8_t* flag = listed ? reinterpret_cast<uint8_t*>(list + arows) : nullptr;
+  const MetRows met{listed ? nullptr : list, cnt, long_row, long_least};
   if (listed) {
-    BCLX_TRY(scratch_alloc_n(ctx, &flag, (size_t)arows));
     k_spmm_find_long<<<(unsigned)std::min<int64_t>(ceil_div(arows, 256), (int64_t)ctx->num_sms * 16), 256, 0,
                        ctx->stream>>>(A, long_row, (int)std::min<int64_t>((int64_t)long_row * 8, INT32_MAX), flag, list, cnt);
     note_launch();
@@ -1427,19 +1460,22 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   auto narrow = [&]() {
     const int64_t blocks = std::min(ceil_div(n_items, kNarrowWarps), (int64_t)ctx->num_sms * 4);
     return launch_after(ctx, listed, (unsigned)blocks, kNarrowWarps * 32, 0, k_spmm_narrow<ST, U, NV, SUB>, A, B, C,
-                        tj0, tjn, L, npanels, n_items, ngroups, long_row, long_least, listed ? nullptr : list, cnt, ctr);
+                        tj0, tjn, L, npanels, n_items, ngroups, met, ctr);
   };
   // A lane group of 32 takes one row; k_spmm shares a warp's set-up among up to
-  // four, and a panel of its lanes is 512 bytes.  So it takes the
-  // short rows where the long ones are listed: k_spmm_narrow against k_spmm,
-  // uniform 186,581 x 150 FP32, 5 entries a row, 438 and 201 us; stencil of
-  // 262,144 x 185 BF16 1041 and 587; R-MAT FP32 of 273,612 x 118 570 and 524, of
-  // 300,000 x 201 1184 and 1001, of 1,432,750 x 87 2467 and 2360 (with rows long
-  // from 512 entries).  With 17 tiles along k and more every row takes 32 lanes,
-  // and k_spmm has the lighter set-up for one as well (by 16-byte vectors where the
-  // rows lie on 16 bytes): R-MAT of 400,000 on 20 x 20 tiles, x 16 FP32 488 and 410 us
-  // (k_spmm with its own long rows, as launch_wide runs it: 640), x 64 572 and
-  // 495 (650), x 64 BF16 649 and 479 (798), x 17 FP32 577 and 447, x 47 597 and 556.
+  // four, and a panel of its lanes is 512 bytes.  So it takes the short rows there:
+  // k_spmm_narrow against k_spmm, uniform 186,581 x 150 FP32, 5 entries a row, 438
+  // and 201 us; stencil of 262,144 x 185 BF16 1041 and 587; uniform 8,069 x 201 43
+  // and 35; R-MAT FP32 of 273,612 x 118 570 and 524, of 300,000 x 201 1184 and 1001,
+  // of 1,432,750 x 87 2467 and 2360, of 20,000 x 201 on 20 x 20 tiles 161 and 139 (long
+  // rows listed and met: from 512 entries, or see kNarrowFewLong).  With 17 tiles along
+  // k and more every row takes 32 lanes, and k_spmm has the lighter set-up for one as
+  // well (by 16-byte vectors where the rows lie on 16 bytes): R-MAT of 400,000 on 20 x
+  // 20 tiles, x 16 FP32 488 and 410 us (k_spmm with its own long rows, as launch_wide
+  // runs it: 640), x 64 572 and 495 (650), x 64 BF16 649 and 479 (798), x 17 FP32 577
+  // and 447, x 47 597 and 556; uniform 20,000 x 64 BF16 49 and 43; with 40 tiles along k
+  // (no chains) uniform 400,000 x 64 BF16 739 and 589, x 201 FP32 1814 and 1270.  Rows of
+  // fewer units stay with k_spmm_narrow: R-MAT of 100,000 x 47 177 and 250.
   auto wide = [&]() {
     const int wp = (int)ceil_div(width, 32 * Vec<ST>::N);
     const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
@@ -1447,13 +1483,17 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
     const int64_t blocks = std::min(ceil_div(items, kSpmmWarps), (int64_t)ctx->num_sms * 4);
     const uint8_t* skip = flag;
     auto go = [&](auto kern) {
-      return launch_after(ctx, true, (unsigned)blocks, kSpmmWarps * 32, 0, kern, A, B, C, tjn, items, wp, R, groups, 1, 0,
-                          skip, true, ctr);
+      return launch_after(ctx, listed, (unsigned)blocks, kSpmmWarps * 32, 0, kern, A, B, C, tjn, items, wp, R, groups, 1,
+                          0, skip, true, met, ctr);
     };
-    if constexpr (U == 16) return R > 1 ? go(k_spmm<ST, true, SUB, false>) : go(k_spmm<ST, false, SUB, false>);
-    else return R > 1 ? go(k_spmm<ST, true, SUB, true>) : go(k_spmm<ST, false, SUB, true>);
+    if constexpr (U == 16) {  // (only for 17 and more tiles along k: R is 1)
+      return met.list ? go(k_spmm<ST, false, SUB, false, true>) : go(k_spmm<ST, false, SUB, false>);
+    } else {
+      if (met.list) return R > 1 ? go(k_spmm<ST, true, SUB, true, true>) : go(k_spmm<ST, false, SUB, true, true>);
+      return R > 1 ? go(k_spmm<ST, true, SUB, true>) : go(k_spmm<ST, false, SUB, true>);
+    }
   };
-  if (!listed) BCLX_TRY(narrow());
+  if (!listed) BCLX_TRY(wide_rows ? wide() : narrow());
   if (chains) {
     auto kern = k_spmm_chain<ST, SUB>;
     BCLX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1464,8 +1504,6 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
                           cnt, ctr + 1));
   }
   if (listed) BCLX_TRY(wide_rows ? wide() : narrow());
-  scratch_free(ctx, flag);
-  scratch_free(ctx, list);
   scratch_free(ctx, ctr);
   return BCLX_OK;
 }
