@@ -90,6 +90,16 @@ constexpr int kSpmmUnroll = 4;  // B-row loads in flight per lane (with 32 warps
 
 constexpr int kSpmmMaxRows = 4;  // rows of one C tile a warp walks together
 
+// A row that a warp walks alone asks L2 for the slices of its next 32 entries from
+// kSpmmAhead entries (of up to 32 stages) on, where B is of kSpmmAheadBytes or more:
+// its chain waits for each group of loads, and there are few such rows (asked for by
+// every row they thrash L2, see spmm_rows).  R-MAT of 400,000 x 256 on 40 x 40 tiles,
+// whose long rows have no kernel of their own, FP32 3.29 -> 2.74 ms, BF16 on 33 x 33
+// 2.91 -> 2.60; R-MAT of 60,000 x 256 FP32 (61 MB) 626 -> 604 us, BF16 (31 MB, in L2 as
+// it is) 549 -> 591.
+constexpr int kSpmmAhead = 256;
+constexpr int64_t kSpmmAheadBytes = 48 << 20;
+
 // Per-warp shared memory of the walk:
 //  * the entry table of a chunk of 32 entries: (B-row address, A value, row) of
 //    each, read back with broadcast 16-byte loads;
@@ -195,7 +205,8 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 template <typename ST, bool GROUP, bool SUB, int EU, bool MET = false, int UNROLL = kSpmmUnroll>
 __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
                                               int64_t tj, int64_t r0, int R, int c0, int W, bool vec,
-                                              const uint8_t* __restrict__ skip, int long_row = INT_MAX) {
+                                              const uint8_t* __restrict__ skip, int long_row = INT_MAX,
+                                              int ahead = INT_MAX) {
   if (!GROUP) R = 1;
   using V = Vec<ST>;
   constexpr int VN = V::N;
@@ -382,6 +393,15 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
         }
       }
       __syncwarp();
+      if (!GROUP && !MET && EU == 0 && e0 + 32 < atot && atot >= ahead) {
+        // a long row's next chunk: its B-row slices, asked for together
+        const char* p = reinterpret_cast<const char*>(
+            reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), nsrc)) +
+            (int64_t)nkc * B.ld + c0);
+        const int bytes = min(W - c0, 32 * VN) * (int)sizeof(ST);
+        if (e0 + 32 + lane < atot)
+          for (int o = 0; o < bytes; o += 128) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p + o));
+      }
     }
   }
   flush();
@@ -437,6 +457,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
   int64_t at = -1;  // the C tile `aligned` and `bound` are for
   bool aligned = false;
   int bound = INT_MAX;
+  const int ahead = B.m * B.ld * (int64_t)sizeof(ST) >= kSpmmAheadBytes ? kSpmmAhead : INT_MAX;
   while (it < (unsigned long long)n_items) {
     unsigned long long nx = 0;
     if (lane == 0) nx = atomicAdd(next_item, 1ULL);
@@ -467,9 +488,9 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
         left = spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N, MET>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag, bound);
       else if (sizeof(ST) == 2 || MET)
         left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, aligned,
-                                                 aligned || all_long ? long_flag : nullptr, bound);
+                                                 aligned || all_long ? long_flag : nullptr, bound, ahead);
       else if (aligned)
-        left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag, bound);
+        left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, true, long_flag, bound, ahead);
       else
         left = spmm_rows<ST, GROUP, SUB, 2, MET>(A, B, C, ti, tj, r0, R, c0, W, false, all_long ? long_flag : nullptr,
                                                  bound);
