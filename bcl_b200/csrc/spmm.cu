@@ -202,7 +202,7 @@ __device__ __forceinline__ bool tiles_aligned(const DGridView& B, const DGridVie
 // 186,581 x 150 FP32 270 us, now 201, stencil of 262,144 x 185 BF16 799, now 587,
 // R-MAT of 273,612 x 118 FP32 765, now 524; tiles whose bases lie off 16 bytes,
 // uniform 300,000 x 256 FP32 1834, now 927.
-template <typename ST, bool GROUP, bool SUB, int EU, bool MET = false, int UNROLL = kSpmmUnroll>
+template <typename ST, bool GROUP, bool SUB, int EU, bool MET = false, int XN = Vec<ST>::N, int UNROLL = kSpmmUnroll>
 __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridView& B, const DGridView& C, int64_t ti,
                                               int64_t tj, int64_t r0, int R, int c0, int W, bool vec,
                                               const uint8_t* __restrict__ skip, int long_row = INT_MAX,
@@ -232,7 +232,7 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
       V::store(p + col, acc);
     } else {
 #pragma unroll
-      for (int x = 0; x < VN; x++)
+      for (int x = 0; x < XN; x++)
         if (col + S * x < W) p[col + S * x] = V::from_f(acc[x]);
     }
   };
@@ -246,7 +246,7 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
     } else {
       const ST* p = crow0 + q * C.ld;
 #pragma unroll
-      for (int x = 0; x < VN; x++) acc[x] = (col + S * x < W) ? V::to_f(p[col + S * x]) : 0.f;
+      for (int x = 0; x < XN; x++) acc[x] = (col + S * x < W) ? V::to_f(p[col + S * x]) : 0.f;
     }
   };
   for (int64_t g0 = 0; g0 < gk; g0 += 32) {
@@ -371,7 +371,7 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
           }
         }
         for (int u0 = 0; EU > 0 && u0 < ne; u0 += EU) {
-          ST raw[EU > 0 ? EU : 1][VN];
+          ST raw[EU > 0 ? EU : 1][XN];
           float vs[EU > 0 ? EU : 1];
 #pragma unroll
           for (int u = 0; u < EU; u++) {
@@ -379,7 +379,7 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
             const ST* rp = reinterpret_cast<const ST*>((uint64_t)en.x | ((uint64_t)en.y << 32));
             vs[u] = __uint_as_float(en.z);
 #pragma unroll
-            for (int x = 0; x < VN; x++)
+            for (int x = 0; x < XN; x++)
               if (col + S * x < W) raw[u][x] = rp[col + S * x];
           }
 #pragma unroll
@@ -387,7 +387,7 @@ __device__ __forceinline__ unsigned spmm_rows(const SpGridView& A, const DGridVi
             if (u0 + u < ne) {
               if (GROUP && ((heads >> (u0 + u)) & 1u)) enter((int)t[u0 + u].w);
 #pragma unroll
-              for (int x = 0; x < VN; x++)
+              for (int x = 0; x < XN; x++)
                 if (col + S * x < W) acc[x] = __fmaf_rn(vs[u], V::to_f(raw[u][x]), acc[x]);
             }
         }
@@ -435,17 +435,17 @@ __device__ __forceinline__ void list_met(const MetRows& met, int64_t x0, unsigne
 // MET: with at most 32 tiles along k, long rows are listed and left out.
 // all_long: every row flagged long is k_spmm_chain's; otherwise k_spmm_long
 // takes them on aligned tiles.
-// ELEM: every tile element by element (rows off 16 bytes).  Otherwise the tiles
+// ELEM: every tile element by element (rows off 16 bytes), ELEM columns a lane.  Otherwise the tiles
 // whose bases lie off 16 bytes are, with as many loads in flight as cost the
 // vector walk no registers (with 16, R-MAT s21 x 256 FP32 3.94 -> 4.26 ms; in BF16
 // a second copy of the walk costs it as much: 2.10 -> 2.22 ms; with MET, uniform
 // 60,000 x 16 FP32 on 20 x 20 tiles 90 -> 96 us).
-template <typename ST, bool GROUP, bool SUB, bool ELEM, bool MET = false>
+template <typename ST, bool GROUP, bool SUB, int ELEM, bool MET = false>
 __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
     k_spmm(SpGridView A, DGridView B, DGridView C, int tjn, int64_t n_items, int npanels, int R, int64_t ngroups,
            int row_align_ok, int panel_major, const uint8_t* __restrict__ long_flag, bool all_long,
            MetRows met, unsigned long long* __restrict__ next_item) {
-  constexpr int PW = 32 * Vec<ST>::N;
+  constexpr int PW = 32 * (ELEM ? ELEM : Vec<ST>::N);
   const int lane = lane_id();
   unsigned long long it = 0;
   if (lane == 0) it = atomicAdd(next_item, 1ULL);
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
       }
       unsigned left;
       if (ELEM)
-        left = spmm_rows<ST, GROUP, SUB, 16 / Vec<ST>::N, MET>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag, bound);
+        left = spmm_rows<ST, GROUP, SUB, 16 / (ELEM ? ELEM : 1), MET, ELEM ? ELEM : 1>(A, B, C, ti, tj, r0, R, c0, W, false, long_flag, bound);
       else if (sizeof(ST) == 2 || MET)
         left = spmm_rows<ST, GROUP, SUB, 0, MET>(A, B, C, ti, tj, r0, R, c0, W, aligned,
                                                  aligned || all_long ? long_flag : nullptr, bound, ahead);
@@ -1054,9 +1054,10 @@ __device__ __forceinline__ void chain_apply(const uint32_t* sw, const float* sv,
 // applied from its buffer, batches b + 1 and b + 2 are in flight.  One barrier
 // per batch: past it batch b has landed (each producer waited for its own
 // copies) and batch b - 1, whose buffer batch b + 2 overwrites, has been
-// applied.  At most 32 stages.  Buffers: slices of `stride` words, then the
+// applied.  MANY: more than 32 stages, 32 at a time (the loop's registers cost the
+// others 1 %).  Buffers: slices of `stride` words, then the
 // values.
-template <typename ST, bool SUB>
+template <typename ST, bool SUB, bool MANY>
 __device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int stride, const SpGridView& A,
                                           const DGridView& B, const DGridView& C, int64_t ti, int64_t tj, int64_t r,
                                           int c0, int W, int unit) {
@@ -1066,121 +1067,128 @@ __device__ __forceinline__ void chain_row(uint32_t* slices, float* vals, int str
   const int nw = (W * (int)sizeof(ST) + 3) >> 2;
   constexpr int each = kChainEach, batch = each * (kChainWarps - 1);
   ST* __restrict__ crow = reinterpret_cast<ST*>(C.tile(ti, tj)) + r * C.ld + c0;
-  const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, lane, true);
-  const int32_t aincl = warp_inclusive_scan(sl.alen);
-  const int32_t atot = __shfl_sync(kFull, aincl, 31);
-  const int32_t aexcl = aincl - sl.alen;
-  const int32_t nb = (atot + batch - 1) / batch;
+  // the lane's columns 2 lane and 2 lane + 1 (BF16) or lane (FP32)
+  float acc[CN];
   if (prod < 0) {
-    // the lane's columns 2 lane and 2 lane + 1 (BF16) or lane (FP32)
-    float acc[CN];
 #pragma unroll
     for (int x = 0; x < CN; x++) acc[x] = lane < nw && lane * CN + x < W ? Vec<ST>::to_f(crow[lane * CN + x]) : 0.f;
-    for (int32_t b = 0; b < nb; b++) {
-      __syncthreads();
-      const int n = min(batch, atot - b * batch);
-      const int base = (b % kChainBuffers) * batch;
-      const uint32_t* sw = slices + base * stride + lane;
-      const float* sv = vals + base;
-      if (stride == 4) chain_apply<ST, 4>(sw, sv, n, acc);
-      else if (stride == 8) chain_apply<ST, 8>(sw, sv, n, acc);
-      else if (stride == 16) chain_apply<ST, 16>(sw, sv, n, acc);
-      else chain_apply<ST, 32>(sw, sv, n, acc);
+  }
+  for (int g0 = 0; g0 == 0 || (MANY && g0 < (int)A.gn); g0 += 32) {  // the stages, a lane each
+    const StageLane<ST> sl = stage_lane<ST, SUB>(A, B, ti, tj, r, g0 + lane, true);
+    const int32_t aincl = warp_inclusive_scan(sl.alen);
+    const int32_t atot = __shfl_sync(kFull, aincl, 31);
+    if (MANY && atot == 0) continue;  // (the same for every warp)
+    const int32_t aexcl = aincl - sl.alen;
+    const int32_t nb = (atot + batch - 1) / batch;
+    if (prod < 0) {
+      for (int32_t b = 0; b < nb; b++) {
+        __syncthreads();
+        const int n = min(batch, atot - b * batch);
+        const int base = (b % kChainBuffers) * batch;
+        const uint32_t* sw = slices + base * stride + lane;
+        const float* sv = vals + base;
+        if (stride == 4) chain_apply<ST, 4>(sw, sv, n, acc);
+        else if (stride == 8) chain_apply<ST, 8>(sw, sv, n, acc);
+        else if (stride == 16) chain_apply<ST, 16>(sw, sv, n, acc);
+        else chain_apply<ST, 32>(sw, sv, n, acc);
+      }
+    } else {
+      const int n_unit = W * (int)sizeof(ST) / unit;  // copies per slice
+      const int trips = (each * n_unit + 31) >> 5;
+      const int u_first = lane / n_unit, q_first = lane - u_first * n_unit;
+      const int u_step = 32 / n_unit, q_step = 32 - u_step * n_unit;
+      int32_t nc = 0;  // the pending A entry: its column, value and B tile
+      float nv = 0.f;
+      const ST* nbt = nullptr;
+      auto fetch = [&](int32_t x) {
+        if (x >= nb) return;
+        const int32_t e = x * batch + prod * each + lane;
+        const int src = min(warp_search_lanes(aincl, e), 31);
+        const int32_t off = e - __shfl_sync(kFull, aexcl, src);
+        const int32_t* sacol = reinterpret_cast<const int32_t*>(
+            __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
+        const float* saval = reinterpret_cast<const float*>(
+            __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
+        nbt = reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), src));
+        if (lane < each && e < atot) {
+          nc = __ldg(sacol + off);
+          nv = __ldg(saval + off);
+        }
+      };
+      auto issue = [&](int32_t x) {  // batch x: its A entries are in nc, nv, nbt
+        if (x < nb) {
+          const int base = (x % kChainBuffers) * batch + prod * each;
+          const int left = min(each, atot - x * batch - prod * each);  // entries of this warp (or none)
+          const unsigned long long addr = reinterpret_cast<unsigned long long>(nbt + (int64_t)nc * B.ld + c0);
+          if (lane < each) vals[base + lane] = nv;
+          char* to = reinterpret_cast<char*>(slices + base * stride);
+          int u = u_first, q = q_first;
+          auto next = [&]() {
+            u += u_step;
+            q += q_step;
+            if (q >= n_unit) {
+              q -= n_unit;
+              u++;
+            }
+          };
+          if (left <= 0) {
+          } else if (unit != 2) {
+#pragma unroll 4
+            for (int i = 0; i < trips; i++) {
+              const char* from = reinterpret_cast<const char*>(__shfl_sync(kFull, addr, u & 31)) + q * unit;
+              char* dst = to + u * stride * 4 + q * unit;
+              if (u < left) {
+                if (unit == 16) cp_async16_nb(dst, from);
+                else cp_async4_nb(dst, from);
+              }
+              next();
+            }
+          } else {  // no asynchronous copy of 2 bytes: eight loads in flight
+            for (int i0 = 0; i0 < trips; i0 += 8) {
+              uint16_t h[8];
+              int at[8];
+#pragma unroll
+              for (int k = 0; k < 8; k++) {
+                const uint16_t* from = reinterpret_cast<const uint16_t*>(__shfl_sync(kFull, addr, u & 31)) + q;
+                at[k] = u < left ? u * stride * 2 + q : -1;
+                if (at[k] >= 0) h[k] = __ldg(from);
+                next();
+              }
+#pragma unroll
+              for (int k = 0; k < 8; k++)
+                if (at[k] >= 0) reinterpret_cast<uint16_t*>(to)[at[k]] = h[k];
+            }
+          }
+        }
+        cp_async_commit();
+      };
+      fetch(0);
+      issue(0);
+      fetch(1);
+      issue(1);
+      fetch(2);
+      for (int32_t b = 0; b < nb; b++) {
+        cp_async_wait_group<1>();  // this warp's part of batch b has landed
+        __syncthreads();
+        issue(b + 2);
+        fetch(b + 3);
+      }
+      cp_async_wait_all();
     }
+    __syncthreads();  // the buffers are free again
+  }
+  if (prod < 0) {
 #pragma unroll
     for (int x = 0; x < CN; x++)
       if (lane < nw && lane * CN + x < W) crow[lane * CN + x] = Vec<ST>::from_f(acc[x]);
-  } else {
-    const int n_unit = W * (int)sizeof(ST) / unit;  // copies per slice
-    const int trips = (each * n_unit + 31) >> 5;
-    const int u_first = lane / n_unit, q_first = lane - u_first * n_unit;
-    const int u_step = 32 / n_unit, q_step = 32 - u_step * n_unit;
-    int32_t nc = 0;  // the pending A entry: its column, value and B tile
-    float nv = 0.f;
-    const ST* nbt = nullptr;
-    auto fetch = [&](int32_t x) {
-      if (x >= nb) return;
-      const int32_t e = x * batch + prod * each + lane;
-      const int src = min(warp_search_lanes(aincl, e), 31);
-      const int32_t off = e - __shfl_sync(kFull, aexcl, src);
-      const int32_t* sacol = reinterpret_cast<const int32_t*>(
-          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.acol), src));
-      const float* saval = reinterpret_cast<const float*>(
-          __shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.aval), src));
-      nbt = reinterpret_cast<const ST*>(__shfl_sync(kFull, reinterpret_cast<unsigned long long>(sl.bt), src));
-      if (lane < each && e < atot) {
-        nc = __ldg(sacol + off);
-        nv = __ldg(saval + off);
-      }
-    };
-    auto issue = [&](int32_t x) {  // batch x: its A entries are in nc, nv, nbt
-      if (x < nb) {
-        const int base = (x % kChainBuffers) * batch + prod * each;
-        const int left = min(each, atot - x * batch - prod * each);  // entries of this warp (or none)
-        const unsigned long long addr = reinterpret_cast<unsigned long long>(nbt + (int64_t)nc * B.ld + c0);
-        if (lane < each) vals[base + lane] = nv;
-        char* to = reinterpret_cast<char*>(slices + base * stride);
-        int u = u_first, q = q_first;
-        auto next = [&]() {
-          u += u_step;
-          q += q_step;
-          if (q >= n_unit) {
-            q -= n_unit;
-            u++;
-          }
-        };
-        if (left <= 0) {
-        } else if (unit != 2) {
-#pragma unroll 4
-          for (int i = 0; i < trips; i++) {
-            const char* from = reinterpret_cast<const char*>(__shfl_sync(kFull, addr, u & 31)) + q * unit;
-            char* dst = to + u * stride * 4 + q * unit;
-            if (u < left) {
-              if (unit == 16) cp_async16_nb(dst, from);
-              else cp_async4_nb(dst, from);
-            }
-            next();
-          }
-        } else {  // no asynchronous copy of 2 bytes: eight loads in flight
-          for (int i0 = 0; i0 < trips; i0 += 8) {
-            uint16_t h[8];
-            int at[8];
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-              const uint16_t* from = reinterpret_cast<const uint16_t*>(__shfl_sync(kFull, addr, u & 31)) + q;
-              at[k] = u < left ? u * stride * 2 + q : -1;
-              if (at[k] >= 0) h[k] = __ldg(from);
-              next();
-            }
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-              if (at[k] >= 0) reinterpret_cast<uint16_t*>(to)[at[k]] = h[k];
-          }
-        }
-      }
-      cp_async_commit();
-    };
-    fetch(0);
-    issue(0);
-    fetch(1);
-    issue(1);
-    fetch(2);
-    for (int32_t b = 0; b < nb; b++) {
-      cp_async_wait_group<1>();  // this warp's part of batch b has landed
-      __syncthreads();
-      issue(b + 2);
-      fetch(b + 3);
-    }
-    cp_async_wait_all();
   }
-  __syncthreads();  // the buffers are free again
 }
 
 // Long rows of tile columns [tj0, tj0 + tjn), a block per (row, tile column,
 // panel).  `met`: list[0, count[0]) holds the rows that k_spmm_narrow met (its
 // programmatic dependent: it waits for it);
 // otherwise the rows k_spmm_find_long listed, and k_spmm_narrow may start.
-template <typename ST, bool SUB>
+template <typename ST, bool SUB, bool MANY>
 __global__ void __launch_bounds__(kChainWarps * 32, 2)
     k_spmm_chain(SpGridView A, DGridView B, DGridView C, int tj0, int tjn, int npanels, int stride, bool met,
                  const int64_t* __restrict__ list, const int32_t* __restrict__ count,
@@ -1219,7 +1227,7 @@ __global__ void __launch_bounds__(kChainWarps * 32, 2)
     if (threadIdx.x == 0) take(slot ^ 1);
     if (c0 < W) {
       const int unit = tile_on<ST, 16>(B, C, ti, tj, W) ? 16 : (tile_on<ST, 4>(B, C, ti, tj, W) ? 4 : 2);
-      chain_row<ST, SUB>(slices, vals, stride, A, B, C, ti, tj, x - ti * A.tm, c0, min(PW, W - c0), unit);
+      chain_row<ST, SUB, MANY>(slices, vals, stride, A, B, C, ti, tj, x - ti * A.tm, c0, min(PW, W - c0), unit);
     } else {
       __syncthreads();  // (chain_row ends with a barrier)
     }
@@ -1401,10 +1409,10 @@ static int launch_wide(Context* ctx, const SpGridView& A, const DGridView& B, co
   const uint8_t* lflag = flag;
   const int pmajor = (int)tuning(ctx, BCLX_TUNE_SPMM_PANEL_MAJOR);
   if (R > 1)
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB, false>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, true, SUB, 0>, A, B, C, tjn, n_items, npanels, R, ngroups, align_ok, pmajor, lflag,
                                false, MetRows{}, ctr));
   else
-    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB, false>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
+    BCLX_CK(cudaLaunchKernelEx(&cfg, k_spmm<ST, false, SUB, 0>, A, B, C, tjn, n_items, npanels, 1, ngroups, align_ok, pmajor, lflag,
                                false, MetRows{}, ctr));
   note_launch();
   BCLX_CK_LAUNCH();
@@ -1455,8 +1463,9 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   while (stride < kChainPanelWords && stride * 4 < width * (int64_t)sizeof(ST)) stride *= 2;
   const size_t smem = chain_bytes(stride);
   const int64_t arows = A.gm * A.tm;
-  const bool chains = A.gn <= 32;  // one lane per stage
-  const bool listed = chains && arows >= spmm_long_min_rows();
+  // (the kernels of short rows tell a long row by its first 32 stages at most, or by its flag, which k_spmm reads)
+  const bool listed = arows >= spmm_long_min_rows() && (A.gn <= 32 || wide_rows);
+  const bool chains = A.gn <= 32 || listed;
   int long_row = (int)tuning(ctx, BCLX_TUNE_SPMM_LONG_ROW);
   const bool few = chains && !listed && long_row <= 0;
   if (long_row <= 0) long_row = std::min(kNarrowLongSteps * L, listed && wide_rows ? 512 : INT_MAX);
@@ -1494,12 +1503,16 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
   // well (by 16-byte vectors where the rows lie on 16 bytes): R-MAT of 400,000 on 20 x
   // 20 tiles, x 16 FP32 488 and 410 us (k_spmm with its own long rows, as launch_wide
   // runs it: 640), x 64 572 and 495 (650), x 64 BF16 649 and 479 (798), x 17 FP32 577
-  // and 447, x 47 597 and 556; uniform 20,000 x 64 BF16 49 and 43; with 40 tiles along k
-  // (no chains) uniform 400,000 x 64 BF16 739 and 589, x 201 FP32 1814 and 1270.  Rows of
-  // fewer units stay with k_spmm_narrow: R-MAT of 100,000 x 47 177 and 250.
+  // and 420, x 47 597 and 528; uniform 20,000 x 64 BF16 49 and 43; on 33 x 33 tiles, where
+  // k_spmm_narrow had no chains, R-MAT of 400,000 x 16 FP32 1865 and 502, x 47 2469 and 627,
+  // x 64 BF16 3306 and 575.  Rows of fewer units stay with k_spmm_narrow: R-MAT of
+  // 100,000 x 47 177 and 250.
   auto wide = [&]() {
-    const int wp = (int)ceil_div(width, 32 * Vec<ST>::N);
-    const int R = spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
+    constexpr int VN = Vec<ST>::N;
+    // rows of 64 columns and fewer (here for the stages' sake): two columns a lane, eight entries' loads in flight
+    const bool two = U != 16 && width <= 64;
+    const int wp = (int)ceil_div(width, 32 * (two ? 2 : VN));
+    const int R = two ? 1 : spmm_rows_per_item(ctx, C, tjn, A.gn, wp);
     const int64_t groups = ceil_div(C.tm, (int64_t)R), items = C.gm * tjn * groups * wp;
     const int64_t blocks = std::min(ceil_div(items, kSpmmWarps), (int64_t)ctx->num_sms * 4);
     const uint8_t* skip = flag;
@@ -1508,15 +1521,16 @@ static int launch_narrow_nv(Context* ctx, const SpGridView& A, const DGridView& 
                           0, skip, true, met, ctr);
     };
     if constexpr (U == 16) {  // (only for 17 and more tiles along k: R is 1)
-      return met.list ? go(k_spmm<ST, false, SUB, false, true>) : go(k_spmm<ST, false, SUB, false>);
+      return met.list ? go(k_spmm<ST, false, SUB, 0, true>) : go(k_spmm<ST, false, SUB, 0>);
     } else {
-      if (met.list) return R > 1 ? go(k_spmm<ST, true, SUB, true, true>) : go(k_spmm<ST, false, SUB, true, true>);
-      return R > 1 ? go(k_spmm<ST, true, SUB, true>) : go(k_spmm<ST, false, SUB, true>);
+      if (two) return met.list ? go(k_spmm<ST, false, SUB, 2, true>) : go(k_spmm<ST, false, SUB, 2>);
+      if (met.list) return R > 1 ? go(k_spmm<ST, true, SUB, VN, true>) : go(k_spmm<ST, false, SUB, VN, true>);
+      return R > 1 ? go(k_spmm<ST, true, SUB, VN>) : go(k_spmm<ST, false, SUB, VN>);
     }
   };
   if (!listed) BCLX_TRY(wide_rows ? wide() : narrow());
   if (chains) {
-    auto kern = k_spmm_chain<ST, SUB>;
+    auto kern = A.gn <= 32 ? k_spmm_chain<ST, SUB, false> : k_spmm_chain<ST, SUB, true>;
     BCLX_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // one block per SM beside k_spmm_narrow, two where it has finished
     const int64_t blocks = std::min<int64_t>(arows * tjn, (int64_t)ctx->num_sms * (listed ? 1 : 2));
