@@ -1956,6 +1956,7 @@ struct bclx_spgemm_plan_s {
   Geom g{};
   int dtype = BCLX_F32;
   int64_t products = 0, nnz = 0, n_light = 0, n_heavy = 0, n_vheavy = 0, n_heavy_items = 0;
+  bool has_vheavy = false;  // rows above kVeryHeavyUb, or n_vheavy > 0 (see numeric_grab)
   int64_t hbm_words = 0;
   int32_t* light_list = nullptr;
   int32_t* heavy_list = nullptr;   // very heavy rows first, then the other heavy rows
@@ -2168,7 +2169,7 @@ static int launch_symbolic(Context* ctx, const SpGridView& A, const SpGridView& 
 // stencil, 10.4M items of 143 products: 24.4 ms with 1, 22.3 with 4, 21.9 with 8
 // and with 16: the counter is one address).
 static int numeric_grab(Context* ctx, const bclx_spgemm_plan_s* P, int64_t n_total) {
-  return P->n_vheavy > 0 ? 1 : queue_grab(ctx, n_total, kWarpsNum, 4, 8);
+  return P->has_vheavy ? 1 : queue_grab(ctx, n_total, kWarpsNum, 4, 8);
 }
 
 template <typename VT, int WORDS, bool LEARNED = false, int VCAP = kVcap, bool SPLIT = false>
@@ -2412,6 +2413,7 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
   // product waits for (numeric pass, graph of 10,000 x sparse features 125 -> 70
   // us, of 3,000 147 -> 86, R-MAT of 5,000 rows squared 166 -> 121)
   P->n_vheavy = cnts[3] + (cnts[3] + n_mid <= ctx->num_sms ? n_mid : 0);
+  P->has_vheavy = P->n_vheavy > 0;
   P->n_heavy = cnts[1] + cnts[3] + n_mid;
   P->products = ctx->pinned[2];
   int64_t* sums_h = nullptr;
@@ -2904,6 +2906,7 @@ static int noalloc_product(Context* ctx, ScratchArena& ar, const bclx_csr_t* a, 
   P.repeats = cnts[5] != 0;
   P.n_light = cnts[0];
   P.n_vheavy = cnts[3];
+  P.has_vheavy = cnts[3] > 0;
   P.n_heavy = cnts[1] + cnts[3];
   if (P.n_vheavy > 0)
     BCLX_CK(cudaMemcpyAsync(P.heavy_list, P.vheavy_list, sizeof(int32_t) * P.n_vheavy, cudaMemcpyDeviceToDevice,
@@ -3077,7 +3080,8 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
   BCLX_CK(cudaMemcpyAsync(&prod, P->products_dev, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
   BCLX_CK(cudaStreamSynchronize(ctx->stream));
   P->n_light = cnts[0];
-  P->n_vheavy = 0;  // the learned cut treats every heavy row alike
+  P->n_vheavy = 0;  // the learned cut treats every heavy row alike,
+  P->has_vheavy = cnts[3] > 0;  // the numeric pass takes its items one by one where there are such rows
   P->n_heavy = cnts[1] + cnts[3];
   P->products = prod;
   P->repeats = cnts[5] != 0;
@@ -3198,6 +3202,7 @@ static int learned_impl(Context* ctx, const SpGridView& A, const SpGridView& B, 
     R->blocks_per_sm = P->blocks_per_sm;
     R->long_seg = P->long_seg;
     R->repeats = P->repeats;
+    R->has_vheavy = P->has_vheavy;
     R->heavy_list = P->failed_list;  // borrowed
     R->light_list = P->light_list;   // borrowed (unused: no light rows)
     R->n_light = 0;
