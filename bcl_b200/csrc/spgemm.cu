@@ -208,13 +208,20 @@ __device__ __forceinline__ P* shfl_ptr(P* p, int src) {
 }
 
 // Shared-memory table of one warp's walk: the non-empty entries of a chunk.
-template <typename VT>
+// COMPACT: no value addresses; a value lies as far from its column as the
+// tile's arrays from each other, which the stage's lane knows (two shuffles a
+// batch).  For tiles of more than 8192 columns: with the whole table three blocks
+// need more than 196 KB of an SM, and the next split leaves 28 KB of L1 for 60
+// (R-MAT s18 39.7 -> 39.2 ms; s20 on 64 x 64 tiles, whose B rows have no table and are
+// searched, 642 -> 592, learned in blocks of 8 tile rows 1.91 -> 1.66 s).
+template <typename VT, bool COMPACT>
 struct WalkTable {
-  ulonglong2 seg[32];  // column and value addresses of the entry's segment (packed: of product 0 of the chunk,
-                       // as this segment continues them)
+  // column (and value) address of the entry's segment (packed: of product 0 of the chunk, as this segment
+  // continues them)
+  std::conditional_t<COMPACT, unsigned long long, ulonglong2> seg[32];
   struct {
     VT a;
-    uint32_t len_stage;  // segment length << 8 | stage
+    uint32_t len_stage;  // segment length << 13 | lane of the stage << 8 | stage
   } av[32];
 };
 
@@ -246,10 +253,10 @@ struct WalkTable {
 // product belongs to is the number of entries that begin at or before it: each
 // entry sets the bit of its first product in the batch, the bits are or-ed
 // over the warp, and a population count gives the entry.
-template <typename VT, typename F, typename FD>
+template <typename VT, bool COMPACT, typename F, typename FD>
 __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridView& B, const Geom& g,
                                               const RowInfo& x, int s0, int s1, bool ranged, int fb_lo, int fb_hi,
-                                              const int32_t* __restrict__ tab, int long_seg, WalkTable<VT>& tbl,
+                                              const int32_t* __restrict__ tab, int long_seg, WalkTable<VT, COMPACT>& tbl,
                                               F&& f, FD&& fd) {
   const int lane = lane_id();
   const unsigned below = (1u << lane) - 1u, upto = below | (1u << lane);
@@ -273,6 +280,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
     const int32_t* bptr = nullptr;
     const int32_t* bci = nullptr;
     const VT* bva = nullptr;
+    long long apart = 0;  // COMPACT: the values' distance from the columns
     if (si < w1) {
       kk = stage_at(g, x.ti, x.tj, si);
       const int64_t k = stage_k(g, kk, x.rot);
@@ -285,6 +293,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       bptr = table ? tab + (k * g.gn + x.tj) * g.tk * (g.nfb + 1) : Bt.row_ptr;
       bci = Bt.col_ind;
       bva = reinterpret_cast<const VT*>(Bt.vals);
+      apart = reinterpret_cast<long long>(bva) - reinterpret_cast<long long>(bci);
     }
     const int32_t aincl = warp_inclusive_scan(alen);
     const int32_t atot = __reduce_add_sync(kFull, alen);
@@ -298,7 +307,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       const VT* saval = shfl_ptr(aval, sl);
       const int32_t* sbptr = shfl_ptr(bptr, sl);
       const int32_t* sbci = shfl_ptr(bci, sl);
-      const VT* sbva = shfl_ptr(bva, sl);
+      const VT* sbva = COMPACT ? nullptr : shfl_ptr(bva, sl);
       const int stage = __shfl_sync(kFull, kk, sl);
       int32_t len = 0, bs = 0;
       VT av = VT(0);
@@ -324,16 +333,35 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
       if (packed) excl = warp_inclusive_scan(len) - len;
       if (len > 0) {
         const int at = __popc(full & below);
-        tbl.seg[at] = make_ulonglong2(reinterpret_cast<unsigned long long>(sbci + bs) - 4ull * (unsigned)excl,
-                                      reinterpret_cast<unsigned long long>(sbva + bs) - 4ull * (unsigned)excl);
+        const unsigned long long col = reinterpret_cast<unsigned long long>(sbci + bs) - 4ull * (unsigned)excl;
+        if constexpr (COMPACT)
+          tbl.seg[at] = col;
+        else
+          tbl.seg[at] = make_ulonglong2(col, reinterpret_cast<unsigned long long>(sbva + bs) - 4ull * (unsigned)excl);
         tbl.av[at].a = av;
-        tbl.av[at].len_stage = (uint32_t)len << 8 | (uint32_t)stage;
+        // (the length is read entry by entry alone, where it is at most a tile's width)
+        tbl.av[at].len_stage = (uint32_t)len << 13 | (uint32_t)sl << 8 | (uint32_t)stage;
       }
       __syncwarp();
       // (straight-line loads: lanes past the end repeat the last product)
       int32_t nj;
       VT na, nb;
       uint32_t nls;
+      auto load = [&](int entry, uint32_t q) {
+        na = tbl.av[entry].a;
+        nls = tbl.av[entry].len_stage;
+        unsigned long long col, val;
+        if constexpr (COMPACT) {
+          col = tbl.seg[entry] + 4ull * q;
+          val = col + (unsigned long long)__shfl_sync(kFull, apart, (int)(nls >> 8 & 31u));
+        } else {
+          const ulonglong2 sg = tbl.seg[entry];
+          col = sg.x + 4ull * q;
+          val = sg.y + 4ull * q;
+        }
+        nj = __ldg(reinterpret_cast<const int32_t*>(col));
+        nb = __ldg(reinterpret_cast<const VT*>(val));
+      };
       if (packed) {
         const int32_t begins = len > 0 ? excl : INT_MAX;  // this entry's first product
         int ahead = -1;                                   // entries begun before the batch, less one
@@ -344,12 +372,7 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
           heads = __reduce_or_sync(kFull, bit_or_none(begins - base));
           const int src = ahead + __popc(heads & upto);
           ahead += __popc(heads);
-          const uint32_t q = min((uint32_t)(base + lane), end);
-          const ulonglong2 sg = tbl.seg[src];
-          na = tbl.av[src].a;
-          nls = tbl.av[src].len_stage;
-          nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * q));
-          nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * q));
+          load(src, min((uint32_t)(base + lane), end));
         };
         fetch(0);
         for (int32_t base = 0; base < total; base += 32) {
@@ -365,21 +388,16 @@ __device__ __forceinline__ void walk_products(const SpGridView& A, const SpGridV
         int ent = 0;
         uint32_t off = 0;  // the step's first product in its segment
         auto fetch = [&]() {
-          const ulonglong2 sg = tbl.seg[ent];
-          na = tbl.av[ent].a;
-          nls = tbl.av[ent].len_stage;
-          const uint32_t q = min(off + (uint32_t)lane, (nls >> 8) - 1u);
-          nj = __ldg(reinterpret_cast<const int32_t*>(sg.x + 4ull * q));
-          nb = __ldg(reinterpret_cast<const VT*>(sg.y + 4ull * q));
+          load(ent, min(off + (uint32_t)lane, (tbl.av[ent].len_stage >> 13) - 1u));
         };
         fetch();
         for (int i = 0; i < steps; i++) {
           const int32_t j = nj;
           const VT a = na, b = nb;
           const int st = (int)(nls & 255u);
-          const bool on = off + (uint32_t)lane < (nls >> 8);
+          const bool on = off + (uint32_t)lane < (nls >> 13);
           off += 32;
-          if (off >= (nls >> 8)) {
+          if (off >= (nls >> 13)) {
             off = 0;
             ent++;
           }
@@ -1392,8 +1410,10 @@ struct WarpSmem {
   alignas(16) VT acc[VCAP];
   alignas(16) VT part[VCAP];
   alignas(16) unsigned char tag[VCAP];
-  WalkTable<VT> walk;
+  WalkTable<VT, (WORDS > 256)> walk;
 };
+static_assert(3 * (sizeof(WarpSmem<float, kMaxWords, kVcap>) * kWarpsNum + 1024) <= 196 * 1024,
+              "three blocks of the widest tiles, in the shared-memory split that leaves 60 KB of L1");
 
 // Items whose stages run as work items of their own, on warps of their own:
 // a column's stage partials are independent chains, added in stage order
@@ -1675,7 +1695,7 @@ __global__ void __launch_bounds__(kWarpsNum * 32, BCLX_NUMERIC_MIN_BLOCKS)
     // An item that holds all of its row's outputs takes every product of the
     // row: the B rows' own bounds serve, without the table or a search.
     const bool ranged = heavy && (LEARNED ? (fb_lo > 0 || fb_hi * kFineCols < x.w) : !whole);
-    walk_products<VT>(A, B, g, x, s0, s1, ranged, fb_lo, fb_hi, tab, long_seg, S.walk, update, update_direct);
+    walk_products<VT, (WORDS > 256)>(A, B, g, x, s0, s1, ranged, fb_lo, fb_hi, tab, long_seg, S.walk, update, update_direct);
 
     // 5. last fold and values out
     if (part_only) {
