@@ -28,11 +28,11 @@ import torch
 
 SPGEMM_LIGHT_UB = (128, 256, 512)
 CANDIDATES = {
-    "grab": (1, 2, 4, 8),
+    "grab": (0, 1, 2, 4, 8),  # 0: by the product
     "blocks_per_sm": (3, 4),
     "long_seg": (6, 14, 28, 1 << 30),
 }
-DEFAULT = (1, 4, 14)
+DEFAULT = (0, 4, 14)  # a plan's own (grab, blocks_per_sm, long_seg)
 SPMM_CANDIDATES = {
     "spmm_rows": (0, 1, 2, 4),
     "spmm_long_row": (0, 512, 1024, 2048),

@@ -646,8 +646,8 @@ def spgemm(a: SPMatrix, b: SPMatrix, stages: str = "fused", keep_plan: bool = Fa
     (all G*G tile products of that stage), adding into C between them;
     ``"batched_graph"`` does the same through a CUDA graph kept by the plan.
     All forms are bit-identical.  ``tuning`` = (grab, blocks_per_sm,
-    long_seg), a dict of those and "light_ub", or "auto" for the autotuner's
-    cached choice."""
+    long_seg), a dict of any of those and "light_ub" (the others keep their
+    defaults), or "auto" for the autotuner's cached choice."""
     params = None
     if tuning == "auto":
         from . import autotune
@@ -663,7 +663,8 @@ def spgemm(a: SPMatrix, b: SPMatrix, stages: str = "fused", keep_plan: bool = Fa
     else:
         plan, out, trp, toff, nnz = spgemm_symbolic(a, b)
     if params:
-        plan.tune(params.get("grab", 1), params.get("blocks_per_sm", 4), params.get("long_seg", 14))
+        from . import autotune
+        plan.tune(*(params.get(k, d) for k, d in zip(("grab", "blocks_per_sm", "long_seg"), autotune.DEFAULT)))
     td = a.tile_row_ptr.device
     ci = torch.empty(max(nnz, 1), dtype=torch.int32, device=td)
     v = torch.empty(max(nnz, 1), dtype=_TORCH_OF[_NP_TO_DT[a.dtype]], device=td)

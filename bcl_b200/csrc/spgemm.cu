@@ -2005,7 +2005,7 @@ struct bclx_spgemm_plan_s {
   SplitItems split;               // the very heavy rows' items, where there are few (split_block)
   void* split_block = nullptr;
   // numeric tuning (bclx_spgemm_plan_tune)
-  int grab = 0, blocks_per_sm = 4, long_seg = kLongSegDefault;  // (grab 0: see numeric_grab)
+  int grab = 0, blocks_per_sm = 4, long_seg = kLongSegDefault;  // (grab 0: numeric_grab)
   int light_ub_max = kLightUb;         // light-row class bound (products), set at symbolic time
   int vcap = kVcap;                    // outputs per heavy item (512 or 1024), set at symbolic time
   // CUDA graph of the staged numeric pass (bclx_spgemm_numeric_staged)
@@ -2656,7 +2656,7 @@ int bclx_spgemm_plan_stats(bclx_spgemm_plan_t P, int64_t* out6) {
 }
 
 int bclx_spgemm_plan_tune(bclx_spgemm_plan_t P, int32_t grab, int32_t blocks_per_sm, int32_t long_seg) {
-  if (!P || grab < 1 || grab > 64 || blocks_per_sm < 1 || blocks_per_sm > 4 || long_seg < 1)
+  if (!P || grab < 0 || grab > 64 || blocks_per_sm < 1 || blocks_per_sm > 4 || long_seg < 1)
     return BCLX_ERR_INVALID;
   P->grab = grab;
   P->blocks_per_sm = blocks_per_sm;

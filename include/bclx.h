@@ -217,7 +217,8 @@ BCLX_API int bclx_spgemm_symbolic_sub(bclx_context_t ctx, const bclx_spgrid_t* a
 BCLX_API int bclx_spgemm_numeric_staged(bclx_context_t ctx, bclx_spgemm_plan_t plan, const bclx_spgrid_t* a,
                                         const bclx_spgrid_t* b, bclx_spgrid_out_t* c, int32_t use_graph);
 /* Numeric-pass tuning of a plan: grab = work items a warp takes from the
- * device work queue at a time (1..64), blocks_per_sm (1..4), long_seg = FP32
+ * device work queue at a time (1..64, or 0, the default: by the product),
+ * blocks_per_sm (1..4), long_seg = FP32
  * B segments of at least this many products (on average over 32 A entries) are
  * walked one after another, shorter ones packed together.  Chosen
  * by the autotuner (bcl_b200/autotune.py); no reference counterpart. */
