@@ -12,8 +12,9 @@ heavy item.
 
 Every candidate is timed with CUDA events on the actual product, best of a
 few runs.  Results are cached in a JSON file keyed by a signature of the
-product (value type, tile shapes, grids, nonzeros rounded to powers of two),
-so a later product of the same kind reuses the choice without tuning.  No
+product (value type, tile shapes, grids, nonzeros rounded to powers of two)
+and the version of the knobs, so a later product of the same kind reuses the
+choice without tuning, and a choice made for other kernels is not used.  No
 knob changes a result: every choice gives the same bits.
 """
 from __future__ import annotations
@@ -41,6 +42,9 @@ SPMM_CANDIDATES = {
     "spmm_panel_major": (0, 1),
 }
 LEARN_TARGETS = (256, 320, 384)
+# Counted up when a knob's meaning or the kernels it was measured on change:
+# 2: long_seg became the mean over 32 A entries, the SpMM long-row kernels new.
+VERSION = 2
 
 
 def cache_path() -> str:
@@ -72,9 +76,9 @@ def _p2(x):
 def signature(a, b, kind: str = "spgemm") -> str:
     """Product signature from what is known before any launch."""
     if kind == "spmm":
-        return (f"spmm|{b.torch_dtype}|t{a.tm}x{a.tn}x{b.tn}|g{a.gm}x{a.gn}x{b.gn}|m{_p2(a.m)}|n{_p2(b.n)}"
+        return (f"v{VERSION}|spmm|{b.torch_dtype}|t{a.tm}x{a.tn}x{b.tn}|g{a.gm}x{a.gn}x{b.gn}|m{_p2(a.m)}|n{_p2(b.n)}"
                 f"|nnz{_p2(a.nnz())}")
-    return (f"{kind}|{a.dtype.str}|t{a.tm}x{a.tn}x{b.tn}|g{a.gm}x{a.gn}x{b.gn}|a{_p2(a.nnz())}"
+    return (f"v{VERSION}|{kind}|{a.dtype.str}|t{a.tm}x{a.tn}x{b.tn}|g{a.gm}x{a.gn}x{b.gn}|a{_p2(a.nnz())}"
             f"|b{_p2(b.nnz())}")
 
 
