@@ -130,9 +130,10 @@ __global__ void __launch_bounds__(256) k_tile_count(int64_t m, int64_t n, const 
   if (__any_sync(kFull, wrong) && lane == 0) atomicExch(bad, 1);
 }
 
-// Local row pointers and tile offsets from the scanned counts E.
-__global__ void k_tile_ptrs(const int64_t* __restrict__ E, int64_t ntiles, int64_t tm, int32_t* __restrict__ trp,
-                            int64_t* __restrict__ toff) {
+// Local row pointers and tile offsets from the scanned counts E (nothing where *bad).
+__global__ void k_tile_ptrs(const int64_t* __restrict__ E, int64_t ntiles, int64_t tm, const int32_t* __restrict__ bad,
+                            int32_t* __restrict__ trp, int64_t* __restrict__ toff) {
+  if (*bad) return;
   const int64_t total = ntiles * (tm + 1);
   for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = x / (tm + 1), lr = x - t * (tm + 1);
@@ -188,9 +189,9 @@ __global__ void k_gather_len(SpGridView g, int32_t* __restrict__ len) {
   }
 }
 
-// (nothing where the entries do not fit an int32 row pointer)
-__global__ void k_rowptr32(const int64_t* __restrict__ off, int64_t m, int32_t* __restrict__ rp) {
-  if (__ldg(off + m) > INT32_MAX) return;
+// (nothing where the entries exceed `most`: an int32 row pointer, or the arrays that the caller gave)
+__global__ void k_rowptr32(const int64_t* __restrict__ off, int64_t m, int64_t most, int32_t* __restrict__ rp) {
+  if (__ldg(off + m) > most) return;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r <= m; r += (int64_t)gridDim.x * blockDim.x)
     rp[r] = (int32_t)off[r];
 }
@@ -373,7 +374,7 @@ int bclx_csr_to_tiles(bclx_context_t c, const bclx_csr_t* a, bclx_spgrid_out_t* 
       BCLX_CK_LAUNCH();
     }
     BCLX_TRY(exclusive_scan_i32_buf(ctx, cnt, E, slots, sums));
-    k_tile_ptrs<<<blocks_for(ctx, slots, 256), 256, 0, ctx->stream>>>(E, ntiles, tm, out->tile_row_ptr,
+    k_tile_ptrs<<<blocks_for(ctx, slots, 256), 256, 0, ctx->stream>>>(E, ntiles, tm, bad, out->tile_row_ptr,
                                                                       out->tile_offset);
     note_launch();
     BCLX_CK_LAUNCH();
@@ -445,7 +446,7 @@ int bclx_tiles_to_csr(bclx_context_t c, const bclx_spgrid_t* g, int32_t* row_ptr
       BCLX_CK_LAUNCH();
     }
     BCLX_TRY(exclusive_scan_i32_buf(ctx, len, off, m, sums));
-    k_rowptr32<<<blocks_for(ctx, m + 1, 256), 256, 0, ctx->stream>>>(off, m, row_ptr);
+    k_rowptr32<<<blocks_for(ctx, m + 1, 256), 256, 0, ctx->stream>>>(off, m, col_ind && vals ? (int64_t)INT32_MAX : 0, row_ptr);
     note_launch();
     BCLX_CK_LAUNCH();
     if (m > 0 && g->n > 0 && col_ind && vals) {
