@@ -294,7 +294,9 @@ class SPMatrix:
         if td.type == "cuda":
             self.desc = torch.empty((ntiles, 7), dtype=torch.int64, device=td)
             # the kernel reads int64 offsets on the tiles' device, one after another
-            toff = self.tile_offset.to(device=td, dtype=torch.int64).contiguous()
+            toff = self.tile_offset
+            if toff.dtype != torch.int64 or toff.device != td or not toff.is_contiguous():
+                toff = toff.to(device=td, dtype=torch.int64).contiguous()
             g = SpGridOut(self.m, self.n, self.tm, self.tn, self.gm, self.gn, self.tile_row_ptr.data_ptr(),
                           toff.data_ptr(), self.col_ind.data_ptr(), self.vals.data_ptr(), _NP_TO_DT[self.dtype], 0)
             call("bclx_spgrid_describe", context(td.index).use_current_stream(), ctypes.byref(g),
