@@ -422,9 +422,19 @@ __device__ __forceinline__ int met_bound(const MetRows& met, const SpGridView& A
   const float nnz = warp_sum(lane_id() < A.gn ? (float)A.tile(ti, lane_id()).nnz : 0.f);
   return min(met.most, max(met.least, (int)min(4.f * nnz / (float)C.rows_of(ti), 1e9f)));
 }
-// Rows x0 + (bits of left), by one lane.
+// Rows x0 + (bits of left), a lane each, or one lane's loop over the bits.  The loop
+// makes k_spmm_narrow spill (50 to 150 bytes), a lane each does not: R-MAT 169,343 x
+// 47 FP32 274 -> 257 us, BF16 of 300,000 x 64 R-MAT 275 -> 255, uniform 114 -> 91.  But
+// FP32 on 16 bytes: R-MAT of 300,000 x 16 207 with the loop, 223 a lane each, x 64 322
+// and 353, of 4,000 x 16 31 and 37 (uniform 300,000 x 16 87 and 81).
+template <bool LOOP>
 __device__ __forceinline__ void list_met(const MetRows& met, int64_t x0, unsigned left) {
-  for (; left; left &= left - 1) met.list[atomicAdd(met.count, 1)] = x0 + __ffs(left) - 1;
+  if (LOOP) {
+    if (lane_id() == 0)
+      for (; left; left &= left - 1) met.list[atomicAdd(met.count, 1)] = x0 + __ffs(left) - 1;
+  } else if ((left >> lane_id()) & 1u) {
+    met.list[atomicAdd(met.count, 1)] = x0 + lane_id();
+  }
 }
 
 // Tile columns [0, tjn) (k_spmm_narrow takes the others).  Warp items come
@@ -494,7 +504,7 @@ __global__ void __launch_bounds__(kSpmmWarps * 32, 4)
       else
         left = spmm_rows<ST, GROUP, SUB, 2, MET>(A, B, C, ti, tj, r0, R, c0, W, false, all_long ? long_flag : nullptr,
                                                  bound);
-      if (MET && left && tj == 0 && panel == 0 && lane == 0) list_met(met, ti * A.tm + r0, left);
+      if (MET && left && tj == 0 && panel == 0) list_met<false>(met, ti * A.tm + r0, left);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
@@ -1269,7 +1279,8 @@ __global__ void __launch_bounds__(kNarrowWarps * 32, NV == 4 ? 3 : 4)
       unsigned left;
       if (on) left = narrow_rows<ST, U, NV, SUB>(A, B, C, ti, tj, r0, L, c0, c1 - c0, long_row);
       else left = elem_rows<ST, SUB>(A, B, C, ti, tj, r0, min(r0 + 32 / L, C.rows_of(ti)), c0, c1, long_row);
-      if (met.list && left && tj == tj0 && panel == 0 && lane == 0) list_met(met, ti * A.tm + r0, left);
+      if (left && met.list && tj == tj0 && panel == 0)
+        list_met<sizeof(ST) == 4 && U == 16>(met, ti * A.tm + r0, left);
     }
     it = __shfl_sync(kFull, nx, 0);
   }
