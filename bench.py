@@ -709,10 +709,11 @@ def spgemm_large_summary(args, wl, stream, block_rows=8):
             fn = (lambda: spgemm_sub(A, A, rows, range(A.gn), form=form, predictor=pred))
             fn()  # warm (and the learned form's statistics)
             if form == "learned":
-                _, pl = spgemm_sub(A, A, rows, range(A.gn), form=form, predictor=pred, keep_plan=True)
+                c, pl = spgemm_sub(A, A, rows, range(A.gn), form=form, predictor=pred, keep_plan=True)
                 for k, v in learned_stats(pl).items():
                     st_sum[k] = st_sum.get(k, 0) + v
                 pl.close()
+                del c  # (beside it the timed call would have to allocate a C of its own)
             torch.cuda.synchronize()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record(stream)
