@@ -1438,8 +1438,8 @@ struct SplitItems {
 #ifndef BCLX_NUMERIC_MIN_BLOCKS
 #define BCLX_NUMERIC_MIN_BLOCKS 4
 #endif
-// Bound by instruction issue (67 % of the slots) and the shared-memory pipe
-// (66 %), not by DRAM: at R-MAT s16 2.3e9 warp instructions, of which an item's
+// Bound by instruction issue (72 % of the slots) and the shared-memory pipe
+// (85 %), not by DRAM: at R-MAT s16 2.3e9 warp instructions, of which an item's
 // set-up and output 27 %, the A-entry walk 13 %, the products the rest.
 // Per launch, before this walk -> now: R-MAT s16 on 8x8 tiles 3.84 -> 2.85 ms,
 // s18 on 16x16 39.3 -> 30.3; R-MAT of 30,011 rows in int32 0.96 -> 0.37; graph x

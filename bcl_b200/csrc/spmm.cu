@@ -780,8 +780,9 @@ __global__ void __launch_bounds__(kLongPairs * 64)
 // run both at once: k_spmm_narrow is launched as k_spmm_chain's programmatic
 // dependent, starts once every chain block has, and ends after it.  With
 // fewer rows (where the extra launch would show) k_spmm_narrow lists the long
-// rows it meets and k_spmm_chain follows.
-// Bound: the short rows by instruction issue (67 % of the slots; a third of a
+// rows it meets and k_spmm_chain follows.  Rows that take all 32 lanes go to
+// k_spmm in place of k_spmm_narrow (see launch_narrow_nv).
+// Bound: the short rows by instruction issue (60-66 % of the slots; a third of a
 // warp's groups wait for its longest row) and by the latency of their loads
 // (A entry, then B row), hidden by 32 warps per SM; a long row by its chain,
 // 4.5 ns per entry (k_spmm_long: 25).  FP32 products, k_spmm before -> now:
