@@ -598,43 +598,60 @@ static int read_back(Context* ctx, std::initializer_list<std::tuple<const void*,
 // Does a row of a B tile name a column twice (or descend)?  Then *repeats is
 // set, and the numeric pass does not take a row's products for products of
 // distinct columns.  A part of the classification kernels, by blocks of 256: of
-// kRepeatRows rows the block counts the entries whose column is not above the
+// its rows the block counts the entries whose column is not above the
 // one before, and takes away the rows that begin with such an entry; what is
 // left are repeats.  (By the rows' ends alone, so that a hub row is no
-// thread's own walk.  After the classification: before it, blocks with more to
+// thread's own walk.  After the classification, or by later blocks: before it, blocks with more to
 // look through appended their rows later, and the lists' order, which the numeric
 // pass re-reads B in, cost the 27-point stencil on 128^3 22.1 -> 22.4 ms.)
+// Up to kRepeatRows rows at once, and so few that every block has some.  (2,048 always,
+// after the rows: the 27-point stencil of 9,261 rows 176 -> 190 us; by blocks of its
+// own, which run beside them, classification 12.1 -> 12.5 us.)
 constexpr int kRepeatRows = 2048;
-__device__ __forceinline__ void look_for_repeats(const SpGridView& B, const Geom& g, int32_t* __restrict__ repeats) {
+__device__ __forceinline__ void look_for_repeats(const SpGridView& B, const Geom& g, int32_t* __restrict__ repeats,
+                                                 uint32_t block, uint32_t blocks) {
   __shared__ int found;
   const int64_t nt = g.gk * g.gn;
-  int64_t t = blockIdx.x;
-  for (int64_t r0 = 0; r0 < g.tk; r0 += kRepeatRows) {  // (these rows of every tile, then the next)
-    for (; t < nt; t += gridDim.x) {
-      const bclx_csr_t Bt = B.tile(0, t);
-      const int64_t r1 = min(r0 + kRepeatRows, Bt.m);  // (the tile's own row count)
-      if (r0 >= r1 || (g.scount && Bt.nnz <= 0)) continue;  // (the stage map leaves such tiles out as well)
-      if (threadIdx.x == 0) found = 0;
-      __syncthreads();
-      const int32_t first = __ldg(Bt.row_ptr + r0), end = __ldg(Bt.row_ptr + r1);
-      int mine = 0;
-      const int n = end - first;
-#pragma unroll 8
-      for (int p = 1 + threadIdx.x; p < n; p += 256)
-        mine += __ldg(Bt.col_ind + first + p) <= __ldg(Bt.col_ind + first + p - 1);
-#pragma unroll 4
-      for (int64_t r = r0 + 1 + threadIdx.x; r < r1; r += 256) {
-        const int32_t s = __ldg(Bt.row_ptr + r);
-        if (s < __ldg(Bt.row_ptr + r + 1) && s > first && s < end)
-          mine -= __ldg(Bt.col_ind + s) <= __ldg(Bt.col_ind + s - 1);
-      }
-      mine = __reduce_add_sync(kFull, mine);
-      if (lane_id() == 0 && mine != 0) atomicAdd(&found, mine);
-      __syncthreads();
-      if (threadIdx.x == 0 && found != 0) *repeats = 1;
-      __syncthreads();
+  const int64_t rows = max((int64_t)16, min((int64_t)kRepeatRows, nt * g.tk / blocks));
+  // part r0 / rows of tile t, the tiles of one part after another; the next is `blocks` further
+  const int64_t ahead_r = blocks / nt * rows, ahead_t = blocks % nt;
+  int64_t r0 = block / nt * rows, t = block % nt;
+  for (; r0 < g.tk; r0 += ahead_r, t += ahead_t) {
+    if (t >= nt) {
+      t -= nt;
+      r0 += rows;
+      if (r0 >= g.tk) break;
     }
-    t -= nt;
+    const bclx_csr_t Bt = B.tile(0, t);
+    const int64_t r1 = min(r0 + rows, Bt.m);  // (the tile's own row count)
+    if (r0 >= r1 || (g.scount && Bt.nnz <= 0)) continue;  // (the stage map leaves such tiles out as well)
+    if (threadIdx.x == 0) found = 0;
+    __syncthreads();
+    const int32_t first = __ldg(Bt.row_ptr + r0), end = __ldg(Bt.row_ptr + r1);
+    int mine = 0;
+    const int n = end - first;
+    for (int p0 = 1 + threadIdx.x; p0 < n; p0 += 8 * 256) {  // (eight entries' loads in flight, the last ones too)
+      int32_t c[8], before[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {
+        const int p = min(p0 + q * 256, n - 1);
+        c[q] = __ldg(Bt.col_ind + first + p);
+        before[q] = __ldg(Bt.col_ind + first + p - 1);
+      }
+#pragma unroll
+      for (int q = 0; q < 8; q++) mine += p0 + q * 256 < n && c[q] <= before[q];
+    }
+#pragma unroll 4
+    for (int64_t r = r0 + 1 + threadIdx.x; r < r1; r += 256) {
+      const int32_t s = __ldg(Bt.row_ptr + r);
+      if (s < __ldg(Bt.row_ptr + r + 1) && s > first && s < end)
+        mine -= __ldg(Bt.col_ind + s) <= __ldg(Bt.col_ind + s - 1);
+    }
+    mine = __reduce_add_sync(kFull, mine);
+    if (lane_id() == 0 && mine != 0) atomicAdd(&found, mine);
+    __syncthreads();
+    if (threadIdx.x == 0 && found != 0) *repeats = 1;
+    __syncthreads();
   }
 }
 
@@ -751,7 +768,7 @@ __global__ void k_classify(SpGridView A, SpGridView B, Geom g, int32_t* __restri
     base = __shfl_sync(kFull, nx, 0);
   }
   if (lane == 0 && mine) atomicAdd(products, mine);
-  look_for_repeats(B, g, counters + 5);
+  look_for_repeats(B, g, counters + 5, blockIdx.x, gridDim.x);
 }
 
 // Products of every row for all of its C tiles at once: a warp takes a row of A's tile row ti, reads its
@@ -781,20 +798,24 @@ constexpr int kClassifyDefer = 64;  // long rows a block can put off
 __global__ void __launch_bounds__(256) k_classify_rows(
     SpGridView A, SpGridView B, Geom g, int32_t* __restrict__ light_list, int32_t* __restrict__ heavy_list,
     int32_t* __restrict__ vheavy_list, int32_t* __restrict__ counters, unsigned long long* __restrict__ products,
-    int heavy_min_cols, int light_ub, const unsigned long long* __restrict__ n_stages) {
+    int heavy_min_cols, int light_ub, const unsigned long long* __restrict__ n_stages, int row_blocks) {
   // counters [4]: rows above kMidHeavyUb, at the end of vheavy_list; [5]: look_for_repeats
   __shared__ int32_t kept_all[8][4][kClassifyKeep * 32];
   __shared__ unsigned long long sums[32];
   __shared__ uint32_t deferred[kClassifyDefer];
   __shared__ int n_deferred;
   if (n_stages && !mostly_full(g, n_stages)) return;
+  if ((int)blockIdx.x >= row_blocks) {  // (beside the rows where the product is small)
+    look_for_repeats(B, g, counters + 5, blockIdx.x - row_blocks, gridDim.x - row_blocks);
+    return;
+  }
   const int wid = threadIdx.x >> 5;
   int32_t(*kept)[kClassifyKeep * 32] = kept_all[wid];
   const int lane = lane_id();
   const unsigned below = (1u << lane) - 1u;
   const uint32_t n_rows = (uint32_t)(g.gm * g.tm), tm = (uint32_t)g.tm;
   const int gk = (int)g.gk, gn = (int)g.gn;
-  const uint32_t warp = wid * gridDim.x + blockIdx.x, nwarps = gridDim.x * 8;
+  const uint32_t warp = wid * row_blocks + blockIdx.x, nwarps = row_blocks * 8;
   unsigned long long mine = 0;
   int n_kept[4] = {0, 0, 0, 0};
   int rows = 0;
@@ -915,7 +936,6 @@ __global__ void __launch_bounds__(256) k_classify_rows(
 #pragma unroll
   for (int d = 16; d > 0; d >>= 1) mine += __shfl_xor_sync(kFull, mine, d);
   if (lane == 0 && mine) atomicAdd(products, mine);
-  look_for_repeats(B, g, counters + 5);
 }
 
 // B-row table: for every row of every B tile (k, j), the position of the
@@ -1066,7 +1086,7 @@ __global__ void __launch_bounds__(256) k_classify_tiles(
     for (int q = 0; q < 8; q++) all += sums[q];
     if (all) atomicAdd(products, all);
   }
-  look_for_repeats(B, g, counters + 5);
+  look_for_repeats(B, g, counters + 5, blockIdx.x, gridDim.x);
 }
 
 // ---- symbolic ----------------------------------------------------------------------
@@ -2408,10 +2428,11 @@ static int symbolic_impl(Context* ctx, const SpGridView& A, const SpGridView& B,
     // (few rows: see k_classify_rows)
     const bool rows = !live || g.gm * g.tm >= (int64_t)ctx->num_sms * kClassifyMinRows;
     const auto* n_stages = live ? reinterpret_cast<const unsigned long long*>(live + live_stages_at(nt)) : nullptr;
+    const unsigned row_blocks = grid_for(ctx, g.gm * g.tm, 8, 8);
     if (rows)
-      k_classify_rows<<<grid_for(ctx, g.gm * g.tm, 8, 8), 256, 0, ctx->stream>>>(
+      k_classify_rows<<<row_blocks + grid_for(ctx, g.gk * g.gn * g.tk / 8 + 1, 8, 4), 256, 0, ctx->stream>>>(
           A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,
-          P->light_ub_max, n_stages);
+          P->light_ub_max, n_stages, (int)row_blocks);
     if (live)
       k_classify_tiles<<<grid_for(ctx, nri / 32 + 1, 8, 8), 256, 0, ctx->stream>>>(
           A, B, g, P->light_list, P->heavy_tmp, P->vheavy_list, P->counters, P->products_dev, heavy_min_cols,

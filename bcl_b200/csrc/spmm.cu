@@ -1567,8 +1567,10 @@ static int launch_narrow_u(Context* ctx, const SpGridView& A, const DGridView& B
   while (L < 32 && (L * per < units || L < A.gn)) L *= 2;
   const int64_t nv = ceil_div(std::min<int64_t>(units, 32 * per), L);
   // rows that take all 32 lanes, for their width or for the stages' sake (k_spmm
-  // starts at tile column 0): see `wide` in launch_narrow_nv
-  const bool wide_rows = L == 32 && tj0 == 0;
+  // starts at tile column 0): see `wide` in launch_narrow_nv.  Not BF16 rows off 16
+  // bytes where they are few: R-MAT of 54,871 x 178 209 us with k_spmm_narrow, 233 with
+  // k_spmm (uniform 8,069 x 252 36 and 34).
+  const bool wide_rows = L == 32 && tj0 == 0 && (sizeof(ST) == 4 || A.gn > 16 || A.gm * A.tm >= spmm_long_min_rows());
   if constexpr (U != 16) {
     if (nv > 2) return launch_narrow_nv<ST, U, 4, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L, wide_rows);
     if (nv > 1) return launch_narrow_nv<ST, U, 2, SUB>(ctx, A, B, C, (int)tj0, (int)tjn, width, L, wide_rows);

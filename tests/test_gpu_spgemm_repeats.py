@@ -83,3 +83,16 @@ def test_accumulated_parts(nparts):
     parts = [matrix(120, 300, 24, "i32", 10 + p, range(p, 120, 4)) for p in range(nparts)]
     parts = [gen.CSR(p.m, p.n, p.row_ptr, p.col_ind, p.vals.astype(np.float32)) for p in parts]
     assert_csr_identical(tile_accumulate([tiled(p, 120, 300) for p in parts]).get(), *O.accumulate(parts))
+
+
+@pytest.mark.parametrize("row", [0, 63, 64, 127, 128, 900, 4999])
+def test_one_repeat_among_many_short_blocks(row):
+    """The rows are dealt to the blocks 64 and more at a time: one row with repeats, at
+    the first and last of such a part, in the last tile along k."""
+    from bcl_b200.containers import spgemm
+    a, b = matrix(64, 10000, 40, "f32", 8), matrix(10000, 300, 20, "f32", 9, (5000 + row,))
+    a.col_ind.reshape(64, 40)[:, -1] = 9999  # (ascending still)
+    a.col_ind.reshape(64, 40)[:, -2] = 5000 + row if row < 4999 else 9998
+    a.col_ind.reshape(64, 40)[:, :-2] = np.arange(38)
+    want = O.gemm_tiled(a, b, 64, 5000, 300)
+    assert_csr_identical(spgemm(tiled(a, 64, 5000), tiled(b, 5000, 300)).get(), *want)
